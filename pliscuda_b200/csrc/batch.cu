@@ -18,16 +18,18 @@ namespace plis {
 __global__ void k_batch_prepare(BatchArgs B, double t_end, unsigned long long n_steps) {
   const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= B.nrep) return;
-  Ctrl* K = B.ctrl + r;
-  if (K->status != PLIS_OK || K->phase != 1u) {
-    if (K->status != PLIS_OK) { K->done = 1; K->stop_reason = PLIS_STOP_ERROR; }
-    return;
+  Ctrl k = B.ctrl[r];
+  if (k.status != PLIS_OK) {
+    k.done = 1;
+    k.stop_reason = PLIS_STOP_ERROR;
+  } else if (k.phase == 1u) {
+    k.t_end = t_end;
+    k.max_step = (n_steps == ~0ull) ? ~0ull : k.step + n_steps;
+    k.done = 0;
+    k.stop_reason = PLIS_STOP_NONE;
+    prepare_step(k, B.o.mode);
   }
-  K->t_end = t_end;
-  K->max_step = (n_steps == ~0ull) ? ~0ull : K->step + n_steps;
-  K->done = 0;
-  K->stop_reason = PLIS_STOP_NONE;
-  prepare_step(K, B.o.mode);
+  B.ctrl[r] = k;
 }
 
 __global__ void k_batch_fill(double* tau0, double* tau1, uint8_t* f0, uint8_t* f1, uint32_t n) {
@@ -192,7 +194,9 @@ int BatchEngine::create(const plis_batch_desc& d, const plis_options& opt) {
   h_dr_ = dr;
   {  // small networks: every replica's tables and rate constants in its argument block (SmallModel)
     SmallModel probe;
-    small_ = fill_small_model(shared_, rr.data(), dr.data(), &probe);
+    small_ = !opt.stage_halo;
+    for (uint32_t r = 0; small_ && r < nrep_; ++r)
+      small_ = fill_small_model(shared_, &rr[(size_t)r * R_], &dr[(size_t)r * S_], opt, &probe);
   }
   if (opt.precision == PLIS_PREC_FP32) {
     const std::vector<float> rf(rr.begin(), rr.end()), df(dr.begin(), dr.end());
@@ -289,15 +293,8 @@ int BatchEngine::layout(const int tile[3]) {
   total_tiles_ = (uint32_t)toff;
   int rc;
   if (total_tiles_ > max_tiles_) {
-    if ((rc = dmalloc((void**)&d_slot_tau_, (size_t)total_tiles_ * 8))) return rc;
-    if ((rc = dmalloc((void**)&d_slot_idx_, (size_t)total_tiles_ * 8))) return rc;
-    if ((rc = dmalloc((void**)&d_slot_cr_, (size_t)total_tiles_ * 4))) return rc;
-    if ((rc = dmalloc((void**)&d_slot_bad_, (size_t)total_tiles_ * 4))) return rc;
+    if ((rc = dmalloc((void**)&d_slot_, (size_t)total_tiles_ * sizeof(SlotRec)))) return rc;
     max_tiles_ = total_tiles_;
-  }
-  if (learned_ && total_tiles_ > plain_tiles_) {
-    if ((rc = dmalloc((void**)&d_slot_plain_, (size_t)total_tiles_ * 8))) return rc;
-    plain_tiles_ = total_tiles_;
   }
   std::vector<KArgs> views(nrep_);
   const size_t rsz = opt_.precision == PLIS_PREC_FP32 ? sizeof(float) : sizeof(double);
@@ -322,16 +319,10 @@ int BatchEngine::layout(const int tile[3]) {
       v.b.flag[i] = d_flag_[i] + coff_[r];
     }
     v.b.D = d_D_ + coff_[r];
-    v.b.slot_tau = d_slot_tau_ + rep[r].tile_off;
-    v.b.slot_idx = d_slot_idx_ + rep[r].tile_off;
-    v.b.slot_cr = d_slot_cr_ + rep[r].tile_off;
-    v.b.slot_bad = d_slot_bad_ + rep[r].tile_off;
+    v.b.slot = d_slot_ + rep[r].tile_off;
     v.b.ctrl = d_ctrl_ + r;
-    if (small_) fill_small_model(shared_, &h_rr_[(size_t)r * R_], &h_dr_[(size_t)r * S_], &v.sm);
-    if (learned_) {
-      v.b.lp = d_lp_;
-      v.b.slot_tau_plain = d_slot_plain_ + rep[r].tile_off;
-    }
+    if (small_) fill_small_model(shared_, &h_rr_[(size_t)r * R_], &h_dr_[(size_t)r * S_], opt_, &v.sm);
+    if (learned_) v.b.lp = d_lp_;
   }
   PLIS_CU(cudaMemcpy(d_views_, views.data(), nrep_ * sizeof(KArgs), cudaMemcpyHostToDevice));
   PLIS_CU(cudaMemcpy(d_rep_, rep.data(), nrep_ * sizeof(RepDesc), cudaMemcpyHostToDevice));
@@ -348,8 +339,7 @@ int BatchEngine::layout(const int tile[3]) {
 
 static BatchArgs make_args(const DevModel& dm, const DevOpts& o, const Geo& g, void* views, void* rep, uint32_t nrep,
                            uint32_t R, uint32_t S, void* rr, void* dr, Ctrl* ctrl, int32_t* const X[3],
-                           double* const tau[2], uint8_t* const flag[2], int32_t* D, double* st, long long* si,
-                           uint32_t* sc, uint32_t* sb, unsigned* work, unsigned* bar, int* err, uint32_t iters) {
+                           double* const tau[2], uint8_t* const flag[2], int32_t* D, unsigned* work, unsigned* bar, int* err, uint32_t iters) {
   BatchArgs B;
   std::memset(&B, 0, sizeof B);
   B.m = dm;
@@ -366,7 +356,6 @@ static BatchArgs make_args(const DevModel& dm, const DevOpts& o, const Geo& g, v
   for (int i = 0; i < 3; ++i) B.X[i] = X[i];
   for (int i = 0; i < 2; ++i) { B.tau[i] = tau[i]; B.flag[i] = flag[i]; }
   B.D = D;
-  B.slot_tau = st; B.slot_idx = si; B.slot_cr = sc; B.slot_bad = sb;
   B.work = work;
   B.bar = bar;
   B.err = err;
@@ -382,7 +371,7 @@ void batch_prepare(const BatchArgs& B, double t_end, unsigned long long n_steps,
 
 int BatchEngine::launch(uint32_t max_iters) {
   BatchArgs B = make_args(dm_, dopt_, geo_, d_views_, d_rep_, nrep_, R_, S_, d_rr_, d_dr_, d_ctrl_, d_X_, d_tau_,
-                          d_flag_, d_D_, d_slot_tau_, d_slot_idx_, d_slot_cr_, d_slot_bad_, d_work_, d_bar_, d_err_,
+                          d_flag_, d_D_, d_work_, d_bar_, d_err_,
                           max_iters);
   if (opt_.wait_polls) B.spin_limit = opt_.wait_polls;
   PLIS_CU(cudaMemsetAsync(d_work_, 0, 12 * sizeof(unsigned), stream_));
@@ -487,7 +476,7 @@ int BatchEngine::run(double t_end, uint64_t n_steps) {
   int rc = init_pending();
   if (rc) return rc;
   BatchArgs B = make_args(dm_, dopt_, geo_, d_views_, d_rep_, nrep_, R_, S_, d_rr_, d_dr_, d_ctrl_, d_X_, d_tau_,
-                          d_flag_, d_D_, d_slot_tau_, d_slot_idx_, d_slot_cr_, d_slot_bad_, d_work_, d_bar_, d_err_, 0);
+                          d_flag_, d_D_, d_work_, d_bar_, d_err_, 0);
   PLIS_CU(cudaEventRecord(ev0_, stream_));
   batch_prepare(B, t_end, (unsigned long long)n_steps, stream_);
   launches_ += 1;

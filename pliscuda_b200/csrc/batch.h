@@ -84,10 +84,7 @@ class BatchEngine {
   double* d_tau_[2] = {nullptr, nullptr};
   uint8_t* d_flag_[2] = {nullptr, nullptr};
   int32_t* d_D_ = nullptr;
-  double* d_slot_tau_ = nullptr;
-  long long* d_slot_idx_ = nullptr;
-  uint32_t* d_slot_cr_ = nullptr;
-  uint32_t* d_slot_bad_ = nullptr;
+  SlotRec* d_slot_ = nullptr;
   unsigned* d_work_ = nullptr;
   unsigned* d_bar_ = nullptr;
   int* d_err_ = nullptr;
@@ -97,8 +94,6 @@ class BatchEngine {
   bool learned_ = false;
   struct LearnedParams* d_lp_ = nullptr;
   float* d_lw_ = nullptr;
-  double* d_slot_plain_ = nullptr;
-  uint32_t plain_tiles_ = 0;
 };
 
 }  // namespace plis

@@ -51,10 +51,6 @@ struct BatchArgs {
   double* tau[2];
   uint8_t* flag[2];
   int32_t* D;
-  double* slot_tau;    // per brick
-  long long* slot_idx;
-  uint32_t* slot_cr;
-  uint32_t* slot_bad;
   unsigned* work;      // [4 phases][3 generations] brick / replica counters
   unsigned* bar;       // grid barrier: [0] arrivals, [1] generation
   int* err;            // 1 = a barrier timed out
@@ -277,7 +273,8 @@ __global__ void __launch_bounds__(256, LEARNED ? PLIS_BATCH_MIN_BLOCKS_LEARNED :
         const Real tl = (Real)K->tau_leap;
         long long ev;
         int big;
-        leap_tile<Real, MAXS, false, false, SM>(sA, w - s_lp[r], L, tl, box, ev, big);
+        if constexpr (SM) leap_tile_small<Real, MAXS, false, true, false>(sA, sA.sm, w - s_lp[r], L, tl, ev, big);
+        else leap_tile<Real, MAXS, false, false>(sA, w - s_lp[r], L, tl, box, ev, big);
         ev = warp_sum(ev);  // events by warp, straight into the replica's counter (integer: order-free)
         if ((threadIdx.x & 31) == 0 && ev) atomicAdd(&K->ev_attempt, (unsigned long long)ev);
         if (big) atomicOr(&K->blocks_done, 0x80000000u);  // rare: an oversized draw forces a rollback
@@ -370,11 +367,12 @@ __global__ void __launch_bounds__(256, LEARNED ? PLIS_BATCH_MIN_BLOCKS_LEARNED :
         if (learned_classify_tile<Real, MAXS, false>(sA, K, C, tile, sA.g.nblocks)) classify_control(sA, K, sA.g.nblocks);
       } else {
         double tn;
-        long long ti;
+        uint32_t ti;
         int fl, bad;
         bool valid;
-        classify_tile<Real, MAXS, false, false, SM>(sA, tile, C, tn, ti, fl, bad, valid);
-        if (classify_slot(sA, K, tile, sA.g.nblocks, tn, ti, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
+        if constexpr (SM) classify_tile_small<Real, MAXS, true>(sA, sA.sm, tile, C, tn, ti, fl, bad, valid);
+        else classify_tile<Real, MAXS, false>(sA, tile, C, tn, ti, fl, bad, valid);
+        if (classify_slot<false>(sA, K, tile, sA.g.nblocks, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
           classify_control(sA, K, sA.g.nblocks);
       }
       __syncthreads();

@@ -78,10 +78,11 @@ int Engine::upload(const std::vector<T>& v, const T** out) {
   return PLIS_OK;
 }
 
-// The SmallModel block of a model that fits it (at most kSmallR reactions and kSmallS species, net
-// changes within int8, one set of rate constants: rrate[R] and drate[S]; rrate null = several sets);
-// sm->on = 0 otherwise.
-bool fill_small_model(const Model& M, const double* rrate, const double* drate, SmallModel* out) {
+// The SmallModel block of a model that fits it; sm->on = 0 otherwise.  It fits with at most kSmallR
+// reactions and kSmallS species, net changes within int8 (32-bit sums of the leap), one set of rate
+// constants (rrate[R] and drate[S]; rrate null = several sets), and jump rates that are zero or far
+// from the ends of the working precision's range (the neighbour terms' division, div_small).
+bool fill_small_model(const Model& M, const double* rrate, const double* drate, const plis_options& opt, SmallModel* out) {
   SmallModel& sm = *out;
   std::memset(&sm, 0, sizeof sm);
   const ReactionTables& t = M.rt;
@@ -91,16 +92,30 @@ bool fill_small_model(const Model& M, const double* rrate, const double* drate, 
       const int nu = M.products[s * M.R + r] - M.reactants[s * M.R + r];
       if (nu < -127 || nu > 127) fits = false;
     }
+  const bool f32 = opt.precision == PLIS_PREC_FP32;
+  const double lo = f32 ? 1e-25 : 1e-250, hi = f32 ? 1e25 : 1e250;
+  for (size_t s = 0; fits && s < M.S; ++s) fits = drate[s] == 0.0 || (drate[s] >= lo && drate[s] <= hi);
   if (!fits) return false;
+  for (int r = 0; r < kSmallR; ++r)
+    for (int s = 0; s < kSmallS; ++s) sm.thr[r][s] = INT32_MIN;
+  const int64_t nc = opt.critical_threshold;
   for (uint32_t r = 0; r < M.R; ++r) {
-    sm.nreac[r] = t.n_reac[r];
     for (int i = 0; i < t.n_reac[r]; ++i) {
-      sm.rs[r][i] = (uint8_t)t.reac_s[r * kMaxReactantSpecies + i];
-      sm.rm[r][i] = t.reac_m[r * kMaxReactantSpecies + i];
-      sm.rnu[r][i] = (int8_t)t.reac_nu[r * kMaxReactantSpecies + i];
-      sm.rmask[sm.rs[r][i]] |= (uint8_t)(1u << r);
+      const uint32_t s = t.reac_s[r * kMaxReactantSpecies + i];
+      const int64_t nu = t.reac_nu[r * kMaxReactantSpecies + i];
+      sm.ord[r][s] = t.reac_m[r * kMaxReactantSpecies + i];
+      sm.rmask[s] |= 1u << r;
+      // reference: the first two reactant species decide, none left or fewer than NC firings' worth
+      // (tau.cu:3-40); corrected: every consumed species, fewer than NC firings' worth
+      int64_t thr = INT32_MIN;
+      if (opt.mode == PLIS_MODE_REFERENCE) {
+        if (i < 2) thr = nu < 0 ? std::max<int64_t>(1, -nu * nc) : 1;
+      } else if (nu < 0) {
+        thr = -nu * nc;
+      }
+      sm.thr[r][s] = (int32_t)std::min<int64_t>(std::max<int64_t>(thr, INT32_MIN), INT32_MAX);
     }
-    for (int i = 0; i < t.n_net[r]; ++i) sm.nu[r][t.net_s[r * kMaxNet + i]] = (int8_t)t.net_nu[r * kMaxNet + i];
+    for (int i = 0; i < t.n_net[r]; ++i) sm.nu[r][t.net_s[r * kMaxNet + i]] = t.net_nu[r * kMaxNet + i];
     sm.inv_denom[r] = t.inv_denom[r];
     sm.rate_d[r] = rrate[r];
     sm.rate_f[r] = (float)rrate[r];
@@ -182,7 +197,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
   }
 
   // a small model's tables in the kernel arguments (SmallModel)
-  fill_small_model(M, M.comp.empty() ? M.rrate.data() : nullptr, M.drate.data(), &args_.sm);
+  fill_small_model(M, M.comp.empty() ? M.rrate.data() : nullptr, M.drate.data(), opt, &args_.sm);
 
   // geometry
   Geo& g = args_.g;
@@ -245,10 +260,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
   // than N/2 events in one attempt fall back to a scan of all deltas)
   if ((rc = dmalloc((void**)&b.D, (cells + dm.Npad) * 4))) return rc;
   PLIS_CU(cudaMemset(b.D, 0, cells * 4));
-  if ((rc = dmalloc((void**)&b.slot_tau, (size_t)g.nblocks * 8))) return rc;
-  if ((rc = dmalloc((void**)&b.slot_idx, (size_t)g.nblocks * 8))) return rc;
-  if ((rc = dmalloc((void**)&b.slot_cr, (size_t)g.nblocks * 4))) return rc;
-  if ((rc = dmalloc((void**)&b.slot_bad, (size_t)g.nblocks * 4))) return rc;
+  if ((rc = dmalloc((void**)&b.slot, (size_t)g.nblocks * sizeof(SlotRec)))) return rc;
   if ((rc = dmalloc((void**)&b.ctrl, sizeof(Ctrl)))) return rc;
   PLIS_CU(cudaMemset(b.ctrl, 0, sizeof(Ctrl)));
 
@@ -262,7 +274,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
   o.replica = opt.replica;
   devopts_keys(o);
   o.pool = pooled_draws_on(opt.pooled_draws, M.R, M.S);
-  if (o.pool) args_.sm.on = 0;  // pooled draws live in the generic leap only
+  if (o.pool || opt.stage_halo) args_.sm.on = 0;  // pooled draws and the staged box live in the generic leap only
 
   launch_ = (opt.precision == PLIS_PREC_FP32) ? pick_f32(M.S) : pick_f64(M.S);
   // shared-memory staging of the leap's brick + halo (lattices only, when the box fits)
@@ -422,7 +434,6 @@ int Engine::set_proposer(const float* weights, double s_max) {
     if (!d_lp_) {
       if ((rc = dmalloc((void**)&d_lp_, sizeof(LearnedParams)))) return rc;
       if ((rc = dmalloc((void**)&d_lw_, PLIS_PROPOSER_WEIGHTS * sizeof(float)))) return rc;
-      if ((rc = dmalloc((void**)&d_slot_plain_, (size_t)args_.g.nblocks * sizeof(double)))) return rc;
     }
     if (opt_.learned_mlp == PLIS_MLP_TCGEN05 && !d_feat_) {  // the split classification's buffers
       const size_t rows = ((size_t)args_.m.Npad + 127) / 128 * 128;
@@ -436,14 +447,12 @@ int Engine::set_proposer(const float* weights, double s_max) {
     learned_pack(d_lw_, s_max, d_lp_, stream_);
     PLIS_CU(cudaGetLastError());
     args_.b.lp = d_lp_;
-    args_.b.slot_tau_plain = d_slot_plain_;
     args_.b.feat = d_feat_;
     args_.b.pre = d_pre_;
     args_.b.pre_kind = d_pre_kind_;
     args_.b.ymlp = d_ymlp_;
   } else {
     args_.b.lp = nullptr;
-    args_.b.slot_tau_plain = nullptr;
   }
   use_learned_ = on;
   const int classify_launches = (on && opt_.learned_mlp == PLIS_MLP_TCGEN05) ? 3 : 1;

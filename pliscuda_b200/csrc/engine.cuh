@@ -18,7 +18,7 @@ constexpr int64_t kBigTile = (int64_t)1 << 30;  // |x + own delta| of one subvol
 // The whole control state of a simulation lives on the device, so a batch of steps (rollbacks
 // included) runs without the host: the reference instead reads the arg-min back and decides on
 // the host every step (driver.cu:267-315).
-struct Ctrl {
+struct alignas(16) Ctrl {
   double t_end;          // stop once t >= t_end
   uint64_t max_step;     // stop once step >= max_step
   double t;              // simulated time (binary64)
@@ -95,17 +95,24 @@ struct EvLog {
   unsigned long long cap;
 };
 
+// What one CTA (brick) of the classification found, two 16-byte words.
+struct alignas(16) SlotRec {
+  double tau;        // min tau
+  double tau_plain;  // learned classification: min of the plain taus
+  uint32_t idx;      // the subvolume of tau (first on ties), 0xFFFFFFFF when the brick has none
+  uint32_t crff;     // #LEAP_CR | #SSA_FF << 16 (<= 1024 each)
+  uint32_t bad;      // 1: a negative count
+  uint32_t pad_;
+};
+static_assert(sizeof(SlotRec) == 32, "SlotRec is read as two uint4");
+
 struct DevBufs {
   int32_t* X[3];
   double* tau[2];
   uint8_t* flag[2];
   int32_t* D;
-  double* slot_tau;
-  long long* slot_idx;
-  uint32_t* slot_cr;
-  uint32_t* slot_bad;
-  double* slot_tau_plain;  // learned classification: per-CTA min of the plain taus (else null)
-  const struct LearnedParams* lp;  // learned classification: the proposer's packed weights
+  SlotRec* slot;           // one per CTA (brick) of the classification
+  const struct LearnedParams* lp;  // learned classification: the proposer's packed weights (else null)
   uint4* feat;             // learned classification (split): normalised BF16 features, 16 B per subvolume
   double2* pre;            // (leap bound or fast-forwarded tau, critical rate) per subvolume
   uint8_t* pre_kind;       // 1: fast-forwarded, 2: leap bound computed
@@ -177,17 +184,16 @@ inline uint32_t pooled_draws_on(int32_t setting, uint32_t R, uint32_t S) {
 }
 struct SmallModel {
   uint32_t on;                   // 1: the model fits and the tables below are filled
-  uint8_t nreac[kSmallR];        // distinct reactant species of reaction r
-  uint8_t rs[kSmallR][3];        // reactant species, increasing
-  uint8_t rm[kSmallR][3];        // their multiplicities (1..3)
-  int8_t rnu[kSmallR][3];        // their net change (the reference's criticality test)
-  int8_t nu[kSmallR][kSmallS];   // net change of every species (0 for species >= S and reactions >= R)
-  uint8_t hor[kSmallS], hmult[kSmallS];
-  uint8_t rmask[kSmallS];        // bit r: species s is a reactant of reaction r
+  // whole words: a table value is a constant-bank operand of the instruction that uses it
+  int32_t ord[kSmallR][kSmallS]; // multiplicity of species s among the reactants of reaction r (0..3)
+  int32_t thr[kSmallR][kSmallS]; // reaction r is critical while species s counts less than this (INT32_MIN: never)
+  int32_t nu[kSmallR][kSmallS];  // net change of every species (0 for species >= S and reactions >= R)
+  int32_t hor[kSmallS], hmult[kSmallS];
+  uint32_t rmask[kSmallS];       // bit r: species s is a reactant of reaction r
   double inv_denom[kSmallR];
   double rate_d[kSmallR];
-  float rate_f[kSmallR];
   double drate_d[kSmallS];
+  float rate_f[kSmallR];
   float drate_f[kSmallS];
 };
 

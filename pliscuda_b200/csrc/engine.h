@@ -24,7 +24,7 @@ struct Launchers {
 };
 
 // SmallModel tables of a model (engine.cu); false, with sm->on = 0, when it does not fit.
-bool fill_small_model(const Model& M, const double* rrate, const double* drate, SmallModel* sm);
+bool fill_small_model(const Model& M, const double* rrate, const double* drate, const plis_options& opt, SmallModel* sm);
 
 class Engine {
  public:
@@ -91,7 +91,6 @@ class Engine {
   LearnedLaunch llaunch_{};
   LearnedParams* d_lp_ = nullptr;
   float* d_lw_ = nullptr;
-  double* d_slot_plain_ = nullptr;
   uint4* d_feat_ = nullptr;
   double2* d_pre_ = nullptr;
   uint8_t* d_pre_kind_ = nullptr;

@@ -542,59 +542,13 @@ __device__ __forceinline__ Real gfun(int hor, int hmult, int32_t x) {
   }
 }
 
-// Small models (SmallModel in the kernel arguments): the same propensity, criticality and rate
-// constants as prop / crit_ref / crit_fix / drate above, from the argument tables.  The product of
-// falling factorials is formed in the same order (reactant species increasing, x, x-1, x-2).
+// rate constants of a small model (SmallModel in the kernel arguments) in the working precision
 template <typename Real> __device__ __forceinline__ Real sm_rate(const SmallModel& t, int r);
 template <> __device__ __forceinline__ double sm_rate<double>(const SmallModel& t, int r) { return t.rate_d[r]; }
 template <> __device__ __forceinline__ float sm_rate<float>(const SmallModel& t, int r) { return t.rate_f[r]; }
 template <typename Real> __device__ __forceinline__ Real sm_drate(const SmallModel& t, int s);
 template <> __device__ __forceinline__ double sm_drate<double>(const SmallModel& t, int s) { return t.drate_d[s]; }
 template <> __device__ __forceinline__ float sm_drate<float>(const SmallModel& t, int s) { return t.drate_f[s]; }
-
-template <typename Real, int MAXS>
-__device__ __forceinline__ Real prop_sm(const SmallModel& t, const Counts<MAXS>& x, int r) {
-  Real prod = (Real)1;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (i < t.nreac[r]) {
-      const Real xs = (Real)x.get(t.rs[r][i]);
-      const int mu = t.rm[r][i];
-      prod = prod * xs;
-      if (mu > 1) prod = prod * (xs - (Real)1);
-      if (mu > 2) prod = prod * (xs - (Real)2);
-    }
-  }
-  return (sm_rate<Real>(t, r) * prod) * (Real)t.inv_denom[r];
-}
-
-template <int MAXS>
-__device__ __forceinline__ bool crit_ref_sm(const SmallModel& t, const Counts<MAXS>& x, int r, int nc) {
-  const int lim = t.nreac[r] < 2 ? t.nreac[r] : 2;
-  bool crit = false;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    if (i < lim) {
-      const int32_t xs = x.get(t.rs[r][i]);
-      if (xs == 0) return true;
-      const int nu = t.rnu[r][i];
-      if (nu < 0 && (long long)(-nu) * nc > xs) crit = true;
-    }
-  }
-  return crit;
-}
-
-template <typename Real, int MAXS>
-__device__ __forceinline__ bool crit_fix_sm(const SmallModel& t, const Counts<MAXS>& x, int r, Real a, int nc) {
-  if (!(a > (Real)0)) return false;
-  bool crit = false;
-#pragma unroll
-  for (int s = 0; s < MAXS; ++s) {
-    const int nu = t.nu[r][s];
-    if (nu < 0 && x.v[s] < (long long)(-nu) * nc) crit = true;
-  }
-  return crit;
-}
 
 template <int MAXS>
 __device__ __forceinline__ void load_counts(const DevModel& m, const int32_t* X, uint32_t c, Counts<MAXS>& x) {
@@ -632,10 +586,6 @@ __device__ __forceinline__ bool classify_ff(int mode, double tau_cur, uint8_t fl
 // flags into a bit mask, and the loops below read them back; without it each loop evaluates them
 // again (the batched and learned kernels, and models with more reactions).  Same values either way.
 constexpr int kPropCache = 20;  // 20 x 256 threads x 8 B = 40 KB: under the 48 KB a launch gets without opting in
-template <typename Real, bool WALK = true, int MAXS>
-__device__ __forceinline__ void cell_tau_parts_sm(const KArgs& A, const Nbr& q, const Counts<MAXS>& x,
-                                                  const int32_t* Xe, Real& tau_ncr_out, Real& rate_cr_out);
-
 template <typename Real, bool WALK = true, bool CACHE = false, int MAXS>
 __device__ __forceinline__ void cell_tau_parts(const KArgs& A, uint32_t c, const Nbr& q, const Counts<MAXS>& x,
                                                const int32_t* Xe, Real& tau_ncr_out, Real& rate_cr_out,
@@ -753,120 +703,6 @@ __device__ __forceinline__ void cell_tau_parts(const KArgs& A, uint32_t c, const
   rate_cr_out = (rsum == (Real)0 && dsum == (Real)0) ? (Real)0 : rsum + dsum;
 }
 
-// cell_tau_parts for a small model (SmallModel in the kernel arguments): the same quantities in the
-// same order, with the species and reaction loops unrolled to the tables' compile-time sizes.
-template <typename Real, bool WALK, int MAXS>
-__device__ __forceinline__ void cell_tau_parts_sm(const KArgs& A, const Nbr& q, const Counts<MAXS>& x,
-                                                  const int32_t* Xe, Real& tau_ncr_out, Real& rate_cr_out) {
-  static_assert(MAXS <= kSmallS, "small-model tables hold kSmallS species");
-  const DevModel& m = A.m;
-  const SmallModel& t = A.sm;
-  const int mode = A.o.mode;
-  const int nc = A.o.nc;
-  const int n = q.n;
-  const int S = (int)m.S, R = (int)m.R;
-  Real tau_ncr = RT<Real>::inf();
-#pragma unroll
-  for (int s = 0; s < MAXS; ++s) {
-    if (s >= S) continue;
-    const int32_t xs = x.v[s];
-    bool include;
-    if (mode == 0) {
-      bool skip_r = false;
-#pragma unroll
-      for (int r = 0; r < kSmallR; ++r)
-        if ((t.rmask[s] >> r) & 1u) skip_r = skip_r || crit_ref_sm(t, x, r, nc);
-      include = !(skip_r && xs < nc);  // tau.cu:165
-    } else {
-      include = false;
-#pragma unroll
-      for (int r = 0; r < kSmallR; ++r)
-        if ((t.rmask[s] >> r) & 1u) {
-          const Real a = prop_sm<Real>(t, x, r);
-          include = include || ((a > (Real)0) && !crit_fix_sm(t, x, r, a, nc));
-        }
-      if (!include && xs >= nc && sm_drate<Real>(t, s) > (Real)0 && n > 0) include = true;
-    }
-    if (!include) continue;
-    const Real g = gfun<Real>(t.hor[s], t.hmult[s], xs);
-    Real mu = (Real)0, s2 = (Real)0;
-#pragma unroll
-    for (int r = 0; r < kSmallR; ++r) {
-      const int nu = t.nu[r][s];  // 0 for reactions >= R
-      if (nu == 0) continue;
-      const Real a = prop_sm<Real>(t, x, r);
-      const bool ncrit = (mode == 0) ? !crit_ref_sm(t, x, r, nc) : ((a > (Real)0) && !crit_fix_sm(t, x, r, a, nc));
-      if (!ncrit) continue;
-      mu = mu + (Real)nu * a;
-      s2 = s2 + (Real)(nu * nu) * a;
-    }
-    const Real dr = sm_drate<Real>(t, s);
-    const Real d = dr * (Real)xs;
-    if (mode == 0) {
-      if (xs >= nc) { mu = mu + d; s2 = s2 + d; }
-      auto term = [&](uint32_t b, int nn) {
-        const Real db = dr * (Real)Xe[(size_t)s * m.Npad + b];
-        const Real qd = db / (Real)nn;
-        mu = mu - qd;
-        s2 = s2 + qd;
-      };
-      if constexpr (WALK) for_each_nbr(m, q, term);
-      else for (int j = 0; j < n; ++j) term(q.nb[j], (int)q.nn[j]);
-    } else {
-      if (xs >= nc && n > 0) {
-        const Real dout = (Real)n * d;
-        mu = mu - dout;
-        s2 = s2 + dout;
-      }
-      auto term = [&](uint32_t b, int) {
-        const int32_t xb = Xe[(size_t)s * m.Npad + b];
-        if (xb >= nc) {
-          const Real qd = dr * (Real)xb;
-          mu = mu + qd;
-          s2 = s2 + qd;
-        }
-      };
-      if constexpr (WALK) for_each_nbr(m, q, term);
-      else for (int j = 0; j < n; ++j) term(q.nb[j], (int)q.nn[j]);
-    }
-    Real mm = ((Real)A.o.eps * (Real)xs) / g;
-    if (!(mm > (Real)1)) mm = (Real)1;
-    const Real t1 = mm / fabs(mu);
-    const Real t2 = (mm * mm) / s2;
-    const Real ts = t1 < t2 ? t1 : t2;
-    if (ts < tau_ncr) tau_ncr = ts;
-  }
-  Real rsum = (Real)0, dsum = (Real)0;
-  const bool ncr_inf = plis_isinf_d((double)tau_ncr);
-  if (mode == 0 || !ncr_inf) {
-#pragma unroll
-    for (int r = 0; r < kSmallR; ++r) {
-      if (r >= R) continue;
-      const Real a = prop_sm<Real>(t, x, r);
-      const bool cr = (mode == 0) ? crit_ref_sm(t, x, r, nc) : crit_fix_sm(t, x, r, a, nc);
-      if (cr) rsum = rsum + a;
-    }
-#pragma unroll
-    for (int s = 0; s < MAXS; ++s) {
-      if (s >= S) continue;
-      const int32_t xs = x.v[s];
-      if (xs < nc) {
-        const Real d = sm_drate<Real>(t, s) * (Real)xs;
-        dsum = dsum + (mode == 0 ? d : (Real)n * d);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < kSmallR; ++r)
-      if (r < R) rsum = rsum + prop_sm<Real>(t, x, r);
-#pragma unroll
-    for (int s = 0; s < MAXS; ++s)
-      if (s < S) dsum = dsum + (Real)n * (sm_drate<Real>(t, s) * (Real)x.v[s]);
-  }
-  tau_ncr_out = tau_ncr;
-  rate_cr_out = (rsum == (Real)0 && dsum == (Real)0) ? (Real)0 : rsum + dsum;
-}
-
 // tau_cr: exponential time of the critical rate (inf when it is zero), tau.cu:193.
 template <typename Real>
 __device__ __forceinline__ double cell_tau_cr(const KArgs& A, uint32_t c, uint64_t step, uint32_t attempt, Real rate) {
@@ -892,14 +728,13 @@ __device__ __forceinline__ void cell_decide(double tn, double tcr, double& tau_o
 // ------------------------------------------------------------------------------------------------
 // classification of one subvolume (compute_taus, tau.cu:197-252)
 // ------------------------------------------------------------------------------------------------
-template <typename Real, bool WALK = true, bool CACHE = false, bool SM = false, int MAXS>
+template <typename Real, bool WALK = true, bool CACHE = false, int MAXS>
 __device__ void classify_cell(const KArgs& A, uint32_t c, const Nbr& q, const Counts<MAXS>& x, const int32_t* Xe,
                               double tau_cur, uint8_t flag_cur, uint64_t step, uint32_t attempt,
                               double ff, double& tau_out, int& flag_out, Real* pc = nullptr, uint32_t stride = 0) {
   if (classify_ff(A.o.mode, tau_cur, flag_cur, step, ff, tau_out, flag_out)) return;
   Real tau_ncr, rate;
-  if constexpr (SM) cell_tau_parts_sm<Real, WALK>(A, q, x, Xe, tau_ncr, rate);
-  else cell_tau_parts<Real, WALK, CACHE>(A, c, q, x, Xe, tau_ncr, rate, pc, stride);
+  cell_tau_parts<Real, WALK, CACHE>(A, c, q, x, Xe, tau_ncr, rate, pc, stride);
   const double tcr = cell_tau_cr<Real>(A, c, step, attempt, rate);
   cell_decide((double)tau_ncr, tcr, tau_out, flag_out);
 }
@@ -907,84 +742,104 @@ __device__ void classify_cell(const KArgs& A, uint32_t c, const Nbr& q, const Co
 // ------------------------------------------------------------------------------------------------
 // control (runs in one thread of the last CTA of k_classify, or in k_prepare)
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void set_attempt(Ctrl* K, int mode) {
+// Both work on a copy of the control block: loaded and stored whole, its fields cost one round trip to
+// L2 instead of one each.
+__device__ __forceinline__ void set_attempt(Ctrl& k, int mode) {
   double scale = 1.0;
-  for (uint32_t i = 0; i < K->attempt; ++i) scale *= 0.5;
-  if (K->learned && K->attempt > 0) {  // a proposal was rolled back: plain Cao step, halved per attempt
-    K->tau_leap = K->tau_step_plain * scale;
-    K->dt = K->tau_leap;
-    K->exact = 0;
-    K->ev_attempt = 0;
-    K->ex_attempt = 0;
+  for (uint32_t i = 0; i < k.attempt; ++i) scale *= 0.5;
+  if (k.learned && k.attempt > 0) {  // a proposal was rolled back: plain Cao step, halved per attempt
+    k.tau_leap = k.tau_step_plain * scale;
+    k.dt = k.tau_leap;
+    k.exact = 0;
+    k.ev_attempt = 0;
+    k.ex_attempt = 0;
     return;
   }
   if (mode == 0) {  // the reference re-leaps with the un-halved tau but advances time by the halved one
-    K->tau_leap = K->tau_min;
-    K->dt = K->tau_min * scale;
+    k.tau_leap = k.tau_min;
+    k.dt = k.tau_min * scale;
   } else {
-    K->tau_leap = K->tau_step * scale;
-    K->dt = K->tau_leap;
+    k.tau_leap = k.tau_step * scale;
+    k.dt = k.tau_leap;
   }
-  const uint32_t af = K->argmin_flag;
+  const uint32_t af = k.argmin_flag;
   uint32_t ex = 0;
   if (mode == 0) {
-    if (K->n_leap_cr > 0) ex |= 1u;
+    if (k.n_leap_cr > 0) ex |= 1u;
     if (af == F_SSA || af == F_SSA_FF) ex |= 2u;
-  } else if (K->attempt == 0 && K->tau_step == K->tau_min &&
+  } else if (k.attempt == 0 && k.tau_step == k.tau_min &&
              (af == F_LEAP_CR || af == F_SSA || af == F_SSA_FF)) {
     ex |= 2u;
   }
-  K->exact = ex;
-  K->ev_attempt = 0;
-  K->ex_attempt = 0;
+  k.exact = ex;
+  k.ev_attempt = 0;
+  k.ex_attempt = 0;
 }
 
-__device__ __forceinline__ void prepare_step(Ctrl* K, int mode) {
-  if (K->done) return;
-  if (K->t >= K->t_end) { K->done = 1; K->stop_reason = PLIS_STOP_TIME; return; }
-  if (K->step >= K->max_step) { K->done = 1; K->stop_reason = PLIS_STOP_STEPS; return; }
-  if (K->argmin < 0 || plis_isinf_d(K->tau_min) || K->tau_min < 0.0) {  // driver.cu:269-272
-    if (mode == 1) { K->t = K->t_end; K->stop_reason = PLIS_STOP_TIME; }
-    else K->stop_reason = PLIS_STOP_NO_EVENT;
-    K->done = 1;
+__device__ __forceinline__ void prepare_step(Ctrl& k, int mode) {
+  if (k.done) return;
+  if (k.t >= k.t_end) { k.done = 1; k.stop_reason = PLIS_STOP_TIME; return; }
+  if (k.step >= k.max_step) { k.done = 1; k.stop_reason = PLIS_STOP_STEPS; return; }
+  if (k.argmin < 0 || plis_isinf_d(k.tau_min) || k.tau_min < 0.0) {  // driver.cu:269-272
+    if (mode == 1) { k.t = k.t_end; k.stop_reason = PLIS_STOP_TIME; }
+    else k.stop_reason = PLIS_STOP_NO_EVENT;
+    k.done = 1;
     return;
   }
-  K->tau_step = K->tau_min;
-  if (mode == 1 && K->t_end - K->t < K->tau_step) K->tau_step = K->t_end - K->t;
-  if (K->learned) {
-    K->tau_step_plain = K->tau_min_plain;
-    if (K->t_end - K->t < K->tau_step_plain) K->tau_step_plain = K->t_end - K->t;
+  k.tau_step = k.tau_min;
+  if (mode == 1 && k.t_end - k.t < k.tau_step) k.tau_step = k.t_end - k.t;
+  if (k.learned) {
+    k.tau_step_plain = k.tau_min_plain;
+    if (k.t_end - k.t < k.tau_step_plain) k.tau_step_plain = k.t_end - k.t;
   }
-  K->attempt = 0;
-  set_attempt(K, mode);
+  k.attempt = 0;
+  set_attempt(k, mode);
 }
 
 #ifdef PLIS_ENGINE_HOST_TU
 __global__ void k_prepare(KArgs A, double t_end, unsigned long long n_steps) {
   Ctrl* K = A.b.ctrl;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (K->status != PLIS_OK) { K->done = 1; K->stop_reason = PLIS_STOP_ERROR; return; }
-  K->t_end = t_end;
-  K->max_step = (n_steps == ~0ull) ? ~0ull : K->step + n_steps;
-  K->done = 0;
-  K->stop_reason = PLIS_STOP_NONE;
-  prepare_step(K, A.o.mode);
+  Ctrl k = *K;
+  if (k.status != PLIS_OK) {
+    k.done = 1;
+    k.stop_reason = PLIS_STOP_ERROR;
+  } else {
+    k.t_end = t_end;
+    k.max_step = (n_steps == ~0ull) ? ~0ull : k.step + n_steps;
+    k.done = 0;
+    k.stop_reason = PLIS_STOP_NONE;
+    prepare_step(k, A.o.mode);
+  }
+  *K = k;
 }
 #endif
 
 // ------------------------------------------------------------------------------------------------
 // reductions
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void min_pair(double& t, long long& i, double t2, long long i2) {
-  if (t2 < t || (t2 == t && i2 < i)) { t = t2; i = i2; }
+// A tau and its subvolume as unsigned integers that order as (tau, index): the sign bit of a
+// positive double set, a negative one inverted; NaN after everything.
+constexpr uint32_t kNoCell = 0xFFFFFFFFu;
+__device__ __forceinline__ uint64_t tau_key(double t) {
+  const uint64_t b = (uint64_t)__double_as_longlong(t);
+  const uint64_t k = b ^ ((uint64_t)((int64_t)b >> 63) | 0x8000000000000000ull);
+  return t == t ? k : ~0ull;
 }
-__device__ __forceinline__ void warp_min_pair(double& t, long long& i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double t2 = __shfl_xor_sync(0xffffffffu, t, o);
-    const long long i2 = __shfl_xor_sync(0xffffffffu, i, o);
-    min_pair(t, i, t2, i2);
-  }
+__device__ __forceinline__ double key_tau(uint64_t k) {
+  return __longlong_as_double((long long)(k ^ ((k >> 63) ? 0x8000000000000000ull : ~0ull)));
+}
+__device__ __forceinline__ void min_key(uint64_t& k, uint32_t& i, uint64_t k2, uint32_t i2) {
+  if (k2 < k || (k2 == k && i2 < i)) { k = k2; i = i2; }
+}
+// min key of the warp and the smallest index that has it: three integer warp reductions in place
+// of five rounds of four shuffles
+__device__ __forceinline__ void warp_min_key(uint64_t& k, uint32_t& i) {
+  const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32));
+  const uint32_t lo = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0xffffffffu);
+  const uint64_t m = ((uint64_t)hi << 32) | lo;
+  i = __reduce_min_sync(0xffffffffu, k == m ? i : kNoCell);
+  k = m;
 }
 __device__ __forceinline__ double warp_min_d(double v) {
 #pragma unroll
@@ -1037,16 +892,17 @@ struct LeapCtx {
   bool ff_free;  // no subvolume is SSA_FF: the receivers' flag updates are no-ops and are skipped
 };
 
+}  // namespace plis
+#include "small_step.cuh"
+namespace plis {
+
 // Leap of one brick (or one 1-D block of a table topology) by the whole CTA; returns this thread's
 // events and guard flag.  leap_step, leap.cu:3-65.
-// SM: a small model whose tables are in A.sm (SmallModel): the reaction and species loops run to
-// the tables' compile-time sizes, so every table read is a constant-bank operand.
 // RK: the group blocks use the round keys in A.o (kernel arguments: constant-bank operands); the
 // batched kernel, whose per-replica arguments sit in shared memory, recomputes them instead.
-template <typename Real, int MAXS, bool LOG, bool WALK = true, bool SM = false, bool RK = false>
+template <typename Real, int MAXS, bool LOG, bool WALK = true, bool RK = false>
 __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const LeapCtx& L, Real tl, const Box& box,
                                           long long& ev, int& big) {
-  static_assert(!SM || MAXS <= kSmallS, "small-model tables hold kSmallS species");
   const DevModel& m = A.m;
   const int mode = A.o.mode, nc = A.o.nc;
   const int32_t* Xc = L.Xc;
@@ -1075,11 +931,11 @@ __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const L
     for (int s = 0; s < MAXS; ++s) dl.v[s] = 0;
     const uint8_t f = flag[c];
     if (f == F_LEAP_CR || f == F_LEAP_NOCR) {  // leap.cu:9-10
-      const int comp = SM ? 0 : comp_of(m, c);
+      const int comp = comp_of(m, c);
       const int S = (int)m.S, R = (int)m.R;
       // pooled draws (plis_stream.h): the running total of the pool and the membership rule, the
       // same in the walk that fills the pool and in the walks that place its events
-      const bool pool_on = !SM && A.o.pool != 0;
+      const bool pool_on = A.o.pool != 0;
       Real pool = (Real)0;
       auto pool_join = [](Real& acc, Real unit, Real w) -> bool {
         if (!(unit < (Real)PLIS_POOL_CUT) || !(acc + w <= (Real)PLIS_POOL_MAX)) return false;
@@ -1100,15 +956,8 @@ __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const L
           u[i] = (Real)0;
           kk[i] = 0;
           if (r < R) {
-            Real a;
-            bool fire;
-            if constexpr (SM) {
-              a = prop_sm<Real>(A.sm, x, r);
-              fire = (mode == 0) ? !crit_ref_sm(A.sm, x, r, nc) : ((a > (Real)0) && !crit_fix_sm(A.sm, x, r, a, nc));
-            } else {
-              a = prop<Real>(m, x, r, comp);
-              fire = (mode == 0) ? !crit_ref(m, x, r, nc) : ((a > (Real)0) && !crit_fix(m, x, r, a, nc));
-            }
+            const Real a = prop<Real>(m, x, r, comp);
+            const bool fire = (mode == 0) ? !crit_ref(m, x, r, nc) : ((a > (Real)0) && !crit_fix(m, x, r, a, nc));
             lam[i] = fire ? tl * a : (Real)0;
             if (pool_on && lam[i] > (Real)0 && pool_join(pool, lam[i], lam[i])) lam[i] = (Real)0;  // pooled
             if (lam[i] > (Real)0) {
@@ -1149,33 +998,15 @@ __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const L
           const long long k = act[i] ? ks[i] : kk[i];
           ev += k;
           if (LOG && k > 0) ev_put(A.b.ev, L.t, step, attempt, c, c, k, r, PLIS_EVENT_LEAP_REACTION);
-          if constexpr (SM) {
-#pragma unroll
-            for (int sp = 0; sp < MAXS; ++sp) {
-              const int nu = A.sm.nu[r][sp];
-              if (nu != 0) {
-                const long long v = k * (long long)nu;
-                if (v >= kBigDraw || v <= -kBigDraw) big = 1;
-                dl.v[sp] += v;
-              }
-            }
-          } else {
-            const int nn = m.n_net[r];
-            for (int q = 0; q < nn; ++q) {
-              const long long v = k * (long long)m.net_nu[r * 8 + q];
-              if (v >= kBigDraw || v <= -kBigDraw) big = 1;
-              dl.add(m.net_s[r * 8 + q], v);
-            }
+          const int nn = m.n_net[r];
+          for (int q = 0; q < nn; ++q) {
+            const long long v = k * (long long)m.net_nu[r * 8 + q];
+            if (v >= kBigDraw || v <= -kBigDraw) big = 1;
+            dl.add(m.net_s[r * 8 + q], v);
           }
         }
       };
-      if constexpr (SM) {
-#pragma unroll
-        for (int r0 = 0; r0 < kSmallR; r0 += 4)
-          if (r0 < R) reaction_group(r0);
-      } else {
-        for (int r0 = 0; r0 < R; r0 += 4) reaction_group(r0);
-      }
+      for (int r0 = 0; r0 < R; r0 += 4) reaction_group(r0);
       Nbr q;
       if (WALK && m.lattice) nbr_scalars(m, cl, q);  // walked by direction below: no slot arrays
       else nbr_info(m, cl, q);
@@ -1191,10 +1022,7 @@ __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const L
         }
       };
       auto species_lam = [&](const int s) -> Real {
-        Real dr;
-        if constexpr (SM) dr = sm_drate<Real>(A.sm, s);
-        else dr = drate<Real>(m, comp, s);
-        return tl * (dr * (Real)x.get(s));
+        return tl * (drate<Real>(m, comp, s) * (Real)x.get(s));
       };
       auto species_jumps = [&](const int s) {
         const int32_t xs = x.get(s);
@@ -1237,14 +1065,8 @@ __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const L
         dl.add(s, -out);
         ev += out;
       };
-      if constexpr (SM) {
-#pragma unroll
-        for (int s = 0; s < MAXS; ++s)
-          if (s < S) species_jumps(s);
-      } else {
-        for (int s = 0; s < S; ++s) species_jumps(s);
-      }
-      if constexpr (!SM) {
+      for (int s = 0; s < S; ++s) species_jumps(s);
+      {
         if (pool > (Real)0) {  // the pool's events: total by inversion, then one walk per event
           const plis_stream g =
               plis_stream_make(A.o.seed, A.o.replica, c, PLIS_PHASE_LEAP, step, attempt, PLIS_CH_POOL);
@@ -1364,15 +1186,7 @@ __device__ __forceinline__ void leap_tile(const KArgs& A, uint32_t tile, const L
   }
 }
 
-template <typename Real, int MAXS, bool LOG, bool SM>
-__global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap(KArgs A) {
-  pdl_entry();
-  Ctrl* K = A.b.ctrl;
-  if (K->done) return;
-  extern __shared__ int32_t s_box[];
-  __shared__ long long s_ev[32];
-  __shared__ int s_big;
-  if (threadIdx.x == 0) s_big = 0;
+__device__ __forceinline__ LeapCtx leap_ctx(const KArgs& A, const Ctrl* K) {
   LeapCtx L;
   L.Xc = A.b.X[K->cur];
   L.Xt = A.b.X[K->tgt];
@@ -1381,6 +1195,49 @@ __global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap(KArgs A) {
   L.attempt = K->attempt;
   L.t = K->t;
   L.ff_free = K->ff_free != 0;
+  return L;
+}
+
+// events and guard flags of the CTA into the control block
+__device__ __forceinline__ void leap_totals(Ctrl* K, long long ev, int big) {
+  __shared__ long long s_ev[32];
+  const int any_big = __any_sync(0xffffffffu, big);
+  ev = warp_sum(ev);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) {
+    s_ev[wid] = ev;
+    if (any_big) atomicOr(&K->blocks_done, 0x80000000u);  // rare: a draw beyond the int32 guards
+  }
+  __syncthreads();
+  if (wid == 0) {
+    const int nw = (blockDim.x + 31) >> 5;
+    long long v = lane < nw ? s_ev[lane] : 0;
+    v = warp_sum(v);
+    if (lane == 0 && v) atomicAdd(&K->ev_attempt, (unsigned long long)v);
+  }
+}
+
+template <typename Real, int MAXS, bool LOG, bool LAT>
+__global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap_small(const __grid_constant__ KArgs A) {
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  const int done = K->done;
+  const LeapCtx L = leap_ctx(A, K);
+  const Real tl = (Real)K->tau_leap;
+  if (done) return;
+  long long ev;
+  int big;
+  leap_tile_small<Real, MAXS, LOG, LAT, true>(A, A.sm, blockIdx.x, L, tl, ev, big);
+  leap_totals(K, ev, big);
+}
+
+template <typename Real, int MAXS, bool LOG>
+__global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap(KArgs A) {
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  if (K->done) return;
+  extern __shared__ int32_t s_box[];
+  const LeapCtx L = leap_ctx(A, K);
   const Real tl = (Real)K->tau_leap;
   Box box;
   box.acc = A.g.staged ? s_box : nullptr;
@@ -1388,25 +1245,10 @@ __global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap(KArgs A) {
   box.by = (int)A.g.ty + 2;
   box.bz = (int)A.g.tz + 2;
   box.size = box.bx * box.by * box.bz;
-  __syncthreads();
   long long ev;
   int big;
-  leap_tile<Real, MAXS, LOG, true, SM, true>(A, blockIdx.x, L, tl, box, ev, big);
-  // events and guard flags of the CTA
-  ev = warp_sum(ev);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (big) s_big = 1;
-  if (lane == 0) s_ev[wid] = ev;
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    long long v = lane < nw ? s_ev[lane] : 0;
-    v = warp_sum(v);
-    if (lane == 0) {
-      if (v) atomicAdd(&K->ev_attempt, (unsigned long long)v);
-      if (s_big) atomicOr(&K->blocks_done, 0x80000000u);
-    }
-  }
+  leap_tile<Real, MAXS, LOG, true, true>(A, blockIdx.x, L, tl, box, ev, big);
+  leap_totals(K, ev, big);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1750,15 +1592,15 @@ __device__ __forceinline__ ClassifyCtx classify_ctx(const KArgs& A, const Ctrl* 
 }
 
 // One thread's subvolume of one brick: negativity check, zeroing of the next target, classification.
-template <typename Real, int MAXS, bool WALK = true, bool CACHE = false, bool SM = false>
+template <typename Real, int MAXS, bool WALK = true, bool CACHE = false>
 __device__ __forceinline__ void classify_tile(const KArgs& A, uint32_t tile, const ClassifyCtx& C, double& tn,
-                                              long long& ti, int& fl, int& bad, bool& valid, Real* pc = nullptr) {
+                                              uint32_t& ti, int& fl, int& bad, bool& valid, Real* pc = nullptr) {
   const DevModel& m = A.m;
   Cell cl;
   valid = cell_of(A, tile, cl);
   const uint32_t c = cl.c;
   tn = PLIS_INF_D;
-  ti = 0x7FFFFFFFFFFFFFFFll;
+  ti = kNoCell;
   fl = F_SSA_FF;
   bad = 0;
   if (!valid) return;
@@ -1773,39 +1615,93 @@ __device__ __forceinline__ void classify_tile(const KArgs& A, uint32_t tile, con
   Nbr q;
   if constexpr (WALK) nbr_lite(m, cl, q);
   else nbr_info(m, cl, q);
-  classify_cell<Real, WALK, CACHE, SM>(A, c, q, x, C.Xe, C.tau_cur[c], C.flag_cur[c], C.step, C.attempt, C.ff, tn, fl,
+  classify_cell<Real, WALK, CACHE>(A, c, q, x, C.Xe, C.tau_cur[c], C.flag_cur[c], C.step, C.attempt, C.ff, tn, fl,
                                        CACHE ? pc + threadIdx.x : nullptr, blockDim.x);
   C.tau_new[c] = tn;
   C.flag_new[c] = (uint8_t)fl;
   ti = c;
 }
 
-// CTA reduction of one brick into slot `slot` (min tau with arg-min, #LEAP_CR, negative flag), then
-// the count of finished bricks; true in the CTA that finished last of `nslots`.
+// The same for a small model (small_step.cuh).
+template <typename Real, int MAXS, bool LAT>
+__device__ __forceinline__ void classify_tile_small(const KArgs& A, const SmallModel& t, uint32_t tile, const ClassifyCtx& C,
+                                                    double& tn, uint32_t& ti, int& fl, int& bad, bool& valid) {
+  const DevModel& m = A.m;
+  Cell cl;
+  valid = cell_of(A, tile, cl);
+  const uint32_t c = cl.c;
+  tn = PLIS_INF_D;
+  ti = kNoCell;
+  fl = F_SSA_FF;
+  bad = 0;
+  if (!valid) return;
+  const double tau_cur = C.tau_cur[c];
+  const uint8_t flag_cur = C.flag_cur[c];
+  int32_t x[MAXS];
+#pragma unroll
+  for (int s = 0; s < MAXS; ++s) x[s] = s < (int)m.S ? C.Xe[(size_t)s * m.Npad + c] : 0;
+#pragma unroll
+  for (int s = 0; s < MAXS; ++s)
+    if (s < (int)m.S) {
+      if (x[s] < 0) bad = 1;
+      C.Xz[(size_t)s * m.Npad + c] = 0;
+    }
+  if (!classify_ff(A.o.mode, tau_cur, flag_cur, C.step, C.ff, tn, fl)) {
+    Real tau_ncr, rate;
+    small_tau_parts<Real, MAXS, LAT>(A, t, cl, x, C.Xe, tau_ncr, rate);
+    cell_decide((double)tau_ncr, cell_tau_cr<Real>(A, c, C.step, C.attempt, rate), tn, fl);
+  }
+  C.tau_new[c] = tn;
+  C.flag_new[c] = (uint8_t)fl;
+  ti = c;
+}
+
+// CTA reduction of one brick into slot `slot` (min tau with arg-min, with PLAIN the min of the plain
+// taus tp, #LEAP_CR, #SSA_FF, negative flag), then the count of finished bricks; true in the CTA that
+// finished last of `nslots`.  Two CTA barriers: after the warps' partial results, and for the verdict.
+template <bool PLAIN>
 __device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t slot, uint32_t nslots, double tn,
-                                              long long ti, bool is_cr, int bad, bool is_ff) {
-  __shared__ double s_t[32];
-  __shared__ long long s_i[32];
+                                              uint32_t ti, double tp, bool is_cr, int bad, bool is_ff) {
+  __shared__ uint64_t s_k[32];
+  __shared__ double s_p[32];
+  __shared__ uint32_t s_i[32], s_c[32];
   __shared__ bool s_last;
-  const int ncr = __syncthreads_count(is_cr);
-  const int nff = __syncthreads_count(is_ff);
-  const int nbad = __syncthreads_or(bad);
-  warp_min_pair(tn, ti);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { s_t[wid] = tn; s_i[wid] = ti; }
+  uint64_t k = tau_key(tn);
+  uint32_t crff = (uint32_t)__popc(__ballot_sync(0xffffffffu, is_cr)) |
+                  ((uint32_t)__popc(__ballot_sync(0xffffffffu, is_ff)) << 15);
+  crff |= __any_sync(0xffffffffu, bad) ? 0x80000000u : 0u;
+  warp_min_key(k, ti);
+  if constexpr (PLAIN) tp = warp_min_d(tp);
+  if (lane == 0) {
+    s_k[wid] = k;
+    s_i[wid] = ti;
+    s_c[wid] = crff;
+    if constexpr (PLAIN) s_p[wid] = tp;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double bt = s_t[0];
-    long long bi = s_i[0];
-    for (int w = 1; w < nw; ++w) min_pair(bt, bi, s_t[w], s_i[w]);
-    A.b.slot_tau[slot] = bt;
-    A.b.slot_idx[slot] = bi;
-    A.b.slot_cr[slot] = (uint32_t)ncr | ((uint32_t)nff << 16);  // #LEAP_CR | #SSA_FF << 16 (<= 1024 each)
-    A.b.slot_bad[slot] = nbad ? 1u : 0u;
-    __threadfence();
-    const uint32_t prev = atomicAdd(&K->blocks_done, 1u);
-    s_last = ((prev & 0x7FFFFFFFu) == nslots - 1);
+  if (wid == 0) {
+    const bool on = lane < (int)((blockDim.x + 31) >> 5);
+    k = on ? s_k[lane] : ~0ull;
+    ti = on ? s_i[lane] : kNoCell;
+    crff = on ? s_c[lane] : 0u;
+    const bool nbad = __any_sync(0xffffffffu, (crff >> 31) != 0u);
+    crff = __reduce_add_sync(0xffffffffu, crff & 0x7fffffffu);  // two counts of at most 1024, 15 bits apart
+    warp_min_key(k, ti);
+    if constexpr (PLAIN) tp = warp_min_d(on ? s_p[lane] : PLIS_INF_D);
+    if (lane == 0) {
+      SlotRec q;
+      q.tau = key_tau(k);
+      q.tau_plain = PLAIN ? tp : PLIS_INF_D;
+      q.idx = ti;
+      q.crff = (crff & 0x7fffu) | ((crff >> 15) << 16);
+      q.bad = nbad ? 1u : 0u;
+      q.pad_ = 0;
+      A.b.slot[slot] = q;
+      __threadfence();
+      const uint32_t prev = atomicAdd(&K->blocks_done, 1u);
+      s_last = ((prev & 0x7FFFFFFFu) == nslots - 1);
+    }
   }
   __syncthreads();
   return s_last;
@@ -1819,115 +1715,114 @@ __device__ __forceinline__ void step_decide(const KArgs& A, Ctrl* K, uint32_t ph
                                             unsigned long long gcr, unsigned long long gff, uint32_t bad, double gp,
                                             bool learned, uint32_t am_flag) {
   const int mode = A.o.mode;
-  K->learned = learned ? 1u : 0u;
+  Ctrl k = *K;
+  k.blocks_done = 0;  // changed by the other CTAs since this one's first reads
+  k.n_touched = 0;
+  k.learned = learned ? 1u : 0u;
   if (phase == 0) {
-    K->tau_min = gt;
-    K->tau_min_plain = gp;
-    K->argmin = gi;
-    K->n_leap_cr = (uint32_t)gcr;
-    K->ff_free = gff == 0 ? 1u : 0u;
-    K->argmin_flag = am_flag;
-    K->tf = tf ^ 1u;
-    K->phase = 1;
-    K->done = 1;  // idle until a run call
+    k.tau_min = gt;
+    k.tau_min_plain = gp;
+    k.argmin = gi;
+    k.n_leap_cr = (uint32_t)gcr;
+    k.ff_free = gff == 0 ? 1u : 0u;
+    k.argmin_flag = am_flag;
+    k.tf = tf ^ 1u;
+    k.phase = 1;
+    k.done = 1;  // idle until a run call
   } else if (bad) {  // check_state + revert (leap.cu:203-212, driver.cu:292-315)
-    K->attempt += 1;
-    if ((int)K->attempt > A.o.max_rollbacks) {
-      K->status = PLIS_ERR_STUCK;
-      K->stop_reason = PLIS_STOP_ERROR;
-      K->done = 1;
+    k.attempt += 1;
+    if ((int)k.attempt > A.o.max_rollbacks) {
+      k.status = PLIS_ERR_STUCK;
+      k.stop_reason = PLIS_STOP_ERROR;
+      k.done = 1;
     } else {
-      const uint32_t t = K->tgt;
-      K->tgt = K->spare;
-      K->spare = t;
-      set_attempt(K, mode);
+      const uint32_t t = k.tgt;
+      k.tgt = k.spare;
+      k.spare = t;
+      set_attempt(k, mode);
     }
   } else {
     // accept: swap state (driver.cu:320-323) by rotating buffer indices
-    K->t = K->t + K->dt;
-    K->step = K->step + 1;
-    K->events += K->ev_attempt;
-    K->exact_events += K->ex_attempt;
-    K->rollbacks += K->attempt;
-    K->last_tau = K->tau_min;
-    K->last_argmin = K->argmin;
-    const uint32_t oc = K->cur;
-    K->cur = K->tgt;
-    K->tgt = K->spare;
-    K->spare = oc;
-    K->tf = tf ^ 1u;
-    K->tau_min = gt;
-    K->tau_min_plain = gp;
-    K->argmin = gi;
-    K->n_leap_cr = (uint32_t)gcr;
-    K->ff_free = gff == 0 ? 1u : 0u;
-    K->argmin_flag = am_flag;
-    prepare_step(K, mode);
+    k.t = k.t + k.dt;
+    k.step = k.step + 1;
+    k.events += k.ev_attempt;
+    k.exact_events += k.ex_attempt;
+    k.rollbacks += k.attempt;
+    k.last_tau = k.tau_min;
+    k.last_argmin = k.argmin;
+    const uint32_t oc = k.cur;
+    k.cur = k.tgt;
+    k.tgt = k.spare;
+    k.spare = oc;
+    k.tf = tf ^ 1u;
+    k.tau_min = gt;
+    k.tau_min_plain = gp;
+    k.argmin = gi;
+    k.n_leap_cr = (uint32_t)gcr;
+    k.ff_free = gff == 0 ? 1u : 0u;
+    k.argmin_flag = am_flag;
+    prepare_step(k, mode);
   }
+  *K = k;
 }
 
 // The whole last CTA: reduce the `nslots` slots (independent L2 loads spread over the block), then
 // one thread takes the step decision (driver.cu:267-334): rollback or accept, time, the next plan.
 __device__ __forceinline__ void classify_control(const KArgs& A, Ctrl* K, uint32_t nslots) {
-  __shared__ double s_t[32];
-  __shared__ long long s_i[32];
-  __shared__ unsigned long long s_cr[32];
-  __shared__ unsigned long long s_ff[32];
-  __shared__ uint32_t s_bad[32];
+  __shared__ uint64_t s_k[32];
   __shared__ double s_p[32];
+  __shared__ uint32_t s_i[32], s_cr[32], s_ff[32], s_bad[32];
   __threadfence();
-  const uint32_t phase = K->phase;
-  const uint32_t tf = K->tf;
-  const uint8_t* flag_new = A.b.flag[tf ^ 1u];
-  double gt = PLIS_INF_D;
-  long long gi = 0x7FFFFFFFFFFFFFFFll;
-  unsigned long long gcr = 0, gff = 0;
-  uint32_t gbad = 0;
-  double gp = PLIS_INF_D;  // learned classification: min of the plain taus
-  const double* sp = A.b.slot_tau_plain;
+  const bool plain = A.b.lp != nullptr;  // learned classification: the min of the plain taus too
+  uint64_t gk = tau_key(PLIS_INF_D);
+  uint32_t gi = kNoCell, gcr = 0, gff = 0, gbad = 0;
+  double gp = PLIS_INF_D;
+#pragma unroll 4
   for (uint32_t b = threadIdx.x; b < nslots; b += blockDim.x) {
-    min_pair(gt, gi, __ldcg(&A.b.slot_tau[b]), __ldcg(&A.b.slot_idx[b]));
-    const uint32_t sc = __ldcg(&A.b.slot_cr[b]);
-    gcr += sc & 0xFFFFu;
-    gff += sc >> 16;
-    gbad |= __ldcg(&A.b.slot_bad[b]);
-    if (sp) gp = fmin(gp, __ldcg(&sp[b]));
+    const uint4* q = reinterpret_cast<const uint4*>(A.b.slot + b);
+    const uint4 u = __ldcg(q), v = __ldcg(q + 1);
+    min_key(gk, gi, tau_key(__hiloint2double((int)u.y, (int)u.x)), v.x);
+    gp = fmin(gp, __hiloint2double((int)u.w, (int)u.z));
+    gcr += v.y & 0xFFFFu;
+    gff += v.y >> 16;
+    gbad |= v.z;
   }
-  warp_min_pair(gt, gi);
-  gcr = (unsigned long long)warp_sum((long long)gcr);
-  gff = (unsigned long long)warp_sum((long long)gff);
-  gbad = __reduce_or_sync(0xffffffffu, gbad);
-  if (sp) gp = warp_min_d(gp);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { s_t[wid] = gt; s_i[wid] = gi; s_cr[wid] = gcr; s_ff[wid] = gff; s_bad[wid] = gbad; s_p[wid] = gp; }
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    gt = lane < nw ? s_t[lane] : PLIS_INF_D;
-    gi = lane < nw ? s_i[lane] : 0x7FFFFFFFFFFFFFFFll;
-    gcr = lane < nw ? s_cr[lane] : 0ull;
-    gff = lane < nw ? s_ff[lane] : 0ull;
-    gbad = lane < nw ? s_bad[lane] : 0u;
-    gp = lane < nw ? s_p[lane] : PLIS_INF_D;
-    warp_min_pair(gt, gi);
-    gcr = (unsigned long long)warp_sum((long long)gcr);
-    gff = (unsigned long long)warp_sum((long long)gff);
+  for (int round = 0; round < 2; ++round) {  // the warps, then their results in warp 0
+    warp_min_key(gk, gi);
+    gcr = __reduce_add_sync(0xffffffffu, gcr);
+    gff = __reduce_add_sync(0xffffffffu, gff);
     gbad = __reduce_or_sync(0xffffffffu, gbad);
-    if (sp) gp = warp_min_d(gp);
+    if (plain) gp = warp_min_d(gp);
+    if (round) break;
+    if (lane == 0) { s_k[wid] = gk; s_i[wid] = gi; s_cr[wid] = gcr; s_ff[wid] = gff; s_bad[wid] = gbad; s_p[wid] = gp; }
+    __syncthreads();
+    if (wid != 0) return;
+    const bool on = lane < (int)((blockDim.x + 31) >> 5);
+    gk = on ? s_k[lane] : ~0ull;
+    gi = on ? s_i[lane] : kNoCell;
+    gcr = on ? s_cr[lane] : 0u;
+    gff = on ? s_ff[lane] : 0u;
+    gbad = on ? s_bad[lane] : 0u;
+    gp = on ? s_p[lane] : PLIS_INF_D;
   }
-  if (threadIdx.x == 0) {
+  if (lane == 0) {
+    const uint32_t phase = K->phase;
+    const uint32_t tf = K->tf;
+    const uint8_t* flag_new = A.b.flag[tf ^ 1u];
     const uint32_t leap_bad = (__ldcg(&K->blocks_done) & 0x80000000u) ? 1u : 0u;
-    K->blocks_done = 0;
-    if (gi == 0x7FFFFFFFFFFFFFFFll) gi = -1;
-    const uint32_t am_flag = gi >= 0 ? __ldcg(&flag_new[gi]) : F_SSA_FF;
+    const long long am = gi == kNoCell ? -1ll : (long long)gi;
+    const uint32_t am_flag = am >= 0 ? __ldcg(&flag_new[am]) : F_SSA_FF;
+    const double gt = key_tau(gk);
     if (A.sl.on) {  // a z-slab: the decision waits for every slab's summary (k_slab_control)
       SlabSummary q;
-      q.tau = gt; q.idx = gi; q.tau_plain = gp; q.ncr = gcr; q.nff = gff; q.bad = gbad; q.leap_bad = leap_bad;
+      q.tau = gt; q.idx = am; q.tau_plain = gp; q.ncr = gcr; q.nff = gff; q.bad = gbad; q.leap_bad = leap_bad;
       q.am_flag = am_flag; q.pad_ = 0;
       *A.sl.summary = q;
+      K->blocks_done = 0;
       return;
     }
-    step_decide(A, K, phase, tf, gt, gi, gcr, gff, gbad | leap_bad, gp, sp != nullptr, am_flag);
+    step_decide(A, K, phase, tf, gt, am, gcr, gff, gbad | leap_bad, gp, plain, am_flag);
   }
 }
 
@@ -1936,7 +1831,24 @@ __device__ __forceinline__ void classify_control(const KArgs& A, Ctrl* K, uint32
 #ifndef PLIS_CLASSIFY_MIN_BLOCKS
 #define PLIS_CLASSIFY_MIN_BLOCKS 4
 #endif
-template <typename Real, int MAXS, bool CACHE, bool SM>
+template <typename Real, int MAXS, bool LAT>
+__global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify_small(const __grid_constant__ KArgs A) {
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  const int done = K->done;
+  const ClassifyCtx C = classify_ctx(A, K);
+  if (blockIdx.x == 0 && threadIdx.x == 0) K->n_touched = 0;  // k_apply has consumed the list
+  if (done) return;
+  double tn;
+  uint32_t ti;
+  int fl, bad;
+  bool valid;
+  classify_tile_small<Real, MAXS, LAT>(A, A.sm, blockIdx.x, C, tn, ti, fl, bad, valid);
+  if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
+    classify_control(A, K, gridDim.x);
+}
+
+template <typename Real, int MAXS, bool CACHE>
 __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify(KArgs A) {
   extern __shared__ __align__(16) unsigned char s_prop[];  // CACHE: R x blockDim propensities
   pdl_entry();
@@ -1945,11 +1857,11 @@ __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify(KArg
   if (K->done) return;
   const ClassifyCtx C = classify_ctx(A, K);
   double tn;
-  long long ti;
+  uint32_t ti;
   int fl, bad;
   bool valid;
-  classify_tile<Real, MAXS, true, CACHE, SM>(A, blockIdx.x, C, tn, ti, fl, bad, valid, reinterpret_cast<Real*>(s_prop));
-  if (classify_slot(A, K, blockIdx.x, gridDim.x, tn, ti, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
+  classify_tile<Real, MAXS, true, CACHE>(A, blockIdx.x, C, tn, ti, fl, bad, valid, reinterpret_cast<Real*>(s_prop));
+  if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
     classify_control(A, K, gridDim.x);
 }
 
@@ -2112,27 +2024,25 @@ template <typename Real, int MAXS>
 struct KernelSet {
   static constexpr bool kSmallOk = MAXS <= kSmallS;  // small-model kernels exist for these species counts
   // the event-log variants (LOG = true) only when the handle's log is on: the plain path carries no logging code
-  static void leap(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
+  template <bool LOG>
+  static void leap_log(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
     if constexpr (kSmallOk) {
       if (a.sm.on) {
-        if (a.b.ev.rec) launch_pdl(k_leap<Real, MAXS, true, true>, g, b, a.g.box_bytes, s, a);
-        else launch_pdl(k_leap<Real, MAXS, false, true>, g, b, a.g.box_bytes, s, a);
+        if (a.m.lattice) launch_pdl(k_leap_small<Real, MAXS, LOG, true>, g, b, 0, s, a);
+        else launch_pdl(k_leap_small<Real, MAXS, LOG, false>, g, b, 0, s, a);
         return;
       }
     }
-    if (a.b.ev.rec) launch_pdl(k_leap<Real, MAXS, true, false>, g, b, a.g.box_bytes, s, a);
-    else launch_pdl(k_leap<Real, MAXS, false, false>, g, b, a.g.box_bytes, s, a);
+    launch_pdl(k_leap<Real, MAXS, LOG>, g, b, a.g.box_bytes, s, a);
+  }
+  static void leap(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
+    if (a.b.ev.rec) leap_log<true>(a, g, b, s);
+    else leap_log<false>(a, g, b, s);
   }
   static cudaError_t leap_smem(int bytes) {
-    cudaError_t e = cudaFuncSetAttribute(k_leap<Real, MAXS, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e = cudaFuncSetAttribute(k_leap<Real, MAXS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_leap<Real, MAXS, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if constexpr (kSmallOk) {
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_leap<Real, MAXS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_leap<Real, MAXS, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    }
+      e = cudaFuncSetAttribute(k_leap<Real, MAXS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e;
   }
   static void exact(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
@@ -2141,17 +2051,18 @@ struct KernelSet {
   }
   static void classify(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
     if constexpr (kSmallOk) {
-      if (a.sm.on) {  // the small-model tables make a propensity cheap: no cache
-        launch_pdl(k_classify<Real, MAXS, false, true>, g, b, 0, s, a);
+      if (a.sm.on) {
+        if (a.m.lattice) launch_pdl(k_classify_small<Real, MAXS, true>, g, b, 0, s, a);
+        else launch_pdl(k_classify_small<Real, MAXS, false>, g, b, 0, s, a);
         return;
       }
     }
     // the cache pays once the grid fills the GPU; on a grid of a few CTAs its extra pass only
     // lengthens each thread's chain (measured: 57 -> 62 us per step on 1,000 subvolumes)
     if (a.m.R <= (uint32_t)kPropCache && g.x >= 148u)
-      launch_pdl(k_classify<Real, MAXS, true, false>, g, b, (size_t)a.m.R * b.x * sizeof(Real), s, a);
+      launch_pdl(k_classify<Real, MAXS, true>, g, b, (size_t)a.m.R * b.x * sizeof(Real), s, a);
     else
-      launch_pdl(k_classify<Real, MAXS, false, false>, g, b, 0, s, a);
+      launch_pdl(k_classify<Real, MAXS, false>, g, b, 0, s, a);
   }
 };
 

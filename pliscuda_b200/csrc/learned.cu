@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) k_learned_pre(KArgs A) {
                              pack_bf16x2(f[6], f[7]));
   }
   const int nbad = __syncthreads_or(bad);
-  if (threadIdx.x == 0) A.b.slot_bad[blockIdx.x] = nbad ? 1u : 0u;
+  if (threadIdx.x == 0) A.b.slot[blockIdx.x].bad = nbad ? 1u : 0u;
 }
 
 __global__ void __launch_bounds__(128) k_mlp_tc(const Ctrl* __restrict__ K, const LearnedParams* __restrict__ P,
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) k_learned_post(KArgs A) {
   const bool valid = cell_of(A, blockIdx.x, cl);
   const uint32_t c = cl.c;
   double tn = PLIS_INF_D, tp = PLIS_INF_D;
-  long long ti = 0x7FFFFFFFFFFFFFFFll;
+  uint32_t ti = kNoCell;
   int fl = F_SSA_FF;
   if (valid) {
     const double2 pr = A.b.pre[c];
@@ -161,9 +161,9 @@ __global__ void __launch_bounds__(256) k_learned_post(KArgs A) {
     C.flag_new[c] = (uint8_t)fl;
     ti = c;
   }
-  const int bad = threadIdx.x == 0 ? (int)A.b.slot_bad[blockIdx.x] : 0;
-  if (classify_slot_learned(A, K, blockIdx.x, gridDim.x, tn, ti, tp, valid && fl == F_LEAP_CR, bad,
-                            valid && fl == F_SSA_FF))
+  const int bad = threadIdx.x == 0 ? (int)A.b.slot[blockIdx.x].bad : 0;
+  if (classify_slot<true>(A, K, blockIdx.x, gridDim.x, tn, ti, tp, valid && fl == F_LEAP_CR, bad,
+                          valid && fl == F_SSA_FF))
     classify_control(A, K, gridDim.x);
 }
 

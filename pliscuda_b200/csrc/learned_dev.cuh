@@ -135,42 +135,6 @@ __device__ __forceinline__ void normalise(const LearnedParams* __restrict__ P, f
 // ------------------------------------------------------------------------------------------------
 // classification with proposals
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool classify_slot_learned(const KArgs& A, Ctrl* K, uint32_t slot, uint32_t nslots,
-                                                      double tn, long long ti, double tp, bool is_cr, int bad,
-                                                      bool is_ff) {
-  __shared__ double s_t[32];
-  __shared__ long long s_i[32];
-  __shared__ double s_p[32];
-  __shared__ bool s_last;
-  const int ncr = __syncthreads_count(is_cr);
-  const int nff = __syncthreads_count(is_ff);
-  const int nbad = __syncthreads_or(bad);
-  warp_min_pair(tn, ti);
-  tp = warp_min_d(tp);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { s_t[wid] = tn; s_i[wid] = ti; s_p[wid] = tp; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    double bt = s_t[0], bp = s_p[0];
-    long long bi = s_i[0];
-    for (int w = 1; w < nw; ++w) {
-      min_pair(bt, bi, s_t[w], s_i[w]);
-      bp = fmin(bp, s_p[w]);
-    }
-    A.b.slot_tau[slot] = bt;
-    A.b.slot_idx[slot] = bi;
-    A.b.slot_tau_plain[slot] = bp;
-    A.b.slot_cr[slot] = (uint32_t)ncr | ((uint32_t)nff << 16);  // #LEAP_CR | #SSA_FF << 16
-    A.b.slot_bad[slot] = nbad ? 1u : 0u;
-    __threadfence();
-    const uint32_t prev = atomicAdd(&K->blocks_done, 1u);
-    s_last = ((prev & 0x7FFFFFFFu) == nslots - 1);
-  }
-  __syncthreads();
-  return s_last;
-}
-
 // The classification of one brick with proposals: the tile's subvolume per thread (features, the
 // warp's MLP by mma.sync, decisions against the proposal and the plain bound), then its CTA slot
 // with the plain min-tau beside the proposed one; true in the CTA that reduces the last slot.  Every
@@ -184,7 +148,7 @@ __device__ __forceinline__ bool learned_classify_tile(const KArgs& A, Ctrl* K, c
   const bool valid = cell_of(A, tile, cl);
   const uint32_t c = cl.c;
   double tn = PLIS_INF_D, tp = PLIS_INF_D;
-  long long ti = 0x7FFFFFFFFFFFFFFFll;
+  uint32_t ti = kNoCell;
   int fl = F_SSA_FF, bad = 0;
   bool ff = false;
   Real tau_ncr = RT<Real>::inf(), rate = (Real)0;
@@ -229,7 +193,7 @@ __device__ __forceinline__ bool learned_classify_tile(const KArgs& A, Ctrl* K, c
     C.flag_new[c] = (uint8_t)fl;
     ti = c;
   }
-  return classify_slot_learned(A, K, tile, nslots, tn, ti, tp, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF);
+  return classify_slot<true>(A, K, tile, nslots, tn, ti, tp, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF);
 }
 
 }  // namespace plis
