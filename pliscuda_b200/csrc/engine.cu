@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -127,6 +128,61 @@ bool fill_small_model(const Model& M, const double* rrate, const double* drate, 
     sm.drate_f[s] = (float)drate[s];
   }
   sm.on = 1;
+  return true;
+}
+
+// NetTab of a model that fits it, false otherwise: sizes, thresholds exact in binary32, jump rates as
+// for a small model, compartments in five bits.
+template <typename Real>
+static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* out) {
+  const ReactionTables& t = M.rt;
+  if (M.R > (uint32_t)kNetR || M.S > (uint32_t)kNetS || M.C > 32u) return false;
+  const int64_t nc = opt.critical_threshold, most = 1 << 24;
+  if (nc > most || nc < -most || t.sp_r.size() > (size_t)kNetE) return false;
+  const double lo = sizeof(Real) == 4 ? 1e-25 : 1e-250, hi = sizeof(Real) == 4 ? 1e25 : 1e250;
+  for (double d : M.drate)
+    if (d != 0.0 && !(d >= lo && d <= hi)) return false;
+  NetTab<Real>& n = *out;
+  std::memset(&n, 0, sizeof n);
+  uint32_t e = 0;
+  for (uint32_t r = 0; r < M.R; ++r) {
+    n.nr[r] = t.n_reac[r];
+    for (int i = 0; i < 3; ++i) n.thr[r][i] = -std::numeric_limits<Real>::infinity();
+    for (int i = 0; i < t.n_reac[r]; ++i) {
+      const uint32_t s = t.reac_s[r * kMaxReactantSpecies + i];
+      const int64_t nu = t.reac_nu[r * kMaxReactantSpecies + i];
+      n.re[r][i] = s | (uint32_t)t.reac_m[r * kMaxReactantSpecies + i] << 8;
+      n.rmask[s] |= 1u << r;
+      int64_t thr = INT64_MIN;  // as in fill_small_model
+      if (opt.mode == PLIS_MODE_REFERENCE) {
+        if (i < 2) thr = nu < 0 ? std::max<int64_t>(1, -nu * nc) : 1;
+      } else if (nu < 0) {
+        thr = -nu * nc;
+      }
+      if (thr > most) return false;
+      if (thr > -most) n.thr[r][i] = (Real)thr;
+    }
+    n.rate[r] = (Real)M.rrate[r];
+    n.inv_denom[r] = (Real)t.inv_denom[r];
+    n.net_off[r] = e;
+    for (int i = 0; i < t.n_net[r]; ++i, ++e) {
+      if (e >= (uint32_t)kNetE) return false;
+      n.net_s[e] = t.net_s[r * kMaxNet + i];
+      n.net_nu[e] = t.net_nu[r * kMaxNet + i];
+    }
+  }
+  n.net_off[M.R] = e;
+  for (uint32_t s = 0; s < M.S; ++s) {
+    n.drate[s] = (Real)M.drate[s];
+    n.hor[s] = t.hor[s];
+    n.hmult[s] = t.hmult[s];
+  }
+  for (uint32_t s = 0; s <= M.S; ++s) n.sp_off[s] = t.sp_off[s];
+  for (size_t i = 0; i < t.sp_r.size(); ++i) {
+    n.sp_r[i] = t.sp_r[i];
+    n.sp_nu[i] = (Real)t.sp_nu[i];
+    n.sp_nu2[i] = (Real)((int)t.sp_nu[i] * (int)t.sp_nu[i]);
+  }
   return true;
 }
 
@@ -277,6 +333,10 @@ int Engine::create(const Model& model, const plis_options& opt) {
   if (o.pool || opt.stage_halo) args_.sm.on = 0;  // pooled draws and the staged box live in the generic leap only
 
   launch_ = (opt.precision == PLIS_PREC_FP32) ? pick_f32(M.S) : pick_f64(M.S);
+  if (!args_.sm.on && !opt.stage_halo) {
+    o.net = opt.precision == PLIS_PREC_FP32 ? fill_net_tab(M, opt, &args_.net.f) : fill_net_tab(M, opt, &args_.net.d);
+    if (o.net) PLIS_CU(launch_.net_smem());
+  }
   // shared-memory staging of the leap's brick + halo (lattices only, when the box fits)
   g.staged = 0;
   g.box_bytes = 0;

@@ -130,6 +130,7 @@ struct DevOpts {
   unsigned long long seed;
   uint32_t replica;
   uint32_t pool;      // 1: pooled draws of small-mean channels in the generic leap (plis_stream.h)
+  uint32_t net;       // 1: the arguments are a NetArgs with filled tables
   uint32_t rk0[10], rk1[10];  // Philox round keys of (seed, replica): plis_round_keys, set with devopts_keys
 };
 
@@ -197,6 +198,25 @@ struct SmallModel {
   float drate_f[kSmallS];
 };
 
+// The tables of a network of at most kNetR reactions, kNetS species and kNetE table entries, in the
+// working precision, held in the kernel arguments of the single-replica kernels (net_step.cuh): values
+// of DevModel's tables (same order of summation), read through the constant bank.
+constexpr int kNetR = 32, kNetS = 16, kNetE = 128;
+template <typename Real> struct NetTab {
+  uint32_t nr[kNetR];            // distinct reactant species of reaction r
+  uint32_t re[kNetR][3];         // species | multiplicity << 8, species increasing
+  Real thr[kNetR][3];            // reaction r is critical while that species counts less than this (-inf: never)
+  Real rate[kNetR], inv_denom[kNetR];
+  Real drate[kNetS];             // rate and drate: one set of rate constants (several: DevModel's rr and dr)
+  int32_t hor[kNetS], hmult[kNetS];
+  uint32_t rmask[kNetS];         // bit r: species s is a reactant of reaction r
+  uint32_t sp_off[kNetS + 1];    // the reactions that change species s, with nu and nu^2
+  uint32_t sp_r[kNetE];
+  Real sp_nu[kNetE], sp_nu2[kNetE];
+  uint32_t net_off[kNetR + 1];   // the species that reaction r changes
+  int32_t net_s[kNetE], net_nu[kNetE];
+};
+
 // z-slab decomposition: this handle computes the subvolumes of whole z-layers [z0, z1) of a lattice
 // whose other layers belong to other ranks.  Arrays stay full size and indices global, so random
 // streams, neighbour counts and the arg-min tie rule are those of a single domain; the kernels touch
@@ -240,6 +260,14 @@ struct KArgs {
   Geo g;
   SmallModel sm;
   SlabArgs sl;
+};
+
+// the argument block of a single-replica handle: with the tables of a network when o.net is set
+struct NetArgs : KArgs {
+  union {
+    NetTab<double> d;
+    NetTab<float> f;
+  } net;
 };
 
 }  // namespace plis

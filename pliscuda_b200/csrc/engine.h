@@ -21,6 +21,7 @@ struct Launchers {
   void (*exact)(const KArgs&, dim3, dim3, cudaStream_t);
   void (*classify)(const KArgs&, dim3, dim3, cudaStream_t);
   cudaError_t (*leap_smem)(int bytes);
+  cudaError_t (*net_smem)();  // shared memory above the default limit for the network kernels
 };
 
 // SmallModel tables of a model (engine.cu); false, with sm->on = 0, when it does not fit.
@@ -70,7 +71,7 @@ class Engine {
 
   Model model_;
   plis_options opt_{};
-  KArgs args_{};
+  NetArgs args_{};
   Launchers launch_{};
   cudaStream_t stream_ = nullptr;
   cudaGraphExec_t graph_exec_ = nullptr;

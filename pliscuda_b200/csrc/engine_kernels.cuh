@@ -527,8 +527,7 @@ __device__ __forceinline__ bool crit_fix(const DevModel& m, const Counts<MAXS>& 
 
 // Cao's g (tau.cu:47-66 for orders <= 2; orders 3 per Cao, Gillespie, Petzold 2006)
 template <typename Real>
-__device__ __forceinline__ Real gfun(int hor, int hmult, int32_t x) {
-  const Real xr = (Real)x;
+__device__ __forceinline__ Real gfun(int hor, int hmult, Real xr) {
   switch (hor) {
     case 0: return RT<Real>::inf();
     case 1: return (Real)1;
@@ -633,7 +632,7 @@ __device__ __forceinline__ void cell_tau_parts(const KArgs& A, uint32_t c, const
     }
     if (!include) continue;
     // compute_tau_sp, tau.cu:68-143
-    const Real g = gfun<Real>(m.hor[s], m.hmult[s], xs);
+    const Real g = gfun<Real>(m.hor[s], m.hmult[s], (Real)xs);
     Real mu = (Real)0, s2 = (Real)0;
     const int p0 = m.sp_off[s], p1 = m.sp_off[s + 1];
     for (int i = p0; i < p1; ++i) {
@@ -1265,6 +1264,34 @@ __device__ __forceinline__ void touch(const KArgs& A, uint32_t c) {
   if (i < A.m.N) touched_list(A)[i] = c;
 }
 
+// The jump of species spi out of LEAP_CR subvolume c, when it had a molecule before the leap (`had`) and has
+// one after it (leap.cu:168-199).
+template <typename Real, bool LOG>
+__device__ __forceinline__ int critical_jump_ref(const KArgs& A, uint32_t c, int spi, bool had, const int32_t* Xt,
+                                                 uint64_t step, uint32_t attempt, int32_t* D, uint8_t* flag) {
+  const DevModel& m = A.m;
+  if (!had || !(Xt[(size_t)spi * m.Npad + c] > 0)) return 0;
+  plis_stream sd = plis_stream_make(A.o.seed, A.o.replica, c, PLIS_PHASE_CRIT, step, attempt, 1);
+  const Real u2 = RT<Real>::uniform(&sd);
+  int slot = (int)(u2 * (Real)6);
+  if (slot > 5) slot = 5;
+  const uint32_t target = canon_slot(m, c, slot);
+  if (target == c) return 0;
+  atomicAdd(&D[(size_t)spi * m.Npad + c], -1);
+  atomicAdd(&D[(size_t)spi * m.Npad + target], 1);
+  touch(A, c);
+  touch(A, target);
+  const uint32_t q = flat_table_entry(m, target);  // leap.cu:192-193
+  if (!A.sl.on || (q + A.sl.has_lo * A.sl.layer >= A.sl.lo && q < A.sl.hi + A.sl.has_hi * A.sl.layer)) {
+    if (flag[q] == F_SSA_FF) flag[q] = F_SSA;
+  } else {  // z-slab: another slab owns q; its owner applies the write after the gather
+    const uint32_t i = atomicAdd(&A.sl.remote->n, 1u);
+    if (i < (uint32_t)kSlabRemote) A.sl.remote->cell[i] = q;
+  }
+  if (LOG) ev_put(A.b.ev, A.b.ctrl->t, step, attempt, c, target, 1, spi, PLIS_EVENT_CRITICAL_DIFFUSION);
+  return 1;
+}
+
 // Reference critical event of one LEAP_CR subvolume (leap.cu:86-199).
 template <typename Real, bool LOG, int MAXS>
 __device__ int critical_event_ref(const KArgs& A, uint32_t c, const Counts<MAXS>& x, const int32_t* Xt,
@@ -1320,27 +1347,7 @@ __device__ int critical_event_ref(const KArgs& A, uint32_t c, const Counts<MAXS>
     if (x.get(spi) < nc) --spic;
   spi = spi - 1;  // leap.cu:160-166
   if (spi < 0) spi = 0;
-  const bool fire = x.get(spi) > 0 && Xt[(size_t)spi * m.Npad + c] > 0;
-  if (!fire) return 0;
-  plis_stream sd = plis_stream_make(A.o.seed, A.o.replica, c, PLIS_PHASE_CRIT, step, attempt, 1);
-  const Real u2 = RT<Real>::uniform(&sd);
-  int slot = (int)(u2 * (Real)6);
-  if (slot > 5) slot = 5;
-  const uint32_t target = canon_slot(m, c, slot);
-  if (target == c) return 0;
-  atomicAdd(&D[(size_t)spi * m.Npad + c], -1);
-  atomicAdd(&D[(size_t)spi * m.Npad + target], 1);
-  touch(A, c);
-  touch(A, target);
-  const uint32_t q = flat_table_entry(m, target);  // leap.cu:192-193
-  if (!A.sl.on || (q + A.sl.has_lo * A.sl.layer >= A.sl.lo && q < A.sl.hi + A.sl.has_hi * A.sl.layer)) {
-    if (flag[q] == F_SSA_FF) flag[q] = F_SSA;
-  } else {  // z-slab: another slab owns q; its owner applies the write after the gather
-    const uint32_t i = atomicAdd(&A.sl.remote->n, 1u);
-    if (i < (uint32_t)kSlabRemote) A.sl.remote->cell[i] = q;
-  }
-  if (LOG) ev_put(A.b.ev, A.b.ctrl->t, step, attempt, c, target, 1, spi, PLIS_EVENT_CRITICAL_DIFFUSION);
-  return 1;
+  return critical_jump_ref<Real, LOG>(A, c, spi, x.get(spi) > 0, Xt, step, attempt, D, flag);
 }
 
 // Exact event of the arg-min subvolume: reference ssa_step (ssa.cu:270-324), or in corrected mode
@@ -1524,6 +1531,91 @@ __global__ void __launch_bounds__(256) k_exact(KArgs A) {
   }
 }
 
+}  // namespace plis
+#include "net_step.cuh"
+namespace plis {
+
+// Binary64 columns of a 10-species, 20-reaction network take 60-72 KB a CTA, so three CTAs share an SM.
+template <typename Real> struct NetCtas { static constexpr int n = sizeof(Real) == 8 ? 3 : 4; };
+
+template <typename Real, bool LOG, bool LAT>
+__global__ void __launch_bounds__(256, NetCtas<Real>::n) k_leap_net(const __grid_constant__ NetArgs A) {
+  extern __shared__ __align__(16) unsigned char s_net[];
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  const int done = K->done;
+  const LeapCtx L = leap_ctx(A, K);
+  const Real tl = (Real)K->tau_leap;
+  if (done) return;
+  long long ev;
+  int big;
+  leap_tile_net<Real, LOG, LAT>(A, net_tab<Real>(A), blockIdx.x, L, tl, reinterpret_cast<Real*>(s_net), ev, big);
+  leap_totals(K, ev, big);
+}
+
+// Exact events (k_exact): a CTA scans up to kNetChunk flags at a time, so that the events of a large
+// lattice are fired in one pass of every CTA, many lanes at once.
+constexpr uint32_t kNetChunk = 4096;
+template <typename Real, bool LOG>
+__global__ void __launch_bounds__(256) k_exact_net(const __grid_constant__ NetArgs A) {
+  extern __shared__ __align__(16) unsigned char s_net[];
+  __shared__ uint16_t s_cell[kNetChunk];
+  __shared__ uint32_t s_n;
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  const uint32_t ex = K->exact;
+  if (K->done || ex == 0) return;
+  const DevModel& m = A.m;
+  const int32_t* Xc = A.b.X[K->cur];
+  int32_t* Xt = A.b.X[K->tgt];
+  uint8_t* flag = A.b.flag[K->tf];
+  const uint64_t step = K->step + 1;
+  const uint32_t attempt = K->attempt;
+  int fired = 0;
+  const uint32_t c_lo = A.sl.on ? A.sl.lo : 0u, c_hi = A.sl.on ? A.sl.hi : m.N;  // a z-slab: its own subvolumes
+  if (ex & 1u) {
+    Real* sx = reinterpret_cast<Real*>(s_net) + threadIdx.x;
+    Real* sa = sx + (size_t)m.S * blockDim.x;
+    const unsigned lane = threadIdx.x & 31u;
+    uint32_t chunk = ((c_hi - c_lo + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
+    if (chunk > kNetChunk) chunk = kNetChunk;
+    for (uint32_t base = c_lo + blockIdx.x * chunk; base < c_hi; base += gridDim.x * chunk) {
+      if (threadIdx.x == 0) s_n = 0;
+      __syncthreads();
+#pragma unroll 4
+      for (uint32_t i = threadIdx.x; i < chunk; i += blockDim.x) {
+        const uint32_t c = base + i;
+        const bool cr = c < c_hi && flag[c] == F_LEAP_CR;
+        const unsigned mask = __ballot_sync(0xffffffffu, cr);
+        unsigned pos = 0;
+        if (lane == 0 && mask) pos = atomicAdd(&s_n, (unsigned)__popc(mask));
+        pos = __shfl_sync(0xffffffffu, pos, 0);
+        if (cr) s_cell[pos + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)i;
+      }
+      __syncthreads();
+      const uint32_t n = s_n;
+      for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
+        fired += critical_event_net<Real, LOG>(A, net_tab<Real>(A), base + s_cell[j], sx, sa, blockDim.x, Xc, Xt, step,
+                                               attempt, A.b.D, flag);
+      __syncthreads();
+    }
+  }
+  if ((ex & 2u) && blockIdx.x == 0 && threadIdx.x == 0 && (uint32_t)K->argmin >= c_lo && (uint32_t)K->argmin < c_hi) {
+    const uint32_t am = (uint32_t)K->argmin;
+    const uint8_t fa = flag[am];
+    int32_t* dst = (ex & 1u) ? A.b.D : Xt;
+    if (fa == F_SSA || fa == F_SSA_FF || (A.o.mode != 0 && fa == F_LEAP_CR)) {
+      Counts<kNetS> x;
+      load_counts(m, Xc, am, x);
+      fired += argmin_event<Real, LOG>(A, am, x, step, attempt, dst, flag, fa == F_LEAP_CR);
+    }
+  }
+  if (fired) {  // exact events are rare: one atomic per firing thread
+    atomicAdd(&K->ev_attempt, (unsigned long long)fired);
+    atomicAdd(&K->ex_attempt, (unsigned long long)fired);
+  }
+}
+
 #ifdef PLIS_ENGINE_HOST_TU
 __global__ void __launch_bounds__(256) k_apply(KArgs A) {
   pdl_entry();
@@ -1649,6 +1741,40 @@ __device__ __forceinline__ void classify_tile_small(const KArgs& A, const SmallM
   if (!classify_ff(A.o.mode, tau_cur, flag_cur, C.step, C.ff, tn, fl)) {
     Real tau_ncr, rate;
     small_tau_parts<Real, MAXS, LAT>(A, t, cl, x, C.Xe, tau_ncr, rate);
+    cell_decide((double)tau_ncr, cell_tau_cr<Real>(A, c, C.step, C.attempt, rate), tn, fl);
+  }
+  C.tau_new[c] = tn;
+  C.flag_new[c] = (uint8_t)fl;
+  ti = c;
+}
+
+// The same for a network with NetTab (net_step.cuh); smem: the CTA's count and propensity columns.
+template <typename Real, bool LAT>
+__device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const ClassifyCtx& C,
+                                                  Real* smem, double& tn, uint32_t& ti, int& fl, int& bad, bool& valid) {
+  const DevModel& m = A.m;
+  const int S = (int)m.S;
+  Cell cl;
+  valid = cell_of(A, tile, cl);
+  const uint32_t c = cl.c;
+  tn = PLIS_INF_D;
+  ti = kNoCell;
+  fl = F_SSA_FF;
+  bad = 0;
+  if (!valid) return;
+  const double tau_cur = C.tau_cur[c];
+  const uint8_t flag_cur = C.flag_cur[c];
+  Real* sx = smem + threadIdx.x;
+#pragma unroll 4
+  for (int s = 0; s < S; ++s) {
+    const int32_t xs = C.Xe[(size_t)s * m.Npad + c];
+    if (xs < 0) bad = 1;
+    sx[s * blockDim.x] = (Real)xs;
+    C.Xz[(size_t)s * m.Npad + c] = 0;
+  }
+  if (!classify_ff(A.o.mode, tau_cur, flag_cur, C.step, C.ff, tn, fl)) {
+    Real tau_ncr, rate;
+    net_tau_parts<Real, LAT>(A, T, cl, sx, sx + (size_t)S * blockDim.x, blockDim.x, C.Xe, tau_ncr, rate);
     cell_decide((double)tau_ncr, cell_tau_cr<Real>(A, c, C.step, C.attempt, rate), tn, fl);
   }
   C.tau_new[c] = tn;
@@ -1848,6 +1974,24 @@ __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify_smal
     classify_control(A, K, gridDim.x);
 }
 
+template <typename Real, bool LAT>
+__global__ void __launch_bounds__(256, NetCtas<Real>::n) k_classify_net(const __grid_constant__ NetArgs A) {
+  extern __shared__ __align__(16) unsigned char s_net[];
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  const int done = K->done;
+  const ClassifyCtx C = classify_ctx(A, K);
+  if (blockIdx.x == 0 && threadIdx.x == 0) K->n_touched = 0;  // k_apply has consumed the list
+  if (done) return;
+  double tn;
+  uint32_t ti;
+  int fl, bad;
+  bool valid;
+  classify_tile_net<Real, LAT>(A, net_tab<Real>(A), blockIdx.x, C, reinterpret_cast<Real*>(s_net), tn, ti, fl, bad, valid);
+  if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
+    classify_control(A, K, gridDim.x);
+}
+
 template <typename Real, int MAXS, bool CACHE>
 __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify(KArgs A) {
   extern __shared__ __align__(16) unsigned char s_prop[];  // CACHE: R x blockDim propensities
@@ -2033,7 +2177,28 @@ struct KernelSet {
         return;
       }
     }
+    if (a.o.net) {
+      const NetArgs& n = static_cast<const NetArgs&>(a);
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, b.x, true);
+      if (a.m.lattice) launch_pdl(k_leap_net<Real, LOG, true>, g, b, bytes, s, n);
+      else launch_pdl(k_leap_net<Real, LOG, false>, g, b, bytes, s, n);
+      return;
+    }
     launch_pdl(k_leap<Real, MAXS, LOG>, g, b, a.g.box_bytes, s, a);
+  }
+  // the largest shared memory any network asks for: one value, so that no handle lowers another's limit
+  static cudaError_t net_smem_limit() {
+    constexpr int leap = (int)net_smem<Real>(kNetS, kNetR, 256, true), rest = (int)net_smem<Real>(kNetS, kNetR, 256, false);
+    const void* leaps[] = {(const void*)k_leap_net<Real, false, false>, (const void*)k_leap_net<Real, false, true>,
+                           (const void*)k_leap_net<Real, true, false>, (const void*)k_leap_net<Real, true, true>};
+    const void* rests[] = {(const void*)k_exact_net<Real, false>, (const void*)k_exact_net<Real, true>,
+                           (const void*)k_classify_net<Real, false>, (const void*)k_classify_net<Real, true>};
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
+      e = cudaFuncSetAttribute(leaps[i], cudaFuncAttributeMaxDynamicSharedMemorySize, leap);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(rests[i], cudaFuncAttributeMaxDynamicSharedMemorySize, rest);
+    }
+    return e;
   }
   static void leap(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
     if (a.b.ev.rec) leap_log<true>(a, g, b, s);
@@ -2046,6 +2211,13 @@ struct KernelSet {
     return e;
   }
   static void exact(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
+    if (a.o.net) {
+      const NetArgs& n = static_cast<const NetArgs&>(a);
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, b.x, false);
+      if (a.b.ev.rec) launch_pdl(k_exact_net<Real, true>, g, b, bytes, s, n);
+      else launch_pdl(k_exact_net<Real, false>, g, b, bytes, s, n);
+      return;
+    }
     if (a.b.ev.rec) launch_pdl(k_exact<Real, MAXS, true>, g, b, 0, s, a);
     else launch_pdl(k_exact<Real, MAXS, false>, g, b, 0, s, a);
   }
@@ -2056,6 +2228,13 @@ struct KernelSet {
         else launch_pdl(k_classify_small<Real, MAXS, false>, g, b, 0, s, a);
         return;
       }
+    }
+    if (a.o.net) {
+      const NetArgs& n = static_cast<const NetArgs&>(a);
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, b.x, false);
+      if (a.m.lattice) launch_pdl(k_classify_net<Real, true>, g, b, bytes, s, n);
+      else launch_pdl(k_classify_net<Real, false>, g, b, bytes, s, n);
+      return;
     }
     // the cache pays once the grid fills the GPU; on a grid of a few CTAs its extra pass only
     // lengthens each thread's chain (measured: 57 -> 62 us per step on 1,000 subvolumes)
@@ -2068,14 +2247,14 @@ struct KernelSet {
 
 template <typename Real>
 Launchers pick_impl(uint32_t S) {
-  if (S <= 1) return {KernelSet<Real, 1>::leap, KernelSet<Real, 1>::exact, KernelSet<Real, 1>::classify, KernelSet<Real, 1>::leap_smem};
-  if (S <= 2) return {KernelSet<Real, 2>::leap, KernelSet<Real, 2>::exact, KernelSet<Real, 2>::classify, KernelSet<Real, 2>::leap_smem};
-  if (S <= 4) return {KernelSet<Real, 4>::leap, KernelSet<Real, 4>::exact, KernelSet<Real, 4>::classify, KernelSet<Real, 4>::leap_smem};
-  if (S <= 8) return {KernelSet<Real, 8>::leap, KernelSet<Real, 8>::exact, KernelSet<Real, 8>::classify, KernelSet<Real, 8>::leap_smem};
-  if (S <= 16) return {KernelSet<Real, 16>::leap, KernelSet<Real, 16>::exact, KernelSet<Real, 16>::classify, KernelSet<Real, 16>::leap_smem};
-  if (S <= 32) return {KernelSet<Real, 32>::leap, KernelSet<Real, 32>::exact, KernelSet<Real, 32>::classify, KernelSet<Real, 32>::leap_smem};
-  if (S <= 64) return {KernelSet<Real, 64>::leap, KernelSet<Real, 64>::exact, KernelSet<Real, 64>::classify, KernelSet<Real, 64>::leap_smem};
-  return {KernelSet<Real, 256>::leap, KernelSet<Real, 256>::exact, KernelSet<Real, 256>::classify, KernelSet<Real, 256>::leap_smem};
+  if (S <= 1) return {KernelSet<Real, 1>::leap, KernelSet<Real, 1>::exact, KernelSet<Real, 1>::classify, KernelSet<Real, 1>::leap_smem, KernelSet<Real, 1>::net_smem_limit};
+  if (S <= 2) return {KernelSet<Real, 2>::leap, KernelSet<Real, 2>::exact, KernelSet<Real, 2>::classify, KernelSet<Real, 2>::leap_smem, KernelSet<Real, 2>::net_smem_limit};
+  if (S <= 4) return {KernelSet<Real, 4>::leap, KernelSet<Real, 4>::exact, KernelSet<Real, 4>::classify, KernelSet<Real, 4>::leap_smem, KernelSet<Real, 4>::net_smem_limit};
+  if (S <= 8) return {KernelSet<Real, 8>::leap, KernelSet<Real, 8>::exact, KernelSet<Real, 8>::classify, KernelSet<Real, 8>::leap_smem, KernelSet<Real, 8>::net_smem_limit};
+  if (S <= 16) return {KernelSet<Real, 16>::leap, KernelSet<Real, 16>::exact, KernelSet<Real, 16>::classify, KernelSet<Real, 16>::leap_smem, KernelSet<Real, 16>::net_smem_limit};
+  if (S <= 32) return {KernelSet<Real, 32>::leap, KernelSet<Real, 32>::exact, KernelSet<Real, 32>::classify, KernelSet<Real, 32>::leap_smem, KernelSet<Real, 32>::net_smem_limit};
+  if (S <= 64) return {KernelSet<Real, 64>::leap, KernelSet<Real, 64>::exact, KernelSet<Real, 64>::classify, KernelSet<Real, 64>::leap_smem, KernelSet<Real, 64>::net_smem_limit};
+  return {KernelSet<Real, 256>::leap, KernelSet<Real, 256>::exact, KernelSet<Real, 256>::classify, KernelSet<Real, 256>::leap_smem, KernelSet<Real, 256>::net_smem_limit};
 }
 
 

@@ -413,7 +413,7 @@ __device__ __forceinline__ void small_tau_parts(const KArgs& A, const SmallModel
     const int32_t* row = Xe + (size_t)s * m.Npad;
 #pragma unroll
     for (int d = 0; d < 6; ++d) xb[d] = (on >> d) & 1u ? row[nb[d]] : 0;
-    const Real g = gfun<Real>(t.hor[s], t.hmult[s], xs);
+    const Real g = gfun<Real>(t.hor[s], t.hmult[s], (Real)xs);
     Real mu = (Real)0, s2 = (Real)0;
 #pragma unroll
     for (int r = 0; r < kSmallR; ++r) {
