@@ -146,13 +146,12 @@ static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* 
   std::memset(&n, 0, sizeof n);
   uint32_t e = 0;
   for (uint32_t r = 0; r < M.R; ++r) {
-    n.nr[r] = t.n_reac[r];
-    for (int i = 0; i < 3; ++i) n.thr[r][i] = -std::numeric_limits<Real>::infinity();
     for (int i = 0; i < t.n_reac[r]; ++i) {
       const uint32_t s = t.reac_s[r * kMaxReactantSpecies + i];
+      const uint32_t mu = t.reac_m[r * kMaxReactantSpecies + i];
       const int64_t nu = t.reac_nu[r * kMaxReactantSpecies + i];
-      n.re[r][i] = s | (uint32_t)t.reac_m[r * kMaxReactantSpecies + i] << 8;
       n.rmask[s] |= 1u << r;
+      n.need[r] |= (s | mu << 5) << (10 * i);
       int64_t thr = INT64_MIN;  // as in fill_small_model
       if (opt.mode == PLIS_MODE_REFERENCE) {
         if (i < 2) thr = nu < 0 ? std::max<int64_t>(1, -nu * nc) : 1;
@@ -160,7 +159,13 @@ static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* 
         thr = -nu * nc;
       }
       if (thr > most) return false;
-      if (thr > -most) n.thr[r][i] = (Real)thr;
+      for (uint32_t j = 0; j < mu; ++j) {
+        if (n.nf[r] == 3) return false;
+        auto& f = n.fac[r][n.nf[r]++];
+        f.off = s * kNetCols * (uint32_t)sizeof(Real);
+        f.j = (Real)j;
+        f.thr = j == 0 && thr > -most ? (Real)thr : -std::numeric_limits<Real>::infinity();
+      }
     }
     n.rate[r] = (Real)M.rrate[r];
     n.inv_denom[r] = (Real)t.inv_denom[r];
@@ -179,9 +184,13 @@ static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* 
   }
   for (uint32_t s = 0; s <= M.S; ++s) n.sp_off[s] = t.sp_off[s];
   for (size_t i = 0; i < t.sp_r.size(); ++i) {
-    n.sp_r[i] = t.sp_r[i];
-    n.sp_nu[i] = (Real)t.sp_nu[i];
-    n.sp_nu2[i] = (Real)((int)t.sp_nu[i] * (int)t.sp_nu[i]);
+    n.sp[i].off = t.sp_r[i] * kNetCols * (uint32_t)sizeof(Real);
+    n.sp[i].nu = (Real)t.sp_nu[i];
+    n.sp[i].nu2 = (Real)((int)t.sp_nu[i] * (int)t.sp_nu[i]);
+  }
+  for (int i = 0; i < 8; ++i) {
+    n.by[i][0] = (Real)i;
+    n.by[i][1] = i ? (Real)1 / (Real)i : (Real)0;
   }
   return true;
 }

@@ -202,19 +202,31 @@ struct SmallModel {
 // working precision, held in the kernel arguments of the single-replica kernels (net_step.cuh): values
 // of DevModel's tables (same order of summation), read through the constant bank.
 constexpr int kNetR = 32, kNetS = 16, kNetE = 128;
+constexpr uint32_t kNetCols = 256;  // columns of a row of the CTA's shared memory (its threads, at most)
 template <typename Real> struct NetTab {
-  uint32_t nr[kNetR];            // distinct reactant species of reaction r
-  uint32_t re[kNetR][3];         // species | multiplicity << 8, species increasing
-  Real thr[kNetR][3];            // reaction r is critical while that species counts less than this (-inf: never)
+  // the propensity of reaction r as a product of up to three factors (count of a species) - j, species
+  // increasing, then j = 0, 1, 2; the first factor of a species carries its critical threshold: the
+  // reaction is critical while the species counts less (-inf: never)
+  struct Factor {
+    uint32_t off;                // byte offset of the species' row
+    Real j, thr;
+  };
+  struct Change {                // reaction r changes a species by nu
+    Real nu, nu2;
+    uint32_t off;                // byte offset of the reaction's row (from the first propensity row)
+  };
+  uint32_t nf[kNetR];
+  Factor fac[kNetR][3];
   Real rate[kNetR], inv_denom[kNetR];
   Real drate[kNetS];             // rate and drate: one set of rate constants (several: DevModel's rr and dr)
   int32_t hor[kNetS], hmult[kNetS];
   uint32_t rmask[kNetS];         // bit r: species s is a reactant of reaction r
-  uint32_t sp_off[kNetS + 1];    // the reactions that change species s, with nu and nu^2
-  uint32_t sp_r[kNetE];
-  Real sp_nu[kNetE], sp_nu2[kNetE];
+  uint32_t sp_off[kNetS + 1];    // the changes of species s: sp[sp_off[s]] .. sp[sp_off[s + 1] - 1]
+  Change sp[kNetE];
   uint32_t net_off[kNetR + 1];   // the species that reaction r changes
   int32_t net_s[kNetE], net_nu[kNetE];
+  uint32_t need[kNetR];          // multiplicities of the reactants: species | multiplicity << 5, 10 bits each
+  Real by[8][2];                 // n and 1/n
 };
 
 // z-slab decomposition: this handle computes the subvolumes of whole z-layers [z0, z1) of a lattice

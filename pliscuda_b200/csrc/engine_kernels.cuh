@@ -1260,7 +1260,11 @@ __device__ __forceinline__ uint32_t* touched_list(const KArgs& A) {
 __device__ __forceinline__ void touch(const KArgs& A, uint32_t c) {
   Ctrl* K = A.b.ctrl;
   if (!K->touched_on) return;
-  const uint32_t i = atomicAdd(&K->n_touched, 1u);
+  namespace cg = cooperative_groups;  // one atomic for the threads that get here together
+  const cg::coalesced_group g = cg::coalesced_threads();
+  uint32_t i = 0;
+  if (g.thread_rank() == 0) i = atomicAdd(&K->n_touched, g.size());
+  i = g.shfl(i, 0) + g.thread_rank();
   if (i < A.m.N) touched_list(A)[i] = c;
 }
 
@@ -1467,6 +1471,15 @@ __device__ int argmin_event(const KArgs& A, uint32_t mcell, const Counts<MAXS>& 
   return 1;
 }
 
+// the events fired by a warp's threads into the control block, one atomic each per warp
+__device__ __forceinline__ void exact_totals(Ctrl* K, int fired) {
+  fired = __reduce_add_sync(0xffffffffu, fired);
+  if ((threadIdx.x & 31) == 0 && fired) {
+    atomicAdd(&K->ev_attempt, (unsigned long long)fired);
+    atomicAdd(&K->ex_attempt, (unsigned long long)fired);
+  }
+}
+
 template <typename Real, int MAXS, bool LOG>
 __global__ void __launch_bounds__(256) k_exact(KArgs A) {
   pdl_entry();
@@ -1525,10 +1538,7 @@ __global__ void __launch_bounds__(256) k_exact(KArgs A) {
       else if (fa == F_SSA || fa == F_SSA_FF) fired += argmin_event<Real, LOG>(A, am, x, step, attempt, dst, flag, false);
     }
   }
-  if (fired) {  // exact events are rare: one atomic per firing thread
-    atomicAdd(&K->ev_attempt, (unsigned long long)fired);
-    atomicAdd(&K->ex_attempt, (unsigned long long)fired);
-  }
+  exact_totals(K, fired);
 }
 
 }  // namespace plis
@@ -1538,8 +1548,8 @@ namespace plis {
 // Binary64 columns of a 10-species, 20-reaction network take 60-72 KB a CTA, so three CTAs share an SM.
 template <typename Real> struct NetCtas { static constexpr int n = sizeof(Real) == 8 ? 3 : 4; };
 
-template <typename Real, bool LOG, bool LAT>
-__global__ void __launch_bounds__(256, NetCtas<Real>::n) k_leap_net(const __grid_constant__ NetArgs A) {
+template <typename Real, bool LOG, bool LAT, bool COMP>
+__global__ void __launch_bounds__(256, 3) k_leap_net(const __grid_constant__ NetArgs A) {
   extern __shared__ __align__(16) unsigned char s_net[];
   pdl_entry();
   Ctrl* K = A.b.ctrl;
@@ -1549,14 +1559,14 @@ __global__ void __launch_bounds__(256, NetCtas<Real>::n) k_leap_net(const __grid
   if (done) return;
   long long ev;
   int big;
-  leap_tile_net<Real, LOG, LAT>(A, net_tab<Real>(A), blockIdx.x, L, tl, reinterpret_cast<Real*>(s_net), ev, big);
+  leap_tile_net<Real, LOG, LAT, COMP>(A, net_tab<Real>(A), blockIdx.x, L, tl, s_net, ev, big);
   leap_totals(K, ev, big);
 }
 
 // Exact events (k_exact): a CTA scans up to kNetChunk flags at a time, so that the events of a large
 // lattice are fired in one pass of every CTA, many lanes at once.
 constexpr uint32_t kNetChunk = 4096;
-template <typename Real, bool LOG>
+template <typename Real, bool LOG, bool COMP>
 __global__ void __launch_bounds__(256) k_exact_net(const __grid_constant__ NetArgs A) {
   extern __shared__ __align__(16) unsigned char s_net[];
   __shared__ uint16_t s_cell[kNetChunk];
@@ -1574,8 +1584,7 @@ __global__ void __launch_bounds__(256) k_exact_net(const __grid_constant__ NetAr
   int fired = 0;
   const uint32_t c_lo = A.sl.on ? A.sl.lo : 0u, c_hi = A.sl.on ? A.sl.hi : m.N;  // a z-slab: its own subvolumes
   if (ex & 1u) {
-    Real* sx = reinterpret_cast<Real*>(s_net) + threadIdx.x;
-    Real* sa = sx + (size_t)m.S * blockDim.x;
+    const Column<Real> sx = column<Real>(s_net, 0), sa = column<Real>(s_net, sizeof(Real) * (size_t)m.S);
     const unsigned lane = threadIdx.x & 31u;
     uint32_t chunk = ((c_hi - c_lo + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x * blockDim.x;
     if (chunk > kNetChunk) chunk = kNetChunk;
@@ -1595,8 +1604,8 @@ __global__ void __launch_bounds__(256) k_exact_net(const __grid_constant__ NetAr
       __syncthreads();
       const uint32_t n = s_n;
       for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
-        fired += critical_event_net<Real, LOG>(A, net_tab<Real>(A), base + s_cell[j], sx, sa, blockDim.x, Xc, Xt, step,
-                                               attempt, A.b.D, flag);
+        fired += critical_event_net<Real, LOG, COMP>(A, net_tab<Real>(A), base + s_cell[j], sx, sa, Xc, Xt, step, attempt,
+                                                     A.b.D, flag);
       __syncthreads();
     }
   }
@@ -1610,10 +1619,7 @@ __global__ void __launch_bounds__(256) k_exact_net(const __grid_constant__ NetAr
       fired += argmin_event<Real, LOG>(A, am, x, step, attempt, dst, flag, fa == F_LEAP_CR);
     }
   }
-  if (fired) {  // exact events are rare: one atomic per firing thread
-    atomicAdd(&K->ev_attempt, (unsigned long long)fired);
-    atomicAdd(&K->ex_attempt, (unsigned long long)fired);
-  }
+  exact_totals(K, fired);
 }
 
 #ifdef PLIS_ENGINE_HOST_TU
@@ -1749,9 +1755,10 @@ __device__ __forceinline__ void classify_tile_small(const KArgs& A, const SmallM
 }
 
 // The same for a network with NetTab (net_step.cuh); smem: the CTA's count and propensity columns.
-template <typename Real, bool LAT>
+template <typename Real, bool LAT, bool COMP>
 __device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const ClassifyCtx& C,
-                                                  Real* smem, double& tn, uint32_t& ti, int& fl, int& bad, bool& valid) {
+                                                  unsigned char* smem, double& tn, uint32_t& ti, int& fl, int& bad,
+                                                  bool& valid) {
   const DevModel& m = A.m;
   const int S = (int)m.S;
   Cell cl;
@@ -1764,17 +1771,17 @@ __device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<R
   if (!valid) return;
   const double tau_cur = C.tau_cur[c];
   const uint8_t flag_cur = C.flag_cur[c];
-  Real* sx = smem + threadIdx.x;
+  const Column<Real> sx = column<Real>(smem, 0);
 #pragma unroll 4
   for (int s = 0; s < S; ++s) {
     const int32_t xs = C.Xe[(size_t)s * m.Npad + c];
     if (xs < 0) bad = 1;
-    sx[s * blockDim.x] = (Real)xs;
+    sx[s] = (Real)xs;
     C.Xz[(size_t)s * m.Npad + c] = 0;
   }
   if (!classify_ff(A.o.mode, tau_cur, flag_cur, C.step, C.ff, tn, fl)) {
     Real tau_ncr, rate;
-    net_tau_parts<Real, LAT>(A, T, cl, sx, sx + (size_t)S * blockDim.x, blockDim.x, C.Xe, tau_ncr, rate);
+    net_tau_parts<Real, LAT, COMP>(A, T, cl, sx, column<Real>(smem, sizeof(Real) * (size_t)S), C.Xe, tau_ncr, rate);
     cell_decide((double)tau_ncr, cell_tau_cr<Real>(A, c, C.step, C.attempt, rate), tn, fl);
   }
   C.tau_new[c] = tn;
@@ -1974,7 +1981,7 @@ __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify_smal
     classify_control(A, K, gridDim.x);
 }
 
-template <typename Real, bool LAT>
+template <typename Real, bool LAT, bool COMP>
 __global__ void __launch_bounds__(256, NetCtas<Real>::n) k_classify_net(const __grid_constant__ NetArgs A) {
   extern __shared__ __align__(16) unsigned char s_net[];
   pdl_entry();
@@ -1987,7 +1994,7 @@ __global__ void __launch_bounds__(256, NetCtas<Real>::n) k_classify_net(const __
   uint32_t ti;
   int fl, bad;
   bool valid;
-  classify_tile_net<Real, LAT>(A, net_tab<Real>(A), blockIdx.x, C, reinterpret_cast<Real*>(s_net), tn, ti, fl, bad, valid);
+  classify_tile_net<Real, LAT, COMP>(A, net_tab<Real>(A), blockIdx.x, C, s_net, tn, ti, fl, bad, valid);
   if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
     classify_control(A, K, gridDim.x);
 }
@@ -2179,20 +2186,30 @@ struct KernelSet {
     }
     if (a.o.net) {
       const NetArgs& n = static_cast<const NetArgs&>(a);
-      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, b.x, true);
-      if (a.m.lattice) launch_pdl(k_leap_net<Real, LOG, true>, g, b, bytes, s, n);
-      else launch_pdl(k_leap_net<Real, LOG, false>, g, b, bytes, s, n);
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, true);
+      if (a.m.lattice) {
+        if (a.m.comp) launch_pdl(k_leap_net<Real, LOG, true, true>, g, b, bytes, s, n);
+        else launch_pdl(k_leap_net<Real, LOG, true, false>, g, b, bytes, s, n);
+      } else {
+        if (a.m.comp) launch_pdl(k_leap_net<Real, LOG, false, true>, g, b, bytes, s, n);
+        else launch_pdl(k_leap_net<Real, LOG, false, false>, g, b, bytes, s, n);
+      }
       return;
     }
     launch_pdl(k_leap<Real, MAXS, LOG>, g, b, a.g.box_bytes, s, a);
   }
   // the largest shared memory any network asks for: one value, so that no handle lowers another's limit
   static cudaError_t net_smem_limit() {
-    constexpr int leap = (int)net_smem<Real>(kNetS, kNetR, 256, true), rest = (int)net_smem<Real>(kNetS, kNetR, 256, false);
-    const void* leaps[] = {(const void*)k_leap_net<Real, false, false>, (const void*)k_leap_net<Real, false, true>,
-                           (const void*)k_leap_net<Real, true, false>, (const void*)k_leap_net<Real, true, true>};
-    const void* rests[] = {(const void*)k_exact_net<Real, false>, (const void*)k_exact_net<Real, true>,
-                           (const void*)k_classify_net<Real, false>, (const void*)k_classify_net<Real, true>};
+    constexpr int leap = (int)net_smem<Real>(kNetS, kNetR, true), rest = (int)net_smem<Real>(kNetS, kNetR, false);
+    cudaError_t e = net_limits<false>(leap, rest);
+    return e == cudaSuccess ? net_limits<true>(leap, rest) : e;
+  }
+  template <bool COMP>
+  static cudaError_t net_limits(int leap, int rest) {
+    const void* leaps[] = {(const void*)k_leap_net<Real, false, false, COMP>, (const void*)k_leap_net<Real, false, true, COMP>,
+                           (const void*)k_leap_net<Real, true, false, COMP>, (const void*)k_leap_net<Real, true, true, COMP>};
+    const void* rests[] = {(const void*)k_exact_net<Real, false, COMP>, (const void*)k_exact_net<Real, true, COMP>,
+                           (const void*)k_classify_net<Real, false, COMP>, (const void*)k_classify_net<Real, true, COMP>};
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
       e = cudaFuncSetAttribute(leaps[i], cudaFuncAttributeMaxDynamicSharedMemorySize, leap);
@@ -2213,9 +2230,14 @@ struct KernelSet {
   static void exact(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
     if (a.o.net) {
       const NetArgs& n = static_cast<const NetArgs&>(a);
-      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, b.x, false);
-      if (a.b.ev.rec) launch_pdl(k_exact_net<Real, true>, g, b, bytes, s, n);
-      else launch_pdl(k_exact_net<Real, false>, g, b, bytes, s, n);
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, false);
+      if (a.m.comp) {
+        if (a.b.ev.rec) launch_pdl(k_exact_net<Real, true, true>, g, b, bytes, s, n);
+        else launch_pdl(k_exact_net<Real, false, true>, g, b, bytes, s, n);
+      } else {
+        if (a.b.ev.rec) launch_pdl(k_exact_net<Real, true, false>, g, b, bytes, s, n);
+        else launch_pdl(k_exact_net<Real, false, false>, g, b, bytes, s, n);
+      }
       return;
     }
     if (a.b.ev.rec) launch_pdl(k_exact<Real, MAXS, true>, g, b, 0, s, a);
@@ -2231,9 +2253,14 @@ struct KernelSet {
     }
     if (a.o.net) {
       const NetArgs& n = static_cast<const NetArgs&>(a);
-      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, b.x, false);
-      if (a.m.lattice) launch_pdl(k_classify_net<Real, true>, g, b, bytes, s, n);
-      else launch_pdl(k_classify_net<Real, false>, g, b, bytes, s, n);
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, false);
+      if (a.m.lattice) {
+        if (a.m.comp) launch_pdl(k_classify_net<Real, true, true>, g, b, bytes, s, n);
+        else launch_pdl(k_classify_net<Real, true, false>, g, b, bytes, s, n);
+      } else {
+        if (a.m.comp) launch_pdl(k_classify_net<Real, false, true>, g, b, bytes, s, n);
+        else launch_pdl(k_classify_net<Real, false, false>, g, b, bytes, s, n);
+      }
       return;
     }
     // the cache pays once the grid fills the GPU; on a grid of a few CTAs its extra pass only

@@ -25,41 +25,73 @@ template <typename Real> __device__ __forceinline__ const NetTab<Real>& net_tab(
 template <> __device__ __forceinline__ const NetTab<double>& net_tab<double>(const NetArgs& A) { return A.net.d; }
 template <> __device__ __forceinline__ const NetTab<float>& net_tab<float>(const NetArgs& A) { return A.net.f; }
 
-// shared memory of one CTA: S count columns, R propensity columns, and for the leap S net changes
+// shared memory of one CTA, rows of kNetCols: S rows of counts, R of propensities, and for the leap S
+// of net changes
 template <typename Real>
-constexpr size_t net_smem(uint32_t S, uint32_t R, uint32_t threads, bool leap) {
-  return (size_t)threads * (sizeof(Real) * (S + R) + (leap ? sizeof(int32_t) * S : 0u));
+constexpr size_t net_smem(uint32_t S, uint32_t R, bool leap) {
+  return (size_t)kNetCols * (sizeof(Real) * (S + R) + (leap ? sizeof(int32_t) * S : 0u));
 }
 
-template <typename Real>
-__device__ __forceinline__ Real net_rate(const NetTab<Real>& T, const DevModel& m, uint32_t comp, int r) {
-  return m.comp ? __ldg((const Real*)m.rr + (size_t)comp * m.R + r) : T.rate[r];
+// One thread's column: byte offsets of the tables, or row numbers, from its first row.
+template <typename T> struct Column {
+  unsigned char* p;
+  __device__ __forceinline__ T& at(uint32_t off) const { return *reinterpret_cast<T*>(p + off); }
+  __device__ __forceinline__ T& operator[](int row) const { return at((uint32_t)row * (kNetCols * (uint32_t)sizeof(T))); }
+};
+template <typename T>
+__device__ __forceinline__ Column<T> column(unsigned char* base, size_t row_bytes) {
+  return Column<T>{base + row_bytes * kNetCols + threadIdx.x * sizeof(T)};
 }
-template <typename Real>
+
+template <typename Real, bool COMP>
 __device__ __forceinline__ Real net_drate(const NetTab<Real>& T, const DevModel& m, uint32_t comp, int s) {
-  return m.comp ? __ldg((const Real*)m.dr + (size_t)comp * m.S + s) : T.drate[s];
+  if constexpr (COMP) return __ldg((const Real*)m.dr + (size_t)comp * m.S + s);
+  else return T.drate[s];
 }
 
-// Propensity of reaction r from the count column (prop()), and whether a reactant species is below its
+// Propensity of reaction r from the counts (prop()), and whether a reactant species is below its
 // threshold (crit_ref(); crit_fix() but for its test that the propensity is positive, see small_rates).
-template <typename Real>
-__device__ __forceinline__ Real net_prop(const NetTab<Real>& T, const DevModel& m, uint32_t comp, const Real* sx,
-                                         uint32_t stride, int r, bool& crit) {
-  const int nr = (int)T.nr[r];
+template <typename Real, bool COMP>
+__device__ __forceinline__ Real net_prop(const NetTab<Real>& T, const DevModel& m, uint32_t comp, Column<Real> sx, int r,
+                                         bool& crit) {
+  const uint32_t nf = T.nf[r];
   Real prod = (Real)1;
   bool cr = false;
-  for (int i = 0; i < nr; ++i) {
-    const uint32_t w = T.re[r][i];
-    const Real xs = sx[(w & 0xFFu) * stride];
-    prod = prod * xs;
-    if (w >> 9) {  // multiplicity 2 or 3
-      prod = prod * (xs - (Real)1);
-      if (w >> 8 == 3u) prod = prod * (xs - (Real)2);
+  if (nf > 0) {
+    const Real x0 = sx.at(T.fac[r][0].off);
+    cr = x0 < T.fac[r][0].thr;
+    prod = x0;  // the first factor has j = 0
+    if (nf > 1) {
+      const Real x1 = sx.at(T.fac[r][1].off);
+      cr = cr || x1 < T.fac[r][1].thr;
+      prod = prod * (x1 - T.fac[r][1].j);
+      if (nf > 2) {
+        const Real x2 = sx.at(T.fac[r][2].off);
+        cr = cr || x2 < T.fac[r][2].thr;
+        prod = prod * (x2 - T.fac[r][2].j);
+      }
     }
-    cr = cr || xs < T.thr[r][i];
   }
   crit = cr;
-  return (net_rate(T, m, comp, r) * prod) * T.inv_denom[r];
+  Real rate;
+  if constexpr (COMP) rate = __ldg((const Real*)m.rr + (size_t)comp * m.R + r);
+  else rate = T.rate[r];
+  return (rate * prod) * T.inv_denom[r];
+}
+
+// one draw by inversion (search4 for a single draw)
+template <typename Real>
+__device__ __forceinline__ int search1(uint32_t w, Real lam) {
+  if (Scaled<Real>::top(w)) return search_top<Real>(w, lam);
+  const Real u = Scaled<Real>::uniform(w);
+  Real p = RT<Real>::emlam(lam) * Scaled<Real>::scale, F = p;
+  int k = 0;
+  while (u > F && k < Scaled<Real>::kmax) {
+    ++k;
+    p = (p * lam) * (Real)plis_inv_k_tab[k];
+    F += p;
+  }
+  return k;
 }
 
 // The neighbours of a subvolume by direction (lattice) or slot (table).
@@ -87,22 +119,21 @@ __device__ __forceinline__ void net_dirs(const DevModel& m, const Cell& cl, Dirs
 // ------------------------------------------------------------------------------------------------
 // leap of one brick (leap_step, leap.cu:3-65), pooled or not
 // ------------------------------------------------------------------------------------------------
-template <typename Real, bool LOG, bool LAT>
+template <typename Real, bool LOG, bool LAT, bool COMP>
 __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const LeapCtx& L,
-                                              Real tl, Real* smem, long long& ev_out, int& big) {
+                                              Real tl, unsigned char* smem, long long& ev_out, int& big) {
   const DevModel& m = A.m;
   const int nc = A.o.nc, mode = A.o.mode;
   const int S = (int)m.S, R = (int)m.R;
-  const uint32_t stride = blockDim.x;
   ev_out = 0;
   big = 0;
   Cell cl;
   if (!cell_of(A, tile, cl)) return;
   const uint32_t c = cl.c;
   const uint8_t f = L.flag[c];
-  Real* sx = smem + threadIdx.x;                         // [S] counts
-  Real* sl = smem + (size_t)S * stride + threadIdx.x;    // [R] means of the firing reactions (0: none)
-  int32_t* sd = reinterpret_cast<int32_t*>(smem + (size_t)(S + R) * stride) + threadIdx.x;  // [S] net changes
+  const Column<Real> sx = column<Real>(smem, 0);                                       // [S] counts
+  const Column<Real> sl = column<Real>(smem, sizeof(Real) * (size_t)S);                // [R] means of the firing reactions
+  const Column<int32_t> sd = column<int32_t>(smem, sizeof(Real) * (size_t)(S + R));    // [S] net changes
   if (!(f == F_LEAP_CR || f == F_LEAP_NOCR)) {  // leap.cu:9-10
     for (int s = 0; s < S; ++s) {
       const int32_t xs = L.Xc[(size_t)s * m.Npad + c];
@@ -113,8 +144,8 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
   }
 #pragma unroll 4
   for (int s = 0; s < S; ++s) {
-    sx[s * stride] = (Real)L.Xc[(size_t)s * m.Npad + c];
-    sd[s * stride] = 0;
+    sx[s] = (Real)L.Xc[(size_t)s * m.Npad + c];
+    sd[s] = 0;
   }
   // Net changes of 2^24 and more go to 64-bit sums in local memory; the others, at most one per
   // reaction and species and one of jumps, stay below 2^30 in the 32-bit column.
@@ -122,7 +153,7 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
   bool has_wide = false;
   auto add = [&](int s, long long v) {
     if (v < (1 << 24) && v > -(1 << 24)) {
-      sd[s * stride] += (int32_t)v;
+      sd[s] += (int32_t)v;
     } else {
       if (!has_wide) {
         for (int i = 0; i < kNetS; ++i) wide[i] = 0;
@@ -131,7 +162,7 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
       wide[s] += v;
     }
   };
-  const uint32_t comp = m.comp ? (uint32_t)m.comp[c] : 0u;
+  const uint32_t comp = COMP ? (uint32_t)m.comp[c] : 0u;
   const bool pool_on = A.o.pool != 0;
   Real pool = (Real)0;
   uint32_t pool_r = 0, pool_s = 0;  // members of the pool
@@ -158,10 +189,10 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
       lam[i] = (Real)0;
       if (r < R) {
         bool crit;
-        const Real a = net_prop<Real>(T, m, comp, sx, stride, r, crit);
+        const Real a = net_prop<Real, COMP>(T, m, comp, sx, r, crit);
         Real lr = crit ? (Real)0 : tl * a;
         if (!(lr > (Real)0)) lr = (Real)0;
-        sl[r * stride] = lr;
+        sl[r] = lr;
         if (lr > (Real)0) {
           if (pool_join(lr, lr)) pool_r |= 1u << r;
           else {
@@ -181,19 +212,15 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
       const long long k = RT<Real>::count(RT<Real>::poisson(&st, li));
       if (k > 0) fired(r0 + i, k);
     }
-    if (need & 15u) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (!((need >> i) & 1u)) lam[i] = (Real)0;
+    if (need & 15u) {  // few of a network's channels are drawn on their own: one search at a time
       const plis_stream g =
           plis_stream_make(A.o.seed, A.o.replica, c, PLIS_PHASE_LEAP, L.step, L.attempt, plis_ch_rgroup((uint32_t)r0 >> 2));
       const plis_u32x4 b = plis_group_block_rk(&g, 0, A.o.rk0, A.o.rk1);
-      const uint32_t w[4] = {b.x, b.y, b.z, b.w};
-      int k[4];
-      search4<Real>(w, lam, k);
-      for (uint32_t todo = (k[0] ? 1u : 0u) | (k[1] ? 2u : 0u) | (k[2] ? 4u : 0u) | (k[3] ? 8u : 0u); todo; todo &= todo - 1u) {
+      for (uint32_t todo = need & 15u; todo; todo &= todo - 1u) {
         const int i = __ffs(todo) - 1;
-        fired(r0 + i, i == 0 ? k[0] : i == 1 ? k[1] : i == 2 ? k[2] : k[3]);
+        const Real li = i == 0 ? lam[0] : i == 1 ? lam[1] : i == 2 ? lam[2] : lam[3];
+        const int k = search1<Real>(i == 0 ? b.x : i == 1 ? b.y : i == 2 ? b.z : b.w, li);
+        if (k) fired(r0 + i, k);
       }
     }
   }
@@ -207,10 +234,10 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
     if (LOG) ev_put(A.b.ev, L.t, L.step, L.attempt, c, b, k, s, PLIS_EVENT_LEAP_DIFFUSION);
   };
   for (int s = 0; s < S; ++s) {
-    const Real xs = sx[s * stride];
+    const Real xs = sx[s];
     if (xs < (Real)nc || n == 0) continue;  // is_critical_diffusion, tau.cu:42-45
     mark = true;
-    const Real lam = tl * (net_drate(T, m, comp, s) * xs);
+    const Real lam = tl * (net_drate<Real, COMP>(T, m, comp, s) * xs);
     if (!(lam > (Real)0)) continue;
     if (pool_join(lam, (Real)n * lam)) {
       pool_s |= 1u << s;
@@ -277,13 +304,13 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
       int pick_r = -1, pick_s = -1, last = -1;
       for (uint32_t todo = pool_r; todo && pick_r < 0; todo &= todo - 1u) {
         last = __ffs(todo) - 1;
-        acc = acc + sl[last * stride];
+        acc = acc + sl[last];
         if (target < acc) pick_r = last;
       }
       if (pick_r < 0) {
         for (uint32_t todo = pool_s; todo && pick_s < 0; todo &= todo - 1u) {
           const int s = __ffs(todo) - 1;
-          acc = acc + (Real)n * (tl * (net_drate(T, m, comp, s) * sx[s * stride]));
+          acc = acc + (Real)n * (tl * (net_drate<Real, COMP>(T, m, comp, s) * sx[s]));
           if (target < acc) pick_s = s;
         }
         if (pick_s < 0) {  // rounding left the target at the total: the last member
@@ -302,7 +329,7 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
           if (d == j) b = q.nb[d];
         ev_out += 1;
         jumps(pick_s, 1, b);
-        sd[pick_s * stride] -= 1;
+        sd[pick_s] -= 1;
       }
     }
   }
@@ -312,7 +339,7 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
       if (((q.on >> d) & 1u) && L.flag[q.nb[d]] == F_SSA_FF) L.flag[q.nb[d]] = F_SSA;
   }
   for (int s = 0; s < S; ++s) {
-    long long tv = (long long)L.Xc[(size_t)s * m.Npad + c] + sd[s * stride];
+    long long tv = (long long)L.Xc[(size_t)s * m.Npad + c] + sd[s];
     if (has_wide) tv += wide[s];
     if (tv >= kBigTile || tv <= -kBigTile) big = 1;
     atomicAdd(&L.Xt[(size_t)s * m.Npad + c], (int)tv);
@@ -322,10 +349,37 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
 // ------------------------------------------------------------------------------------------------
 // classification of one subvolume (compute_taus, tau.cu:68-195): cell_tau_parts
 // ------------------------------------------------------------------------------------------------
-template <typename Real, bool LAT>
-__device__ __forceinline__ void net_tau_parts(const KArgs& A, const NetTab<Real>& T, const Cell& cl, const Real* sx,
-                                              Real* sa, uint32_t stride, const int32_t* Xe, Real& tau_ncr_out,
-                                              Real& rate_cr_out) {
+// The leap bound of one species from its drift mu and spread s2 (tau.cu:127-143).
+template <typename Real>
+__device__ __forceinline__ Real net_tau_species(const KArgs& A, int hor, int hmult, Real xs, Real mu, Real s2) {
+  Real mm = ((Real)A.o.eps * xs) / gfun<Real>(hor, hmult, xs);
+  if (!(mm > (Real)1)) mm = (Real)1;
+  const Real t1 = mm / fabs(mu);
+  const Real t2 = (mm * mm) / s2;
+  return t1 < t2 ? t1 : t2;
+}
+// The same to about 1e-6 in binary32 (0, inf or NaN outside its range).
+template <typename Real>
+__device__ __forceinline__ float net_tau_near(float eps, int hor, int hmult, Real xs, Real mu, Real s2) {
+  const float x = (float)xs;
+  float mm = eps * x;
+  if (hor != 1) {
+    float g;
+    if (hor == 0) g = __int_as_float(0x7f800000);
+    else if (hmult == 1) g = hor == 2 ? 2.f : 3.f;
+    else {
+      const float i1 = __fdividef(1.f, x - 1.f);
+      g = hor == 2 ? 2.f + i1 : hmult == 2 ? 1.5f * (2.f + i1) : 3.f + i1 + __fdividef(2.f, x - 2.f);
+    }
+    mm = __fdividef(mm, g);
+  }
+  mm = fmaxf(mm, 1.f);
+  return fminf(__fdividef(mm, fabsf((float)mu)), __fdividef(mm * mm, (float)s2));
+}
+
+template <typename Real, bool LAT, bool COMP>
+__device__ __forceinline__ void net_tau_parts(const KArgs& A, const NetTab<Real>& T, const Cell& cl, Column<Real> sx,
+                                              Column<Real> sa, const int32_t* Xe, Real& tau_ncr_out, Real& rate_cr_out) {
   const DevModel& m = A.m;
   const int mode = A.o.mode, nc = A.o.nc;
   const int S = (int)m.S, R = (int)m.R;
@@ -346,47 +400,62 @@ __device__ __forceinline__ void net_tau_parts(const KArgs& A, const NetTab<Real>
     for (int d = 0; d < 6; ++d)
       if ((q.on >> d) & 1u) nn |= (uint32_t)m.ncount[q.nb[d]] << (4 * d);
   }
-  const uint32_t comp = m.comp ? (uint32_t)m.comp[cl.c] : 0u;
-  if (m.comp) {
+  const uint32_t comp = COMP ? (uint32_t)m.comp[cl.c] : 0u;
+  if constexpr (COMP) {
 #pragma unroll
     for (int d = 0; d < 6; ++d)
       if ((q.on >> d) & 1u) ncomp |= (uint32_t)m.comp[q.nb[d]] << (5 * d);
   }
+  // the rows keep the propensities of the non-critical reactions, 0 for the others: a critical reaction
+  // then adds nothing to mu and s2, as if left out
   uint32_t critm = 0, posm = 0;
+  Real rcrit = (Real)0, rall = (Real)0;
 #pragma unroll 2
   for (int r = 0; r < R; ++r) {
     bool crit;
-    const Real a = net_prop<Real>(T, m, comp, sx, stride, r, crit);
-    sa[r * stride] = a;
-    critm |= (uint32_t)crit << r;
-    posm |= (uint32_t)(a > (Real)0) << r;
+    const Real a = net_prop<Real, COMP>(T, m, comp, sx, r, crit);
+    sa[r] = crit ? (Real)0 : a;
+    if (crit) {
+      critm |= 1u << r;
+      rcrit = rcrit + a;
+    } else if (a > (Real)0) {
+      posm |= 1u << r;
+    }
+    if (mode != 0) rall = rall + a;
   }
+  // The bound is a min over species.  Each species' bound is first formed in binary32; only the
+  // smallest, and any within 1e-4 of it or outside binary32's range, is then computed in full.
   Real tau_ncr = RT<Real>::inf();
+  const float eps = (float)A.o.eps;
+  float near_ = __int_as_float(0x7f800000);
+  Real b_mu = (Real)0, b_s2 = (Real)0;
+  int b_s = -1;
 #pragma unroll 1
   for (int s = 0; s < S; ++s) {
-    const Real xs = sx[s * stride];
-    const Real dr = net_drate(T, m, comp, s);
+    const Real xs = sx[s];
+    const Real dr = net_drate<Real, COMP>(T, m, comp, s);
     const uint32_t rmask = T.rmask[s];
+    const bool leaps = !(xs < (Real)nc);
     bool include;
-    if (mode == 0) include = !((critm & rmask) != 0u && xs < (Real)nc);  // tau.cu:165
-    else include = (posm & ~critm & rmask) != 0u || (!(xs < (Real)nc) && dr > (Real)0 && n > 0);
+    if (mode == 0) include = (critm & rmask) == 0u || leaps;  // tau.cu:165
+    else include = (posm & rmask) != 0u || (leaps && dr > (Real)0 && n > 0);
     if (!include) continue;
     int32_t xb[6];
     const int32_t* row = Xe + (size_t)s * m.Npad;
 #pragma unroll
     for (int d = 0; d < 6; ++d) xb[d] = (q.on >> d) & 1u ? row[q.nb[d]] : 0;
     Real mu = (Real)0, s2 = (Real)0;
-    for (uint32_t e = T.sp_off[s]; e < T.sp_off[s + 1]; ++e) {
-      const uint32_t r = T.sp_r[e];
-      if ((critm >> r) & 1u) continue;
-      const Real a = sa[r * stride];
-      mu = mu + T.sp_nu[e] * a;
-      s2 = s2 + T.sp_nu2[e] * a;
+    const uint32_t e1 = T.sp_off[s + 1];
+#pragma unroll 2
+    for (uint32_t e = T.sp_off[s]; e < e1; ++e) {
+      const Real a = sa.at(T.sp[e].off);
+      mu = mu + T.sp[e].nu * a;
+      s2 = s2 + T.sp[e].nu2 * a;
     }
     const Real d0 = dr * xs;
     if (mode == 0) {
-      if (!(xs < (Real)nc)) { mu = mu + d0; s2 = s2 + d0; }
-      if (deep && !m.comp) {
+      if (leaps) { mu = mu + d0; s2 = s2 + d0; }
+      if (deep && !COMP) {
 #pragma unroll
         for (int d = 0; d < 6; ++d) {
           const Real v = div_small(dr * (Real)xb[d], (Real)6, (Real)(1.0 / 6.0));
@@ -396,15 +465,15 @@ __device__ __forceinline__ void net_tau_parts(const KArgs& A, const NetTab<Real>
       } else {
 #pragma unroll
         for (int d = 0; d < 6; ++d) {  // an absent direction has count 0: v = 0 leaves mu and s2
-          const Real db = m.comp ? net_drate(T, m, (ncomp >> (5 * d)) & 31u, s) : dr;
-          const uint32_t nd = (nn >> (4 * d)) & 15u;
-          const Real v = div_small(db * (Real)xb[d], (Real)nd, (Real)plis_inv_k_tab[nd]);
+          const Real db = COMP ? net_drate<Real, COMP>(T, m, (ncomp >> (5 * d)) & 31u, s) : dr;
+          const Real* by = T.by[(nn >> (4 * d)) & 7u];
+          const Real v = div_small(db * (Real)xb[d], by[0], by[1]);
           mu = mu - v;
           s2 = s2 + v;
         }
       }
     } else {
-      if (!(xs < (Real)nc) && n > 0) {
+      if (leaps && n > 0) {
         const Real dout = (Real)n * d0;
         mu = mu - dout;
         s2 = s2 + dout;
@@ -412,41 +481,42 @@ __device__ __forceinline__ void net_tau_parts(const KArgs& A, const NetTab<Real>
 #pragma unroll
       for (int d = 0; d < 6; ++d) {
         if (xb[d] >= nc && ((q.on >> d) & 1u)) {
-          const Real v = (m.comp ? net_drate(T, m, (ncomp >> (5 * d)) & 31u, s) : dr) * (Real)xb[d];
+          const Real v = (COMP ? net_drate<Real, COMP>(T, m, (ncomp >> (5 * d)) & 31u, s) : dr) * (Real)xb[d];
           mu = mu + v;
           s2 = s2 + v;
         }
       }
     }
-    const int hor = T.hor[s], hmult = T.hmult[s];
-    Real mm;
-    {
-      const Real ex = (Real)A.o.eps * xs;
-      if (hor == 1) mm = ex;  // g = 1
-      else if (hor == 0) mm = (Real)0;  // g = inf
-      else if (hor == 2 && hmult == 1) mm = ex * (Real)0.5;  // g = 2
-      else mm = ex / gfun<Real>(hor, hmult, xs);
+    const float t = net_tau_near<Real>(eps, T.hor[s], T.hmult[s], xs, mu, s2);
+    const bool sane = t > 1e-30f && t < 1e30f;
+    if (sane && t < near_ * 0.9999f) {
+      near_ = t;
+      b_mu = mu;
+      b_s2 = s2;
+      b_s = s;
+    } else if (!sane || t < near_ * 1.0001f) {
+      const Real ts = net_tau_species<Real>(A, T.hor[s], T.hmult[s], xs, mu, s2);
+      if (ts < tau_ncr) tau_ncr = ts;
     }
-    if (!(mm > (Real)1)) mm = (Real)1;
-    const Real t1 = mm / fabs(mu);
-    const Real t2 = (mm * mm) / s2;
-    const Real ts = t1 < t2 ? t1 : t2;
+  }
+  if (b_s >= 0) {
+    const Real ts = net_tau_species<Real>(A, T.hor[b_s], T.hmult[b_s], sx[b_s], b_mu, b_s2);
     if (ts < tau_ncr) tau_ncr = ts;
   }
   // critical (or, corrected SSA subvolume: total) rate, compute_tau_cr tau.cu:176-195
-  Real rsum = (Real)0, dsum = (Real)0;
+  Real rsum, dsum = (Real)0;
   if (mode == 0 || !plis_isinf_d((double)tau_ncr)) {
-    for (uint32_t todo = critm; todo; todo &= todo - 1u) rsum = rsum + sa[(__ffs(todo) - 1) * stride];
+    rsum = rcrit;
     for (int s = 0; s < S; ++s) {
-      const Real xs = sx[s * stride];
+      const Real xs = sx[s];
       if (xs < (Real)nc) {
-        const Real d = net_drate(T, m, comp, s) * xs;
+        const Real d = net_drate<Real, COMP>(T, m, comp, s) * xs;
         dsum = dsum + (mode == 0 ? d : (Real)n * d);
       }
     }
   } else {
-    for (int r = 0; r < R; ++r) rsum = rsum + sa[r * stride];
-    for (int s = 0; s < S; ++s) dsum = dsum + (Real)n * (net_drate(T, m, comp, s) * sx[s * stride]);
+    rsum = rall;
+    for (int s = 0; s < S; ++s) dsum = dsum + (Real)n * (net_drate<Real, COMP>(T, m, comp, s) * sx[s]);
   }
   tau_ncr_out = tau_ncr;
   rate_cr_out = (rsum == (Real)0 && dsum == (Real)0) ? (Real)0 : rsum + dsum;
@@ -456,16 +526,16 @@ __device__ __forceinline__ void net_tau_parts(const KArgs& A, const NetTab<Real>
 // critical event of one LEAP_CR subvolume, reference semantics (leap.cu:86-199): critical_event_ref
 // with its propensities evaluated once
 // ------------------------------------------------------------------------------------------------
-template <typename Real, bool LOG>
-__device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<Real>& T, uint32_t c, Real* sx, Real* sa,
-                                                  uint32_t stride, const int32_t* Xc, const int32_t* Xt, uint64_t step,
+template <typename Real, bool LOG, bool COMP>
+__device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<Real>& T, uint32_t c, Column<Real> sx,
+                                                  Column<Real> sa, const int32_t* Xc, const int32_t* Xt, uint64_t step,
                                                   uint32_t attempt, int32_t* D, uint8_t* flag) {
   const DevModel& m = A.m;
   const int nc = A.o.nc;
   const int S = (int)m.S, R = (int)m.R;
-  const uint32_t comp = m.comp ? (uint32_t)m.comp[c] : 0u;
+  const uint32_t comp = COMP ? (uint32_t)m.comp[c] : 0u;
 #pragma unroll 4
-  for (int s = 0; s < S; ++s) sx[s * stride] = (Real)Xc[(size_t)s * m.Npad + c];
+  for (int s = 0; s < S; ++s) sx[s] = (Real)Xc[(size_t)s * m.Npad + c];
   plis_stream su = plis_stream_make(A.o.seed, A.o.replica, c, PLIS_PHASE_CRIT, step, attempt, 0);
   const Real u = RT<Real>::uniform(&su);
   uint32_t critm = 0;
@@ -473,17 +543,17 @@ __device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<R
 #pragma unroll 2
   for (int r = 0; r < R; ++r) {
     bool crit;
-    const Real a = net_prop<Real>(T, m, comp, sx, stride, r, crit);
-    sa[r * stride] = a;
+    const Real a = net_prop<Real, COMP>(T, m, comp, sx, r, crit);
+    sa[r] = a;
     critm |= (uint32_t)crit << r;
     if (crit) rsum = rsum + a;
   }
   uint32_t dcrit = 0;
   for (int s = 0; s < S; ++s) {
-    const Real xs = sx[s * stride];
+    const Real xs = sx[s];
     if (xs < (Real)nc) {
       dcrit |= 1u << s;
-      dsum = dsum + net_drate(T, m, comp, s) * xs;
+      dsum = dsum + net_drate<Real, COMP>(T, m, comp, s) * xs;
     }
   }
   if (rsum + dsum == (Real)0) return 0;
@@ -492,7 +562,7 @@ __device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<R
     Real partial = (Real)0;
     int ric = 0;
     while (partial <= scaled && ric < R) {
-      if ((critm >> ric) & 1u) partial = partial + sa[ric * stride];
+      if ((critm >> ric) & 1u) partial = partial + sa[ric];
       ++ric;
     }
     int ri = 0;
@@ -505,9 +575,9 @@ __device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<R
     bool fire = true;
     for (int s = 0; s < S; ++s) {
       int need = 0;
-      for (uint32_t i = 0; i < T.nr[ri]; ++i)
-        if ((T.re[ri][i] & 0xFFu) == (uint32_t)s) need = (int)(T.re[ri][i] >> 8);
-      fire = fire && !(sx[s * stride] < (Real)need) && Xt[(size_t)s * m.Npad + c] >= need;
+      for (uint32_t w = T.need[ri]; w; w >>= 10)
+        if ((w & 31u) == (uint32_t)s) need = (int)((w >> 5) & 31u);
+      fire = fire && !(sx[s] < (Real)need) && Xt[(size_t)s * m.Npad + c] >= need;
     }
     if (!fire) return 0;
     for (uint32_t e = T.net_off[ri]; e < T.net_off[ri + 1]; ++e)
@@ -520,7 +590,7 @@ __device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<R
   Real partial = (Real)0;
   int spic = 0;
   while (partial <= scaled && spic < S) {
-    if ((dcrit >> spic) & 1u) partial = partial + net_drate(T, m, comp, spic) * sx[spic * stride];
+    if ((dcrit >> spic) & 1u) partial = partial + net_drate<Real, COMP>(T, m, comp, spic) * sx[spic];
     ++spic;
   }
   int spi = 0;
@@ -528,7 +598,7 @@ __device__ __forceinline__ int critical_event_net(const KArgs& A, const NetTab<R
     if ((dcrit >> spi) & 1u) --spic;
   spi = spi - 1;  // leap.cu:160-166
   if (spi < 0) spi = 0;
-  return critical_jump_ref<Real, LOG>(A, c, spi, sx[spi * stride] > (Real)0, Xt, step, attempt, D, flag);
+  return critical_jump_ref<Real, LOG>(A, c, spi, sx[spi] > (Real)0, Xt, step, attempt, D, flag);
 }
 
 }  // namespace plis
