@@ -325,7 +325,8 @@ int Engine::create(const Model& model, const plis_options& opt) {
   // than N/2 events in one attempt fall back to a scan of all deltas)
   if ((rc = dmalloc((void**)&b.D, (cells + dm.Npad) * 4))) return rc;
   PLIS_CU(cudaMemset(b.D, 0, cells * 4));
-  if ((rc = dmalloc((void**)&b.slot, (size_t)g.nblocks * sizeof(SlotRec)))) return rc;
+  // a record per brick, or per tile of 128 rows where a learned classification decides
+  if ((rc = dmalloc((void**)&b.slot, std::max<size_t>(g.nblocks, ((size_t)dm.Npad + 127) / 128) * sizeof(SlotRec)))) return rc;
   if ((rc = dmalloc((void**)&b.ctrl, sizeof(Ctrl)))) return rc;
   PLIS_CU(cudaMemset(b.ctrl, 0, sizeof(Ctrl)));
 
@@ -510,7 +511,6 @@ int Engine::set_proposer(const float* weights, double s_max) {
       PLIS_CU(cudaMemset(d_feat_, 0, rows * sizeof(uint4)));
       if ((rc = dmalloc((void**)&d_pre_, (size_t)args_.m.Npad * sizeof(double2)))) return rc;
       if ((rc = dmalloc((void**)&d_pre_kind_, (size_t)args_.m.Npad))) return rc;
-      if ((rc = dmalloc((void**)&d_ymlp_, rows * sizeof(float)))) return rc;
     }
     PLIS_CU(cudaMemcpyAsync(d_lw_, weights, PLIS_PROPOSER_WEIGHTS * sizeof(float), cudaMemcpyHostToDevice, stream_));
     learned_pack(d_lw_, s_max, d_lp_, stream_);
@@ -519,12 +519,11 @@ int Engine::set_proposer(const float* weights, double s_max) {
     args_.b.feat = d_feat_;
     args_.b.pre = d_pre_;
     args_.b.pre_kind = d_pre_kind_;
-    args_.b.ymlp = d_ymlp_;
   } else {
     args_.b.lp = nullptr;
   }
   use_learned_ = on;
-  const int classify_launches = (on && opt_.learned_mlp == PLIS_MLP_TCGEN05) ? 3 : 1;
+  const int classify_launches = (on && opt_.learned_mlp == PLIS_MLP_TCGEN05) ? 2 : 1;
   kernels_per_step_ = ((opt_.mode == PLIS_MODE_REFERENCE) ? 4 : 3) + classify_launches - 1;
   if (graph_exec_) {  // the graph holds the kernel arguments by value
     cudaGraphExecDestroy(graph_exec_);

@@ -95,14 +95,13 @@ struct EvLog {
   unsigned long long cap;
 };
 
-// What one CTA (brick) of the classification found, two 16-byte words.
+// What one CTA of the classification found, two 16-byte words.
 struct alignas(16) SlotRec {
   double tau;        // min tau
   double tau_plain;  // learned classification: min of the plain taus
   uint32_t idx;      // the subvolume of tau (first on ties), 0xFFFFFFFF when the brick has none
-  uint32_t crff;     // #LEAP_CR | #SSA_FF << 16 (<= 1024 each)
+  uint32_t ncr, nff; // #LEAP_CR, #SSA_FF
   uint32_t bad;      // 1: a negative count
-  uint32_t pad_;
 };
 static_assert(sizeof(SlotRec) == 32, "SlotRec is read as two uint4");
 
@@ -116,7 +115,6 @@ struct DevBufs {
   uint4* feat;             // learned classification (split): normalised BF16 features, 16 B per subvolume
   double2* pre;            // (leap bound or fast-forwarded tau, critical rate) per subvolume
   uint8_t* pre_kind;       // 1: fast-forwarded, 2: leap bound computed
-  float* ymlp;             // MLP output per subvolume
   Ctrl* ctrl;
   EvLog ev;                // event log (rec == null: off)
 };

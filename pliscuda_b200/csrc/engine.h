@@ -95,7 +95,6 @@ class Engine {
   uint4* d_feat_ = nullptr;
   double2* d_pre_ = nullptr;
   uint8_t* d_pre_kind_ = nullptr;
-  float* d_ymlp_ = nullptr;
   EvRec* d_evrec_ = nullptr;
   unsigned long long* d_evhead_ = nullptr;
   uint32_t slab_blocks_ = 0;  // bricks of this handle's z-slab (0: not a slab)

@@ -1789,47 +1789,49 @@ __device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<R
   ti = c;
 }
 
-// CTA reduction of one brick into slot `slot` (min tau with arg-min, with PLAIN the min of the plain
-// taus tp, #LEAP_CR, #SSA_FF, negative flag), then the count of finished bricks; true in the CTA that
-// finished last of `nslots`.  Two CTA barriers: after the warps' partial results, and for the verdict.
+// CTA reduction into slot `slot` of its threads' min tau with arg-min (key, ti), with PLAIN the min of
+// their plain taus tp, #LEAP_CR, #SSA_FF and negative flags, then the count of finished CTAs; true in
+// the CTA that finished last of `nslots`.  Two CTA barriers: after the warps' partial results, and for
+// the verdict.
 template <bool PLAIN>
-__device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t slot, uint32_t nslots, double tn,
-                                              uint32_t ti, double tp, bool is_cr, int bad, bool is_ff) {
+__device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t slot, uint32_t nslots, uint64_t key,
+                                              uint32_t ti, double tp, uint32_t ncr, uint32_t nff, int bad) {
   __shared__ uint64_t s_k[32];
   __shared__ double s_p[32];
-  __shared__ uint32_t s_i[32], s_c[32];
+  __shared__ uint32_t s_i[32], s_cr[32], s_ff[32];
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint64_t k = tau_key(tn);
-  uint32_t crff = (uint32_t)__popc(__ballot_sync(0xffffffffu, is_cr)) |
-                  ((uint32_t)__popc(__ballot_sync(0xffffffffu, is_ff)) << 15);
-  crff |= __any_sync(0xffffffffu, bad) ? 0x80000000u : 0u;
-  warp_min_key(k, ti);
+  ncr = __reduce_add_sync(0xffffffffu, ncr);
+  nff = __reduce_add_sync(0xffffffffu, nff);
+  const bool wbad = __any_sync(0xffffffffu, bad);
+  warp_min_key(key, ti);
   if constexpr (PLAIN) tp = warp_min_d(tp);
   if (lane == 0) {
-    s_k[wid] = k;
+    s_k[wid] = key;
     s_i[wid] = ti;
-    s_c[wid] = crff;
+    s_cr[wid] = ncr;
+    s_ff[wid] = nff | (wbad ? 0x80000000u : 0u);
     if constexpr (PLAIN) s_p[wid] = tp;
   }
   __syncthreads();
   if (wid == 0) {
     const bool on = lane < (int)((blockDim.x + 31) >> 5);
-    k = on ? s_k[lane] : ~0ull;
+    key = on ? s_k[lane] : ~0ull;
     ti = on ? s_i[lane] : kNoCell;
-    crff = on ? s_c[lane] : 0u;
-    const bool nbad = __any_sync(0xffffffffu, (crff >> 31) != 0u);
-    crff = __reduce_add_sync(0xffffffffu, crff & 0x7fffffffu);  // two counts of at most 1024, 15 bits apart
-    warp_min_key(k, ti);
+    ncr = __reduce_add_sync(0xffffffffu, on ? s_cr[lane] : 0u);
+    nff = on ? s_ff[lane] : 0u;
+    const bool cbad = __any_sync(0xffffffffu, (nff >> 31) != 0u);
+    nff = __reduce_add_sync(0xffffffffu, nff & 0x7fffffffu);
+    warp_min_key(key, ti);
     if constexpr (PLAIN) tp = warp_min_d(on ? s_p[lane] : PLIS_INF_D);
     if (lane == 0) {
       SlotRec q;
-      q.tau = key_tau(k);
+      q.tau = key_tau(key);
       q.tau_plain = PLAIN ? tp : PLIS_INF_D;
       q.idx = ti;
-      q.crff = (crff & 0x7fffu) | ((crff >> 15) << 16);
-      q.bad = nbad ? 1u : 0u;
-      q.pad_ = 0;
+      q.ncr = ncr;
+      q.nff = nff;
+      q.bad = cbad ? 1u : 0u;
       A.b.slot[slot] = q;
       __threadfence();
       const uint32_t prev = atomicAdd(&K->blocks_done, 1u);
@@ -1838,6 +1840,12 @@ __device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t 
   }
   __syncthreads();
   return s_last;
+}
+// the same with one subvolume per thread
+template <bool PLAIN>
+__device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t slot, uint32_t nslots, double tn,
+                                              uint32_t ti, double tp, bool is_cr, int bad, bool is_ff) {
+  return classify_slot<PLAIN>(A, K, slot, nslots, tau_key(tn), ti, tp, is_cr ? 1u : 0u, is_ff ? 1u : 0u, bad);
 }
 
 // The step decision (driver.cu:267-334) from the grid-wide reductions: the arg-min gt / gi (gi = -1 when
@@ -1849,8 +1857,9 @@ __device__ __forceinline__ void step_decide(const KArgs& A, Ctrl* K, uint32_t ph
                                             bool learned, uint32_t am_flag) {
   const int mode = A.o.mode;
   Ctrl k = *K;
-  k.blocks_done = 0;  // changed by the other CTAs since this one's first reads
+  k.blocks_done = 0;  // these three may have changed since this SM first read the block
   k.n_touched = 0;
+  k.status = __ldcg(&K->status);
   k.learned = learned ? 1u : 0u;
   if (phase == 0) {
     k.tau_min = gt;
@@ -1916,9 +1925,9 @@ __device__ __forceinline__ void classify_control(const KArgs& A, Ctrl* K, uint32
     const uint4 u = __ldcg(q), v = __ldcg(q + 1);
     min_key(gk, gi, tau_key(__hiloint2double((int)u.y, (int)u.x)), v.x);
     gp = fmin(gp, __hiloint2double((int)u.w, (int)u.z));
-    gcr += v.y & 0xFFFFu;
-    gff += v.y >> 16;
-    gbad |= v.z;
+    gcr += v.y;
+    gff += v.z;
+    gbad |= v.w;
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int round = 0; round < 2; ++round) {  // the warps, then their results in warp 0

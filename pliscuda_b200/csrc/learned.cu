@@ -7,8 +7,8 @@
 //    is, after bias + ReLU + BF16 rounding, exactly the A fragment of the next layer, so hidden
 //    activations never leave registers; B fragments are pre-packed per lane (16 KB per layer, read
 //    through L1).
-//  * k_classify_learned (MLP by mma.sync inside the classification) or k_learned_pre + k_mlp_tc
-//    (tcgen05, tc_mlp.cuh) + k_learned_post: the classification with proposals, a second (plain)
+//  * k_classify_learned (MLP by mma.sync inside the classification) or k_learned_pre +
+//    k_learned_decide (tcgen05, tc_mlp.cuh): the classification with proposals, a second (plain)
 //    min-tau reduction for the rollback fallback, and the usual last-CTA control.
 //  * k_trace_features / k_trace_label: recording of (features, label) pairs from plain steps.
 //  * k_train / k_adam / feature statistics / k_pack: training in FP32 (one CTA = 128 records, the
@@ -69,101 +69,133 @@ __global__ void __launch_bounds__(256, 2) k_classify_learned(KArgs A) {
   if (learned_classify_tile<Real, MAXS>(A, K, C, blockIdx.x, gridDim.x)) classify_control(A, K, gridDim.x);
 }
 
-// The classification with proposals split in three launches, the MLP on tcgen05 in between:
-// k_learned_pre (per subvolume: negativity check, zeroing of the next target, fast-forward or leap
-// bound and critical rate, normalised BF16 features), k_mlp_tc (persistent, tc_mlp.cuh), and
-// k_learned_post (critical time, decision against the proposal and the plain bound, reductions,
-// last-CTA control).  The pre and post passes keep the plain classification's occupancy.
-template <typename Real, int MAXS>
-__global__ void __launch_bounds__(256) k_learned_pre(KArgs A) {
+// The classification with proposals in two launches: k_learned_pre (per subvolume: negativity check,
+// zeroing of the next target, fast-forward or leap bound and critical rate, normalised BF16 features)
+// keeps the plain classification's occupancy; k_learned_decide runs the MLP on tcgen05 (persistent,
+// tc_mlp.cuh) and, in the thread that holds a row's result, the critical time, the decisions against
+// the proposal and the plain bound, and the reductions.
+// SMALL: a small model on a lattice (small_step.cuh): the plain classification's leap bound, and the
+// features from its propensities and neighbour counts.
+template <typename Real, int MAXS, bool SMALL>
+__global__ void __launch_bounds__(256, 4) k_learned_pre(const __grid_constant__ KArgs A) {
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  if (K->done) return;
+  const int done = K->done;
   const ClassifyCtx C = classify_ctx(A, K);
+  if (done) return;
   const LearnedParams* P = A.b.lp;
   const DevModel& m = A.m;
   Cell cl;
-  const bool valid = cell_of(A, blockIdx.x, cl);
+  if (!cell_of(A, blockIdx.x, cl)) return;
   const uint32_t c = cl.c;
+  Counts<MAXS> x;
+  load_counts(m, C.Xe, c, x);
   int bad = 0;
-  if (valid) {
-    Counts<MAXS> x;
-    load_counts(m, C.Xe, c, x);
 #pragma unroll
-    for (int s = 0; s < MAXS; ++s)
-      if (s < (int)m.S) {
-        if (x.v[s] < 0) bad = 1;
-        C.Xz[(size_t)s * m.Npad + c] = 0;
-      }
-    Nbr q;
-    nbr_info(m, cl, q);
-    double tn;
-    int fl;
-    float f[kFeat];
-#pragma unroll
-    for (int k = 0; k < kFeat; ++k) f[k] = 0.f;
-    if (classify_ff(A.o.mode, C.tau_cur[c], C.flag_cur[c], C.step, C.ff, tn, fl)) {
-      A.b.pre[c] = make_double2(tn, 0.0);
-      A.b.pre_kind[c] = 1;
-    } else {
-      Real tau_ncr, rate;
-      cell_tau_parts<Real>(A, c, q, x, C.Xe, tau_ncr, rate);
-      A.b.pre[c] = make_double2((double)tau_ncr, (double)rate);
-      A.b.pre_kind[c] = 2;
-      if (!plis_isinf_d((double)tau_ncr)) {
-        cell_features<Real>(A, c, q, x, C.Xe, tau_ncr, f);
-        normalise(P, f);
-      }
+  for (int s = 0; s < MAXS; ++s)
+    if (s < (int)m.S) {
+      if (x.v[s] < 0) bad = 1;
+      C.Xz[(size_t)s * m.Npad + c] = 0;
     }
-    A.b.feat[c] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
-                             pack_bf16x2(f[6], f[7]));
+  if (bad) atomicOr(&K->blocks_done, 0x80000000u);  // rare: the attempt is rolled back
+  double tn;
+  int fl;
+  float f[kFeat];
+#pragma unroll
+  for (int k = 0; k < kFeat; ++k) f[k] = 0.f;
+  if (classify_ff(A.o.mode, C.tau_cur[c], C.flag_cur[c], C.step, C.ff, tn, fl)) {
+    A.b.pre[c] = make_double2(tn, 0.0);
+    A.b.pre_kind[c] = 1;
+  } else {
+    Real tau_ncr, rate;
+    if constexpr (SMALL) {
+      small_tau_parts<Real, MAXS, true>(A, A.sm, cl, x.v, C.Xe, tau_ncr, rate);
+      if (!plis_isinf_d((double)tau_ncr)) small_features<Real, MAXS>(A, cl, x, C.Xe, tau_ncr, f);
+    } else {
+      Nbr q;
+      nbr_info(m, cl, q);
+      cell_tau_parts<Real>(A, c, q, x, C.Xe, tau_ncr, rate);
+      if (!plis_isinf_d((double)tau_ncr)) cell_features<Real>(A, c, q, x, C.Xe, tau_ncr, f);
+    }
+    A.b.pre[c] = make_double2((double)tau_ncr, (double)rate);
+    A.b.pre_kind[c] = 2;
+    if (!plis_isinf_d((double)tau_ncr)) normalise(P, f);
   }
-  const int nbad = __syncthreads_or(bad);
-  if (threadIdx.x == 0) A.b.slot[blockIdx.x].bad = nbad ? 1u : 0u;
+  A.b.feat[c] = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
+                           pack_bf16x2(f[6], f[7]));
 }
 
-__global__ void __launch_bounds__(128) k_mlp_tc(const Ctrl* __restrict__ K, const LearnedParams* __restrict__ P,
-                                                const uint4* __restrict__ feats, float* __restrict__ y, uint32_t nrows,
-                                                uint32_t ntiles, int* status, uint32_t wait_limit) {
+// MLP outputs into an array (Learner::predict).
+struct PredictSink {
+  float* y;
+  uint32_t nrows;
+  __device__ __forceinline__ void begin(uint32_t) {}
+  __device__ __forceinline__ void end(uint32_t row, float v) {
+    if (row < nrows) y[row] = v;
+  }
+};
+__global__ void __launch_bounds__(tc::kThreads, 2) k_mlp_tc(const LearnedParams* __restrict__ P,
+                                                            const uint4* __restrict__ feats, float* __restrict__ y,
+                                                            uint32_t nrows, uint32_t ntiles, int* status) {
   extern __shared__ __align__(128) uint8_t tsm[];
-  pdl_entry();
-  if (K && K->done) return;
-  tc::mlp_tiles(tc_params(P), feats, y, nrows, ntiles, tsm, status, wait_limit);
+  PredictSink sink{y, nrows};
+  tc::mlp_tiles(tc_params(P), feats, ntiles, tsm, status, 0u, sink);
 }
 
-template <typename Real, int MAXS>
-__global__ void __launch_bounds__(256) k_learned_post(KArgs A) {
-  pdl_entry();
-  Ctrl* K = A.b.ctrl;
-  if (K->done) return;
-  const ClassifyCtx C = classify_ctx(A, K);
-  const LearnedParams* P = A.b.lp;
-  Cell cl;
-  const bool valid = cell_of(A, blockIdx.x, cl);
-  const uint32_t c = cl.c;
-  double tn = PLIS_INF_D, tp = PLIS_INF_D;
-  uint32_t ti = kNoCell;
-  int fl = F_SSA_FF;
-  if (valid) {
-    const double2 pr = A.b.pre[c];
-    if (A.b.pre_kind[c] == 1) {
+// The step's decision for each row's subvolume, and the thread's running reductions.
+template <typename Real> struct DecideSink {
+  const KArgs& A;
+  const ClassifyCtx& C;
+  float log_smax;
+  uint64_t key = tau_key(PLIS_INF_D);
+  uint32_t ti = kNoCell, ncr = 0, nff = 0;
+  double tp = PLIS_INF_D;
+  double2 pr;
+  uint32_t kind;
+  __device__ __forceinline__ DecideSink(const KArgs& a, const ClassifyCtx& c, float ls) : A(a), C(c), log_smax(ls) {}
+  __device__ __forceinline__ void begin(uint32_t c) {
+    kind = 0;
+    if (c < A.m.N) {
+      pr = A.b.pre[c];
+      kind = A.b.pre_kind[c];
+    }
+  }
+  __device__ __forceinline__ void end(uint32_t c, float y) {
+    if (kind == 0) return;
+    double tn, plain;
+    int fl = F_SSA_FF;
+    if (kind == 1) {
       tn = pr.x;
-      tp = tn;
+      plain = tn;
     } else {
       const double tcr = cell_tau_cr<Real>(A, c, C.step, C.attempt, (Real)pr.y);
       int fp;
-      cell_decide(pr.x, tcr, tp, fp);
-      const float ls = fminf(fmaxf(A.b.ymlp[c], 0.f), P->log_smax);
+      cell_decide(pr.x, tcr, plain, fp);
+      const float ls = fminf(fmaxf(y, 0.f), log_smax);
       const double sc = ls > 0.f ? (double)expf(ls) : 1.0;
       cell_decide(plis_isinf_d(pr.x) ? pr.x : pr.x * sc, tcr, tn, fl);
     }
     C.tau_new[c] = tn;
     C.flag_new[c] = (uint8_t)fl;
-    ti = c;
+    min_key(key, ti, tau_key(tn), c);
+    tp = fmin(tp, plain);
+    ncr += fl == F_LEAP_CR;
+    nff += fl == F_SSA_FF;
   }
-  const int bad = threadIdx.x == 0 ? (int)A.b.slot[blockIdx.x].bad : 0;
-  if (classify_slot<true>(A, K, blockIdx.x, gridDim.x, tn, ti, tp, valid && fl == F_LEAP_CR, bad,
-                          valid && fl == F_SSA_FF))
+};
+
+template <typename Real>
+__global__ void __launch_bounds__(tc::kThreads, 2) k_learned_decide(const __grid_constant__ KArgs A, uint32_t ntiles) {
+  extern __shared__ __align__(128) uint8_t tsm[];
+  pdl_entry();
+  Ctrl* K = A.b.ctrl;
+  const int done = K->done;
+  const ClassifyCtx C = classify_ctx(A, K);
+  if (blockIdx.x == 0 && threadIdx.x == 0) K->n_touched = 0;
+  if (done) return;
+  DecideSink<Real> sink(A, C, A.b.lp->log_smax);
+  tc::mlp_tiles(tc_params(A.b.lp), A.b.feat, ntiles, tsm, (int*)&K->status, A.o.mlp_wait, sink);
+  if (classify_slot<true>(A, K, blockIdx.x, gridDim.x, sink.key, sink.ti, sink.tp, sink.ncr, sink.nff, 0))
     classify_control(A, K, gridDim.x);
 }
 
@@ -238,7 +270,7 @@ __global__ void k_trace_label(KArgs A, TraceRec* recs, uint32_t count, double ta
   recs[i] = r;
 }
 
-// persistent grid of the tile kernel: 4 CTAs per SM at most, never more CTAs than tiles
+// persistent grid of the tile kernels: two CTAs per SM at most, never more CTAs than they have tiles for
 static uint32_t mlp_grid(uint32_t ntiles) {
   static int sms = 0;
   if (sms == 0) {
@@ -246,8 +278,8 @@ static uint32_t mlp_grid(uint32_t ntiles) {
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   }
-  const uint32_t g = 4u * (uint32_t)sms;
-  return ntiles < g ? (ntiles ? ntiles : 1u) : g;
+  const uint32_t g = 2u * (uint32_t)sms, need = (ntiles + tc::kGroups - 1) / tc::kGroups;
+  return need < g ? (need ? need : 1u) : g;
 }
 
 template <typename Real, int MAXS>
@@ -256,12 +288,10 @@ struct LearnedSet {
     launch_pdl(k_classify_learned<Real, MAXS>, g, b, 0, s, a);
   }
   static void classify_split(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
-    launch_pdl(k_learned_pre<Real, MAXS>, g, b, 0, s, a);
+    if (a.sm.on && a.m.lattice) launch_pdl(k_learned_pre<Real, MAXS, true>, g, b, 0, s, a);
+    else launch_pdl(k_learned_pre<Real, MAXS, false>, g, b, 0, s, a);
     const uint32_t ntiles = a.m.Npad / 128u + ((a.m.Npad % 128u) ? 1u : 0u);
-    launch_pdl(k_mlp_tc, dim3(mlp_grid(ntiles)), dim3(128), tc::kPSmemBytes, s, (const Ctrl*)a.b.ctrl,
-               (const LearnedParams*)a.b.lp, (const uint4*)a.b.feat, a.b.ymlp, a.m.Npad, ntiles, (int*)&a.b.ctrl->status,
-               a.o.mlp_wait);
-    launch_pdl(k_learned_post<Real, MAXS>, g, b, 0, s, a);
+    launch_pdl(k_learned_decide<Real>, dim3(mlp_grid(ntiles)), dim3(tc::kThreads), tc::kPSmemBytes, s, a, ntiles);
   }
   static void features(const KArgs& a, TraceRec* out, uint32_t offset, uint32_t stride, uint32_t count,
                        cudaStream_t s) {
@@ -276,7 +306,8 @@ template <typename Real, int MAXS>
 static LearnedLaunch learned_set(int mlp) {
   using L = LearnedSet<Real, MAXS>;
   if (mlp == PLIS_MLP_MMA_SYNC) return {L::classify, L::features, L::label};
-  if (cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kPSmemBytes) != cudaSuccess)
+  if (cudaFuncSetAttribute(k_learned_decide<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kPSmemBytes) !=
+      cudaSuccess)
     return {nullptr, nullptr, nullptr};
   return {L::classify_split, L::features, L::label};
 }
@@ -891,8 +922,8 @@ int Learner::predict(const float* features, uint64_t n, float* y, int mlp_kernel
         e = cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kPSmemBytes);
       if (e == cudaSuccess) {
         k_feat_rows<<<(unsigned)((ntiles * 128 + 255) / 256), 256, 0, stream_>>>(packed_, d_f, n, ntiles * 128, d_rows);
-        k_mlp_tc<<<mlp_grid((uint32_t)ntiles), 128, tc::kPSmemBytes, stream_>>>(nullptr, packed_, d_rows, d_y,
-                                                                                (uint32_t)n, (uint32_t)ntiles, d_st, 0u);
+        k_mlp_tc<<<mlp_grid((uint32_t)ntiles), tc::kThreads, tc::kPSmemBytes, stream_>>>(packed_, d_rows, d_y, (uint32_t)n,
+                                                                                         (uint32_t)ntiles, d_st);
         e = cudaStreamSynchronize(stream_);
       }
       if (d_rows) cudaFree(d_rows);

@@ -30,6 +30,34 @@ __device__ __forceinline__ void cell_features(const KArgs& A, uint32_t c, const 
   f[7] = log1pf(dt);
 }
 
+// cell_features for a small model on a lattice: the same values, the propensities from the argument
+// tables and the neighbours by direction (the leap bound's pass has just read both).
+template <typename Real, int MAXS>
+__device__ __forceinline__ void small_features(const KArgs& A, const Cell& cl, const Counts<MAXS>& x, const int32_t* Xe,
+                                               Real tau_ncr, float f[kFeat]) {
+  const DevModel& m = A.m;
+  const uint32_t on = lattice_dirs(m, cl), XY = m.X * m.Y, c = cl.c;
+  const uint32_t nb[6] = {c - 1, c + 1, c - m.X, c + m.X, c - XY, c + XY};
+  const int n = __popc(on);
+  const float x0 = (float)x.v[0];
+  float ns = 0.f;
+#pragma unroll
+  for (int d = 0; d < 6; ++d)
+    if ((on >> d) & 1u) ns += (float)Xe[nb[d]];
+  Real a[kSmallR];
+  small_rates<Real, MAXS>(A.sm, x.v, a);
+  f[0] = log1pf(x0);
+  f[1] = log1pf(n > 0 ? ns / (float)n : x0);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) f[2 + r] = r < (int)m.R ? log1pf((float)a[r]) : 0.f;
+  f[6] = logf(fminf(fmaxf((float)tau_ncr, 1e-30f), 1e30f));
+  float dt = 0.f;
+#pragma unroll
+  for (int s = 0; s < MAXS; ++s)
+    if (s < (int)m.S) dt += (float)n * ((float)sm_drate<Real>(A.sm, s) * (float)x.v[s]);
+  f[7] = log1pf(dt);
+}
+
 // ------------------------------------------------------------------------------------------------
 // warp-level tensor-core MLP
 // ------------------------------------------------------------------------------------------------

@@ -7,15 +7,22 @@
 // are contiguous 16-byte rows: the layer-1 tile is the stored features as they are (K chunk 0)
 // followed by a zero chunk (K padded from 8 to 16).  A weight image (64 output rows) has
 // LBO = 1024.  One tcgen05.mma (M = 128, N = 64, K = 16, kind::f16, BF16 x BF16 -> FP32) covers
-// two K chunks: one per tile for layer 1, four for layers 2 and 3.  Accumulators are TMEM columns
-// 0..63, lane = row, so after each layer each of the 128 threads reads its own row back with
+// two K chunks: one per tile for layer 1, four for layers 2 and 3.  Accumulators are 64 TMEM columns,
+// lane = row, so after each layer each of the 128 threads of a tile reads its own row back with
 // tcgen05.ld.32x32b (a warp reads the 32 lanes of its quarter), applies bias + ReLU, rounds to
 // BF16 and writes the next layer's A row.
 //
-// Synchronisation.  One thread issues the MMAs and commits them to an mbarrier; every thread
-// waits on it with an iteration limit.  A wait that runs out stops the CTA with a status; TMEM is
-// always freed.  A CTA allocates 64 TMEM columns, so the 512 columns of an SM hold 8 CTAs and its
-// shared memory keeps at most 5 on an SM: allocation never has to wait.
+// A tile is a chain of three MMA round trips, so what counts is the number of tiles in flight and the
+// instructions of the epilogue.  A CTA holds the weights once for four groups of 128 threads, each
+// with a tile, an mbarrier and 64 TMEM columns of its own: with two CTAs an SM has eight tiles in
+// flight (one-tile CTAs, each with its 18 KB of weights, fitted five).  The epilogue adds the bias two
+// columns at a time (add.rn.f32x2) and applies ReLU in the conversion to BF16.
+//
+// Synchronisation.  One thread of a group issues the MMAs and commits them to the group's mbarrier;
+// every thread of the group waits on it with an iteration limit, and one named barrier per layer
+// joins the group.  A wait that runs out stops the group with a status; TMEM is always freed.  A CTA
+// allocates 256 TMEM columns and its shared memory keeps at most two on an SM: allocation never has
+// to wait.
 #ifndef PLIS_TC_MLP_CUH_
 #define PLIS_TC_MLP_CUH_
 
@@ -83,9 +90,21 @@ __device__ __forceinline__ void ld16(uint32_t taddr, float v[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
+// two binary32 sums at once, and two values to BF16 (lo in the low half) with negative ones to zero
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+  return (uint64_t)__float_as_uint(hi) << 32 | __float_as_uint(lo);
+}
+__device__ __forceinline__ uint32_t relu_bf16x2(uint64_t v) {
+  uint32_t r;
+  asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;"
+      : "=r"(r)
+      : "f"(__uint_as_float((uint32_t)(v >> 32))), "f"(__uint_as_float((uint32_t)v)));
+  return r;
 }
 
 // byte offset of element (row, k) in a K-major canonical tile whose K chunks are `chunk` bytes apart
@@ -112,122 +131,156 @@ struct Params {
   float b4;
 };
 
-// Persistent tile kernel: shared memory of one CTA (128 threads, one 128-row tile at a time)
+// Persistent tile kernel: shared memory of one CTA, kGroups groups of 128 threads with a tile each
+constexpr uint32_t kGroups = 4;
+constexpr uint32_t kThreads = kGroups * 128;
 constexpr uint32_t kPOffW = 0;
-constexpr uint32_t kPOffA1 = kPOffW + kWImageBytes;  // features: K chunk 0 of the layer-1 A tile
-constexpr uint32_t kPOffZero = kPOffA1 + 2048;       // K chunk 1: zeros (the padding of K 8 -> 16)
-constexpr uint32_t kPOffA = kPOffZero + 2048;        // A tile of layers 2, 3
-constexpr uint32_t kPOffVec = kPOffA + kABytes;
-constexpr uint32_t kPOffBar = kPOffVec + 4 * 64 * 4;
-constexpr uint32_t kPSmemBytes = kPOffBar + 16;
-constexpr uint32_t kPTmemCols = 64;  // <= 8 CTAs per SM ever fit the 512 columns
-static_assert(kPSmemBytes * 6 > 228 * 1024, "at most 5 CTAs per SM");
+constexpr uint32_t kPOffA = kPOffW + kWImageBytes;            // A tiles of layers 2, 3, one per group
+constexpr uint32_t kPOffA1 = kPOffA + kGroups * kABytes;      // features: K chunk 0 of the layer-1 A tiles
+constexpr uint32_t kPOffZero = kPOffA1 + kGroups * 2048;      // K chunk 1: zeros (the padding of K 8 -> 16)
+constexpr uint32_t kPOffVec = kPOffZero + 2048;
+constexpr uint32_t kPOffBar = kPOffVec + 4 * 64 * 4;          // an mbarrier per group, then the TMEM address
+constexpr uint32_t kPSmemBytes = kPOffBar + kGroups * 8 + 16;
+constexpr uint32_t kPTmemCols = kGroups * 64;
+static_assert(kPSmemBytes * 3 > 228 * 1024 && kPTmemCols * 2 <= 512, "two CTAs per SM, and TMEM for both");
 
-// y[r] for the rows of `feats` (normalised BF16 features, 16 bytes per row, rows 0 .. 128*ntiles-1
-// readable) with the MLP on tcgen05.  Tiles are taken round robin; every CTA loads the weights once.
-// A wait that runs out sets *status and the CTA stops; TMEM is always freed.
-static __device__ void mlp_tiles(const Params& P, const uint4* __restrict__ feats, float* __restrict__ y, uint32_t nrows,
-                          uint32_t ntiles, uint8_t* smem, int* status, uint32_t wait_limit = 0) {
+__device__ __forceinline__ void group_sync(uint32_t group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory"); }
+
+// The MLP on tcgen05 for the rows of `feats` (normalised BF16 features, 16 bytes per row, rows
+// 0 .. 128 * ntiles - 1 readable), tiles taken round robin by the groups of the grid.
+// sink.begin(row) is called when a tile's rows are known (to start loads), sink.end(row, y) with its
+// result, by the thread that owns the row.  A wait that runs out sets *status and its group stops.
+template <class Sink>
+static __device__ __forceinline__ void mlp_tiles(const Params& P, const uint4* __restrict__ feats, uint32_t ntiles,
+                                                 uint8_t* smem, int* status, uint32_t wait_limit, Sink& sink) {
   if (wait_limit == 0) wait_limit = kWaitLimit;
-  __shared__ int s_err;
-  const uint32_t tid = threadIdx.x;  // blockDim.x == 128
-  const uint32_t warp = tid >> 5;
+  __shared__ int s_err[kGroups];
+  const uint32_t tid = threadIdx.x;  // blockDim.x == kThreads
+  const uint32_t group = tid >> 7, t = tid & 127u;
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar = sbase + kPOffBar;
-  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + kPOffBar + 8);
+  const uint32_t bar = sbase + kPOffBar + 8u * group;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + kPOffBar + kGroups * 8);
   float* vec = reinterpret_cast<float*>(smem + kPOffVec);
-  if (tid == 0) s_err = 0;
   {
     uint4* dst = reinterpret_cast<uint4*>(smem + kPOffW);
-    for (uint32_t i = tid; i < kWImageBytes / 16; i += 128) dst[i] = __ldg(&P.wimg[i]);
-    reinterpret_cast<uint4*>(smem + kPOffZero)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t i = tid; i < kWImageBytes / 16; i += kThreads) dst[i] = __ldg(&P.wimg[i]);
+    if (tid < 128) reinterpret_cast<uint4*>(smem + kPOffZero)[tid] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < 64) {
       vec[tid] = __ldg(&P.b1[tid]);
       vec[64 + tid] = __ldg(&P.b2[tid]);
       vec[128 + tid] = __ldg(&P.b3[tid]);
       vec[192 + tid] = __ldg(&P.w4[tid]);
     }
-    if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    if (warp == 0) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + kPOffBar + 8),
+    if (t == 0) {
+      s_err[group] = 0;
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    }
+    if (tid < 32) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
                    "r"(kPTmemCols)
                    : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
   }
   fence_before();
+  fence_async_smem();
   __syncthreads();
   fence_after();
-  const uint32_t tmem = *slot;
-  const uint32_t my_cols = tmem + ((32u * warp) << 16);
-  const volatile int* err = &s_err;
+  const uint32_t tmem = *slot + 64u * group;
+  const uint32_t my_cols = tmem + ((t & 96u) << 16);  // lanes 32 * (warp of the group)
+  uint8_t* a1 = smem + kPOffA1 + 2048u * group;
+  uint8_t* a = smem + kPOffA + kABytes * group;
+  const uint32_t sa1 = sbase + kPOffA1 + 2048u * group, sa = sbase + kPOffA + kABytes * group;
+  volatile int* err = &s_err[group];
   uint32_t phase = 0;
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint32_t r = tile * 128u + tid;
-    // row tid of chunk 0 of the layer-1 A tile sits at tid * 16: the features as they are stored
-    reinterpret_cast<uint4*>(smem + kPOffA1)[tid] = feats[r];
+  const uint32_t first = blockIdx.x * kGroups + group, step = gridDim.x * kGroups;
+  uint4 next = first < ntiles ? feats[first * 128u + t] : make_uint4(0u, 0u, 0u, 0u);
+  bool ok = true;
+  for (uint32_t tile = first; tile < ntiles && ok; tile += step) {
+    const uint32_t row = tile * 128u + t;
+    // row t of chunk 0 of the layer-1 A tile sits at t * 16: the features as they are stored
+    reinterpret_cast<uint4*>(a1)[t] = next;
+    sink.begin(row);
+    if (tile + step < ntiles) next = feats[(tile + step) * 128u + t];
     fence_before();
     fence_async_smem();
-    __syncthreads();
-    bool ok = true;
+    group_sync(group);
     float out = 0.f;
-    for (int layer = 0; layer < 3 && ok; ++layer) {
-      if (tid == 0 && !*err) {
+#pragma unroll
+    for (int layer = 0; layer < 3; ++layer) {
+      if (t == 0) {
         fence_after();
         if (layer == 0) {
-          mma(tmem, sdesc(sbase + kPOffA1, kPOffZero - kPOffA1, 128), sdesc(sbase + kPOffW, 1024, 128), 0u);
+          mma(tmem, sdesc(sa1, sbase + kPOffZero - sa1, 128), sdesc(sbase + kPOffW, 1024, 128), 0u);
         } else {
-          const uint32_t wofs = kPOffW + kW1Bytes + (layer == 1 ? 0u : kWBytes);
+          const uint32_t w = sbase + kPOffW + kW1Bytes + (layer == 1 ? 0u : kWBytes);
           for (uint32_t ks = 0; ks < 4; ++ks)
-            mma(tmem, sdesc(sbase + kPOffA + ks * 2u * 2048u, 2048, 128), sdesc(sbase + wofs + ks * 2u * 1024u, 1024, 128),
-                ks > 0 ? 1u : 0u);
+            mma(tmem, sdesc(sa + ks * 2u * 2048u, 2048, 128), sdesc(w + ks * 2u * 1024u, 1024, 128), ks > 0 ? 1u : 0u);
         }
         commit(bar);
       }
-      bool got = !*err && wait_phase(bar, phase & 1u, (volatile int*)err, wait_limit);
+      const bool got = wait_phase(bar, phase & 1u, err, wait_limit);
       phase += 1;
       fence_after();
-      ok = __syncthreads_and(got && !*err) != 0;
-      if (!ok) break;
-      if (layer < 2) {
-        const float* b = vec + 64 * layer;
-        uint8_t* a = smem + kPOffA;
+      __syncwarp();
+      if (__all_sync(0xffffffffu, got)) {
+        if (layer < 2) {
+          const ulonglong2* b = reinterpret_cast<const ulonglong2*>(vec + 64 * layer);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float v[16];
-          ld16(my_cols + 16u * c, v);
-          uint32_t p[8];
+          for (int c = 0; c < 4; ++c) {
+            float v[16];
+            ld16(my_cols + 16u * c, v);
+            uint32_t p[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            p[i] = bf16x2(fmaxf(v[2 * i] + b[16 * c + 2 * i], 0.f), fmaxf(v[2 * i + 1] + b[16 * c + 2 * i + 1], 0.f));
-          *reinterpret_cast<uint4*>(a + canon(tid, 16u * c, 2048)) = make_uint4(p[0], p[1], p[2], p[3]);
-          *reinterpret_cast<uint4*>(a + canon(tid, 16u * c + 8u, 2048)) = make_uint4(p[4], p[5], p[6], p[7]);
+            for (int i = 0; i < 4; ++i) {
+              const ulonglong2 bb = b[4 * c + i];
+              p[2 * i] = relu_bf16x2(add2(pair(v[4 * i], v[4 * i + 1]), bb.x));
+              p[2 * i + 1] = relu_bf16x2(add2(pair(v[4 * i + 2], v[4 * i + 3]), bb.y));
+            }
+            *reinterpret_cast<uint4*>(a + canon(t, 16u * c, 2048)) = make_uint4(p[0], p[1], p[2], p[3]);
+            *reinterpret_cast<uint4*>(a + canon(t, 16u * c + 8u, 2048)) = make_uint4(p[4], p[5], p[6], p[7]);
+          }
+        } else {
+          const float4* b = reinterpret_cast<const float4*>(vec + 128);
+          const float4* w = reinterpret_cast<const float4*>(vec + 192);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            float v[16];
+            ld16(my_cols + 16u * c, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 bb = b[4 * c + i], ww = w[4 * c + i];
+              out = out + fmaxf(v[4 * i] + bb.x, 0.f) * ww.x;
+              out = out + fmaxf(v[4 * i + 1] + bb.y, 0.f) * ww.y;
+              out = out + fmaxf(v[4 * i + 2] + bb.z, 0.f) * ww.z;
+              out = out + fmaxf(v[4 * i + 3] + bb.w, 0.f) * ww.w;
+            }
+          }
+          out = out + P.b4;
         }
       } else {
-        const float* b = vec + 128;
-        const float* w = vec + 192;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float v[16];
-          ld16(my_cols + 16u * c, v);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) out = out + fmaxf(v[i] + b[16 * c + i], 0.f) * w[16 * c + i];
-        }
-        out = out + P.b4;
+        *err = 1;
       }
       fence_before();
       fence_async_smem();
-      __syncthreads();
+      group_sync(group);
+      if (*err) {  // the same for the whole group: only its own threads set it, before the barrier
+        ok = false;
+        break;
+      }
     }
-    if (!ok) break;
-    if (r < nrows) y[r] = out;
+    if (ok) sink.end(row, out);
+  }
+  if (!ok) {  // the MMAs in flight finish before their TMEM is freed
+    int late = 0;
+    wait_phase(bar, (phase - 1u) & 1u, &late, kWaitLimit);
   }
   fence_before();
   __syncthreads();
   fence_after();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kPTmemCols) : "memory");
-  if (tid == 0 && s_err) atomicExch(status, 6 /* PLIS_ERR_TIMEOUT */);
+  if (tid < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*slot), "r"(kPTmemCols) : "memory");
+  if (t == 0 && s_err[group]) atomicExch(status, 6 /* PLIS_ERR_TIMEOUT */);
 }
 
 }  // namespace tc
