@@ -423,191 +423,294 @@ __global__ void k_predict(const LearnedParams* __restrict__ P, const float* __re
 // ------------------------------------------------------------------------------------------------
 // training
 // ------------------------------------------------------------------------------------------------
+// One CTA takes 128 records through the forward and backward pass.  The work is 26,000 multiply-adds per
+// record in binary32, each a product rounded and then added (no fma, as everywhere in this library),
+// and every sum runs in a fixed order; 128 CTAs of a 16,384-record batch take 27 us at the FP32 rate of
+// 128 SMs.  So the layout serves the issue slots: activations record-major with a pitch of 68 floats
+// (16-byte loads of four consecutive units, conflict-free across records), register tiles of 32 or 64
+// sums, products and sums two units at a time (mul / add.rn.f32x2, the same roundings), the weights of
+// the backward pass transposed once by the Adam kernel, and the weight gradient of a layer, its backward
+// pass and its bias gradient side by side on warps 0-3, 4-7 and 8-9.  Measured on one B200, 16,384
+// records: 45 us an Adam step, where one thread per record with scalar loads took 115.
 constexpr int kTB = 128;          // records per training CTA
-constexpr int kLd = kTB + 1;      // row pitch of the activation tiles (bank-conflict-free columns)
-constexpr size_t kTrainSmem = (size_t)(kNParams + (kFeat + 3 * kHid) * kLd + kTB + 32) * sizeof(float);
+constexpr int kTT = 320;          // its threads
+constexpr int kLd = kHid + 4;     // floats per record of an activation buffer
+constexpr int kLdF = kFeat + 4;   // floats per record of the features
+constexpr int kNWt = 2 * kHid * kHid;           // W2^T, W3^T
+constexpr int kSmW = (kNParams + 3) & ~3;       // shared memory, in floats: the weights,
+constexpr int kSmWt = kSmW;                     // the transposed weights,
+constexpr int kSmF = kSmWt + kNWt;              // features,
+constexpr int kSmH = kSmF + kTB * kLdF;         // four activation buffers,
+constexpr int kSmDy = kSmH + 4 * kTB * kLd;     // output gradients, warp sums
+constexpr size_t kTrainSmem = (size_t)(kSmDy + kTB + 32) * sizeof(float);
+static_assert(kTrainSmem <= 227 * 1024, "one training CTA per SM");
 constexpr int kStatN = 2 * kFeat + 2;  // sums of f, f^2, label, count
 
-// dW[k][j] = sum_u A[k][u] G[j][u] for a 64x64 layer: each thread a 4x8 tile
-__device__ __forceinline__ void grad_tile(const float* A, const float* G, float* out, int t) {
-  const int k0 = (t >> 3) * 4, j0 = (t & 7) * 8;
-  float acc[4][8];
+__device__ __forceinline__ uint64_t dup2(float v) { return tc::pair(v, v); }
+// Two products, each rounded: a b + (-0), with the -0 from a kernel argument, which the assembler cannot
+// fold (it fuses a mul.rn.f32x2, or a fma with a constant -0, with the add that follows, although both
+// are rounded operations: measured as other bits).
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b, uint64_t nz) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+  return r;
+}
+constexpr uint64_t kMinusZeros = 0x8000000080000000ull;
+__device__ __forceinline__ float lo2(uint64_t v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+// acc[i][2p], acc[i][2p + 1] += sum over k = 0 .. K-1, in order, of In[u_i][k] * W[k][j], for the tile's NU records
+// u_i = u0 + i * du and its units j = 4 jt .. + 3 (pairs p = 0, 1) and 32 + 4 jt .. + 3 (p = 2, 3).
+template <int NU>
+__device__ __forceinline__ void tile_sums(const float* In, int ld, int K, const float* W, int ldw, int u0, int du, int jt,
+                                          uint64_t nz, uint64_t acc[NU][4]) {
+#pragma unroll 1
+  for (int k = 0; k < K; k += 4) {
+    float4 h[NU];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < NU; ++i) h[i] = *reinterpret_cast<const float4*>(In + (u0 + i * du) * ld + k);
 #pragma unroll
-    for (int l = 0; l < 8; ++l) acc[i][l] = 0.f;
+    for (int q = 0; q < 4; ++q) {
+      const ulonglong2 wa = *reinterpret_cast<const ulonglong2*>(W + (k + q) * ldw + 4 * jt);
+      const ulonglong2 wb = *reinterpret_cast<const ulonglong2*>(W + (k + q) * ldw + 32 + 4 * jt);
+#pragma unroll
+      for (int i = 0; i < NU; ++i) {
+        const uint64_t hh = dup2(q == 0 ? h[i].x : q == 1 ? h[i].y : q == 2 ? h[i].z : h[i].w);
+        acc[i][0] = tc::add2(acc[i][0], mul2(hh, wa.x, nz));
+        acc[i][1] = tc::add2(acc[i][1], mul2(hh, wa.y, nz));
+        acc[i][2] = tc::add2(acc[i][2], mul2(hh, wb.x, nz));
+        acc[i][3] = tc::add2(acc[i][3], mul2(hh, wb.y, nz));
+      }
+    }
+  }
+}
+
+// H[u][j] = relu(b[j] + sum_k In[u][k] W[k][j]) by threads 0..255
+__device__ __forceinline__ void forward_layer(const float* In, int ld, int K, float* H, const float* W, const float* b, int t,
+                                              uint64_t nz) {
+  const int jt = t & 7, u0 = t >> 3;
+  uint64_t acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    acc[i][0] = *reinterpret_cast<const uint64_t*>(b + 4 * jt);
+    acc[i][1] = *reinterpret_cast<const uint64_t*>(b + 4 * jt + 2);
+    acc[i][2] = *reinterpret_cast<const uint64_t*>(b + 32 + 4 * jt);
+    acc[i][3] = *reinterpret_cast<const uint64_t*>(b + 32 + 4 * jt + 2);
+  }
+  tile_sums<4>(In, ld, K, W, kHid, u0, 32, jt, nz, acc);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float* row = H + (u0 + 32 * i) * kLd;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      *reinterpret_cast<float4*>(row + 32 * q + 4 * jt) =
+          make_float4(fmaxf(lo2(acc[i][2 * q]), 0.f), fmaxf(hi2(acc[i][2 * q]), 0.f), fmaxf(lo2(acc[i][2 * q + 1]), 0.f),
+                      fmaxf(hi2(acc[i][2 * q + 1]), 0.f));
+  }
+}
+
+// Out[u][k] = H[u][k] > 0 ? sum_j G[u][j] W[k][j] : 0 with Wt[j][k], by 128 threads
+__device__ __forceinline__ void backprop_layer(const float* G, const float* Wt, const float* H, float* Out, int t, uint64_t nz) {
+  const int jt = t & 7, u0 = t >> 3;
+  uint64_t acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int p = 0; p < 4; ++p) acc[i][p] = 0ull;
+  tile_sums<8>(G, kLd, kHid, Wt, kHid, u0, 16, jt, nz, acc);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int u = u0 + 16 * i;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float4 h = *reinterpret_cast<const float4*>(H + u * kLd + 32 * q + 4 * jt);
+      *reinterpret_cast<float4*>(Out + u * kLd + 32 * q + 4 * jt) =
+          make_float4(h.x > 0.f ? lo2(acc[i][2 * q]) : 0.f, h.y > 0.f ? hi2(acc[i][2 * q]) : 0.f,
+                      h.z > 0.f ? lo2(acc[i][2 * q + 1]) : 0.f, h.w > 0.f ? hi2(acc[i][2 * q + 1]) : 0.f);
+    }
+  }
+}
+
+// out[k][j] = sum over records in order of A[u][k] G[u][j] for a 64 x 64 layer, by 128 threads: 8 x 4 sums each
+__device__ __forceinline__ void grad_tile(const float* A, const float* G, float* out, int t, uint64_t nz) {
+  const int k0 = (t >> 4) * 8, j0 = (t & 15) * 4;
+  uint64_t acc[8][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = 0ull;
+#pragma unroll 2
   for (int u = 0; u < kTB; ++u) {
-    float a[4], g[8];
+    const float4 a0 = *reinterpret_cast<const float4*>(A + u * kLd + k0);
+    const float4 a1 = *reinterpret_cast<const float4*>(A + u * kLd + k0 + 4);
+    const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(G + u * kLd + j0);
+    const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = A[(k0 + i) * kLd + u];
-#pragma unroll
-    for (int l = 0; l < 8; ++l) g[l] = G[(j0 + l) * kLd + u];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int l = 0; l < 8; ++l) acc[i][l] = acc[i][l] + a[i] * g[l];
+    for (int i = 0; i < 8; ++i) {
+      const uint64_t aa = dup2(a[i]);
+      acc[i][0] = tc::add2(acc[i][0], mul2(aa, g.x, nz));
+      acc[i][1] = tc::add2(acc[i][1], mul2(aa, g.y, nz));
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 8; ++i)  // the rows of a CTA's gradient are not 16-byte aligned (8961 floats)
 #pragma unroll
-    for (int l = 0; l < 8; ++l) out[(k0 + i) * kHid + j0 + l] = acc[i][l];
+    for (int l = 0; l < 4; ++l) out[(k0 + i) * kHid + j0 + l] = l & 1 ? hi2(acc[i][l >> 1]) : lo2(acc[i][l >> 1]);
 }
 
-// column t: H[k] <- (sum_j G[j] W[k][j]) * (H[k] > 0)
-__device__ __forceinline__ void backprop_layer(const float* G, float* H, const float* W, int t) {
-  float acc[kHid];
-#pragma unroll
-  for (int k = 0; k < kHid; ++k) acc[k] = 0.f;
-  for (int j = 0; j < kHid; ++j) {
-    const float gj = G[j * kLd + t];
-#pragma unroll
-    for (int k = 0; k < kHid; ++k) acc[k] = acc[k] + gj * W[k * kHid + j];
-  }
-#pragma unroll
-  for (int k = 0; k < kHid; ++k) {
-    const float h = H[k * kLd + t];
-    H[k * kLd + t] = h > 0.f ? acc[k] : 0.f;
-  }
-}
-
-// column t: H[j] <- relu(b[j] + sum_k In[k] W[k][j])
-__device__ __forceinline__ void forward_layer(const float* In, float* H, const float* W, const float* b, int t) {
-  float acc[kHid];
-#pragma unroll
-  for (int j = 0; j < kHid; ++j) acc[j] = b[j];
-  for (int k = 0; k < kHid; ++k) {
-    const float h = In[k * kLd + t];
-#pragma unroll
-    for (int j = 0; j < kHid; ++j) acc[j] = acc[j] + h * W[k * kHid + j];
-  }
-#pragma unroll
-  for (int j = 0; j < kHid; ++j) H[j * kLd + t] = fmaxf(acc[j], 0.f);
+// sum over records in order of G[u][j]
+__device__ __forceinline__ float column_sum(const float* G, int j) {
+  float s = 0.f;
+#pragma unroll 8
+  for (int u = 0; u < kTB; ++u) s = s + G[u * kLd + j];
+  return s;
 }
 
 // One CTA: forward and backward pass of 128 records; writes its summed gradient (already scaled by
 // inv_batch) and its summed loss.  fixed: record blockIdx*128 + t; else Philox-sampled records.
-__global__ void __launch_bounds__(kTB) k_train(const TraceRec* __restrict__ recs, uint64_t n,
-                                                const float* __restrict__ W, float* __restrict__ partial,
-                                                float* __restrict__ loss_out, uint64_t iter, uint32_t seed_lo,
-                                                uint32_t seed_hi, float quantile, int fixed, float inv_batch) {
-  extern __shared__ float sm[];
+__global__ void __launch_bounds__(kTT, 1) k_train(const TraceRec* __restrict__ recs, uint64_t n, const float* W,
+                                                  const float* Wt, float* __restrict__ partial, float* __restrict__ loss_out,
+                                                  uint64_t iter, uint32_t seed_lo, uint32_t seed_hi, float quantile, int fixed,
+                                                  float inv_batch, uint64_t nz) {
+  extern __shared__ __align__(16) float sm[];
   float* sW = sm;
-  float* F = sW + kNParams;
-  float* H1 = F + kFeat * kLd;
-  float* H2 = H1 + kHid * kLd;
-  float* H3 = H2 + kHid * kLd;
-  float* dy = H3 + kHid * kLd;
+  float* sWt = sm + kSmWt;
+  float* F = sm + kSmF;
+  float* H1 = sm + kSmH;
+  float* H2 = H1 + kTB * kLd;
+  float* H3 = H2 + kTB * kLd;
+  float* G = H3 + kTB * kLd;
+  float* dy = sm + kSmDy;
   float* red = dy + kTB;
   const int t = threadIdx.x;
-  for (int i = t; i < kNParams; i += kTB) sW[i] = W[i];
-  uint64_t idx;
-  bool use;
-  if (fixed) {
-    idx = (uint64_t)blockIdx.x * kTB + t;
-    use = idx < n;
-  } else {
-    plis_u32x4 ctr = {(uint32_t)(blockIdx.x * kTB + t), (uint32_t)iter, (uint32_t)(iter >> 32), 0x7A11u};
-    const plis_u32x4 r = plis_philox4x32_10(ctr, seed_lo, seed_hi);
-    idx = (((uint64_t)r.x << 32) | r.y) % n;
-    use = true;
-  }
+  // the records do not depend on the previous step's weights: fetched before the wait for them
   float f[kFeat], label = 0.f;
-  if (use) {
-    const TraceRec& r = recs[idx];
-    label = r.label;
-    use = !isnan(label);
-#pragma unroll
-    for (int k = 0; k < kFeat; ++k) f[k] = (r.f[k] - W[kNParams + k]) * W[kNParams + kFeat + k];
+  bool use = false;
+  if (t < kTB) {
+    uint64_t idx;
+    if (fixed) {
+      idx = (uint64_t)blockIdx.x * kTB + t;
+      use = idx < n;
+    } else {
+      plis_u32x4 ctr = {(uint32_t)(blockIdx.x * kTB + t), (uint32_t)iter, (uint32_t)(iter >> 32), 0x7A11u};
+      const plis_u32x4 r = plis_philox4x32_10(ctr, seed_lo, seed_hi);
+      idx = (((uint64_t)r.x << 32) | r.y) % n;
+      use = true;
+    }
+    if (use) {
+      const float4* q = reinterpret_cast<const float4*>(recs + idx);
+      const float4 fa = __ldg(q), fb = __ldg(q + 1), fc = __ldg(q + 2);
+      f[0] = fa.x; f[1] = fa.y; f[2] = fa.z; f[3] = fa.w;
+      f[4] = fb.x; f[5] = fb.y; f[6] = fb.z; f[7] = fb.w;
+      label = fc.z;
+      use = !isnan(label);
+    }
   }
-  if (!use) {
+  pdl_entry();
+  for (int i = t; i < kNParams; i += kTT) sW[i] = __ldcg(W + i);
+  for (int i = t; i < kNWt / 4; i += kTT) reinterpret_cast<float4*>(sWt)[i] = __ldcg(reinterpret_cast<const float4*>(Wt) + i);
+  if (t < kTB) {
 #pragma unroll
-    for (int k = 0; k < kFeat; ++k) f[k] = 0.f;
+    for (int k = 0; k < kFeat; ++k)
+      F[t * kLdF + k] = use ? (f[k] - __ldcg(W + kNParams + k)) * __ldcg(W + kNParams + kFeat + k) : 0.f;
   }
-#pragma unroll
-  for (int k = 0; k < kFeat; ++k) F[k * kLd + t] = f[k];
   __syncthreads();
-  // forward
-  for (int j = 0; j < kHid; ++j) {
-    float s = sW[kOffB1 + j];
+  if (t < 256) forward_layer(F, kLdF, kFeat, H1, sW + kOffW1, sW + kOffB1, t, nz);
+  __syncthreads();
+  if (t < 256) forward_layer(H1, kLd, kHid, H2, sW + kOffW2, sW + kOffB2, t, nz);
+  __syncthreads();
+  if (t < 256) forward_layer(H2, kLd, kHid, H3, sW + kOffW3, sW + kOffB3, t, nz);
+  __syncthreads();
+  if (t < kTB) {
+    float y = sW[kOffB4];
+#pragma unroll 4
+    for (int j = 0; j < kHid; j += 4) {
+      const float4 h = *reinterpret_cast<const float4*>(H3 + t * kLd + j);
+      const float4 w = *reinterpret_cast<const float4*>(sW + kOffW4 + j);
+      y = y + h.x * w.x;
+      y = y + h.y * w.y;
+      y = y + h.z * w.z;
+      y = y + h.w * w.w;
+    }
+    float loss = 0.f, g = 0.f;
+    if (use) {
+      const float res = label - y;
+      loss = res >= 0.f ? quantile * res : (quantile - 1.f) * res;
+      g = res > 0.f ? -quantile : (res < 0.f ? 1.f - quantile : 0.f);
+    }
+    dy[t] = g * inv_batch;
 #pragma unroll
-    for (int k = 0; k < kFeat; ++k) s = s + f[k] * sW[kOffW1 + k * kHid + j];
-    H1[j * kLd + t] = fmaxf(s, 0.f);
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if ((t & 31) == 0) red[t >> 5] = loss;
   }
-  forward_layer(H1, H2, sW + kOffW2, sW + kOffB2, t);
-  forward_layer(H2, H3, sW + kOffW3, sW + kOffB3, t);
-  float y = sW[kOffB4];
-  for (int j = 0; j < kHid; ++j) y = y + H3[j * kLd + t] * sW[kOffW4 + j];
-  float loss = 0.f, g = 0.f;
-  if (use) {
-    const float res = label - y;
-    loss = res >= 0.f ? quantile * res : (quantile - 1.f) * res;
-    g = res > 0.f ? -quantile : (res < 0.f ? 1.f - quantile : 0.f);
-  }
-  dy[t] = g * inv_batch;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-  if ((t & 31) == 0) red[t >> 5] = loss;
   __syncthreads();
   if (t == 0) loss_out[blockIdx.x] = red[0] + red[1] + red[2] + red[3];
   float* P = partial + (size_t)blockIdx.x * kNParams;
-  // output layer
-  if (t < kHid) {
+  // output layer, and G = dy w4 relu'(H3)
+  if (t >= 256) {
+    const int j = t - 256;
     float s = 0.f;
-    for (int u = 0; u < kTB; ++u) s = s + H3[t * kLd + u] * dy[u];
-    P[kOffW4 + t] = s;
-  } else if (t == kHid) {
-    float s = 0.f;
-    for (int u = 0; u < kTB; ++u) s = s + dy[u];
-    P[kOffB4] = s;
-  }
-  __syncthreads();
-  {  // G3 = dy * w4 * relu'(H3), in place
-    const float d = dy[t];
-    for (int j = 0; j < kHid; ++j) {
-      const float h = H3[j * kLd + t];
-      H3[j * kLd + t] = h > 0.f ? d * sW[kOffW4 + j] : 0.f;
+#pragma unroll 8
+    for (int u = 0; u < kTB; ++u) s = s + H3[u * kLd + j] * dy[u];
+    P[kOffW4 + j] = s;
+  } else {
+    if (t == 0) {
+      float s = 0.f;
+      for (int u = 0; u < kTB; ++u) s = s + dy[u];
+      P[kOffB4] = s;
+    }
+    const int j = (t & 15) * 4;
+    const float4 w = *reinterpret_cast<const float4*>(sW + kOffW4 + j);
+#pragma unroll
+    for (int u = t >> 4; u < kTB; u += 16) {
+      const float4 h = *reinterpret_cast<const float4*>(H3 + u * kLd + j);
+      const float d = dy[u];
+      *reinterpret_cast<float4*>(G + u * kLd + j) = make_float4(h.x > 0.f ? d * w.x : 0.f, h.y > 0.f ? d * w.y : 0.f,
+                                                                h.z > 0.f ? d * w.z : 0.f, h.w > 0.f ? d * w.w : 0.f);
     }
   }
   __syncthreads();
-  grad_tile(H2, H3, P + kOffW3, t);
-  if (t < kHid) {
-    float s = 0.f;
-    for (int u = 0; u < kTB; ++u) s = s + H3[t * kLd + u];
-    P[kOffB3 + t] = s;
-  }
+  // layer 3: gradients, and the gradient of layer 2's units into H3
+  if (t < 128) grad_tile(H2, G, P + kOffW3, t, nz);
+  else if (t < 256) backprop_layer(G, sWt + kHid * kHid, H2, H3, t - 128, nz);
+  else P[kOffB3 + t - 256] = column_sum(G, t - 256);
   __syncthreads();
-  backprop_layer(H3, H2, sW + kOffW3, t);  // G2 in place of H2
+  // layer 2, and the gradient of layer 1's units into G
+  if (t < 128) grad_tile(H1, H3, P + kOffW2, t, nz);
+  else if (t < 256) backprop_layer(H3, sWt, H1, G, t - 128, nz);
+  else P[kOffB2 + t - 256] = column_sum(H3, t - 256);
   __syncthreads();
-  grad_tile(H1, H2, P + kOffW2, t);
-  if (t < kHid) {
-    float s = 0.f;
-    for (int u = 0; u < kTB; ++u) s = s + H2[t * kLd + u];
-    P[kOffB2 + t] = s;
-  }
-  __syncthreads();
-  backprop_layer(H2, H1, sW + kOffW2, t);  // G1 in place of H1
-  __syncthreads();
-  for (int e = t; e < kFeat * kHid; e += kTB) {
-    const int k = e / kHid, j = e % kHid;
-    float s = 0.f;
-    for (int u = 0; u < kTB; ++u) s = s + F[k * kLd + u] * H1[j * kLd + u];
-    P[kOffW1 + e] = s;
-  }
-  if (t < kHid) {
-    float s = 0.f;
-    for (int u = 0; u < kTB; ++u) s = s + H1[t * kLd + u];
-    P[kOffB1 + t] = s;
+  if (t < 256) {  // layer 1: two sums per thread
+    const int k = t >> 5, j = (t & 31) * 2;
+    uint64_t s = 0ull;
+#pragma unroll 8
+    for (int u = 0; u < kTB; ++u)
+      s = tc::add2(s, mul2(dup2(F[u * kLdF + k]), *reinterpret_cast<const uint64_t*>(G + u * kLd + j), nz));
+    P[kOffW1 + k * kHid + j] = lo2(s);
+    P[kOffW1 + k * kHid + j + 1] = hi2(s);
+  } else {
+    P[kOffB1 + t - 256] = column_sum(G, t - 256);
   }
 }
 
+// the transposed weights of the backward pass: Wt[layer][j][k] = W_layer[k][j], layers 2 and 3
+__device__ __forceinline__ void put_transposed(float* Wt, int p, float v) {
+  const int layer = p >= kOffW3 ? 1 : 0, e = p - (layer ? kOffW3 : kOffW2);
+  if (p >= kOffW2 && e < kHid * kHid) Wt[layer * kHid * kHid + (e % kHid) * kHid + e / kHid] = v;
+}
+__global__ void k_transpose(const float* __restrict__ W, float* __restrict__ Wt) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < kNParams) put_transposed(Wt, p, W[p]);
+}
+
 // gradient = sum over CTAs (fixed order); Adam step when lr > 0, else the gradient into out
-__global__ void k_adam(float* __restrict__ W, float* __restrict__ m, float* __restrict__ v,
-                       const float* __restrict__ partial, uint32_t nblk, float lr, float bc1, float bc2,
-                       float* __restrict__ out) {
+__global__ void __launch_bounds__(64) k_adam(float* W, float* Wt, float* __restrict__ m, float* __restrict__ v,
+                                             const float* __restrict__ partial, uint32_t nblk, float lr, float bc1, float bc2,
+                                             float* __restrict__ out) {
+  pdl_entry();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kNParams) return;
   float g = 0.f;
-  for (uint32_t b = 0; b < nblk; ++b) g = g + partial[(size_t)b * kNParams + p];
+#pragma unroll 16
+  for (uint32_t b = 0; b < nblk; ++b) g = g + __ldcg(&partial[(size_t)b * kNParams + p]);
   if (out) {
     out[p] = g;
     return;
@@ -617,7 +720,9 @@ __global__ void k_adam(float* __restrict__ W, float* __restrict__ m, float* __re
   const float vv = b2 * v[p] + (1.f - b2) * g * g;
   m[p] = mm;
   v[p] = vv;
-  W[p] = W[p] - lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
+  const float w = W[p] - lr * (mm / bc1) / (sqrtf(vv / bc2) + eps);
+  W[p] = w;
+  put_transposed(Wt, p, w);
 }
 
 // per-CTA sums of the usable records' features, squares, labels and count
@@ -748,6 +853,7 @@ int Learner::create(uint64_t capacity, int device) {
   int rc;
   if ((rc = dmalloc((void**)&recs_, capacity * sizeof(TraceRec)))) return rc;
   if ((rc = dmalloc((void**)&w_, kNWeights * sizeof(float)))) return rc;
+  if ((rc = dmalloc((void**)&wt_, kNWt * sizeof(float)))) return rc;
   if ((rc = dmalloc((void**)&m_, kNParams * sizeof(float)))) return rc;
   if ((rc = dmalloc((void**)&v_, kNParams * sizeof(float)))) return rc;
   if ((rc = dmalloc((void**)&stats_, (kStatBlocks * kStatN + 2) * sizeof(double)))) return rc;
@@ -842,14 +948,15 @@ int Learner::train(const plis_train_params& p, plis_train_report* out) {
   std::vector<float> lossbuf(nblk);
   double loss_first = 0.0, loss_last = 0.0;
   const float inv_b = 1.f / (float)p.batch;
+  k_transpose<<<(kNParams + 255) / 256, 256, 0, stream_>>>(w_, wt_);
   double b1t = 1.0, b2t = 1.0;
   for (uint64_t it = 0; it < p.iterations; ++it) {
-    k_train<<<nblk, kTB, kTrainSmem, stream_>>>(recs_, count_, w_, partial_, loss_, it, (uint32_t)p.seed,
-                                                 (uint32_t)(p.seed >> 32), p.quantile, 0, inv_b);
+    launch_pdl(k_train, dim3(nblk), dim3(kTT), kTrainSmem, stream_, (const TraceRec*)recs_, count_, (const float*)w_,
+               (const float*)wt_, partial_, loss_, it, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), p.quantile, 0, inv_b, kMinusZeros);
     b1t *= 0.9;
     b2t *= 0.999;
-    k_adam<<<(kNParams + 255) / 256, 256, 0, stream_>>>(w_, m_, v_, partial_, nblk, p.learning_rate,
-                                                         (float)(1.0 - b1t), (float)(1.0 - b2t), nullptr);
+    launch_pdl(k_adam, dim3((kNParams + 63) / 64), dim3(64), 0, stream_, w_, wt_, m_, v_, (const float*)partial_, nblk,
+               p.learning_rate, (float)(1.0 - b1t), (float)(1.0 - b2t), (float*)nullptr);
     if (it == 0 || it + 1 == p.iterations) {
       PLIS_LCU(cudaMemcpyAsync(lossbuf.data(), loss_, nblk * sizeof(float), cudaMemcpyDeviceToHost, stream_));
       PLIS_LCU(cudaStreamSynchronize(stream_));
@@ -885,9 +992,10 @@ int Learner::gradient(float* grad, double* loss, float quantile) {
   if (rc) return rc;
   float* d_g = nullptr;
   PLIS_LCU(cudaMalloc(&d_g, kNParams * sizeof(float)));
-  k_train<<<nblk, kTB, kTrainSmem, stream_>>>(recs_, count_, w_, partial_, loss_, 0, 0, 0, quantile, 1,
-                                               1.f / (float)count_);
-  k_adam<<<(kNParams + 255) / 256, 256, 0, stream_>>>(w_, m_, v_, partial_, nblk, 0.f, 1.f, 1.f, d_g);
+  k_transpose<<<(kNParams + 255) / 256, 256, 0, stream_>>>(w_, wt_);
+  k_train<<<nblk, kTT, kTrainSmem, stream_>>>(recs_, count_, w_, wt_, partial_, loss_, 0, 0, 0, quantile, 1,
+                                               1.f / (float)count_, kMinusZeros);
+  k_adam<<<(kNParams + 63) / 64, 64, 0, stream_>>>(w_, wt_, m_, v_, partial_, nblk, 0.f, 1.f, 1.f, d_g);
   std::vector<float> lossbuf(nblk);
   cudaError_t e = cudaMemcpyAsync(grad, d_g, kNParams * sizeof(float), cudaMemcpyDeviceToHost, stream_);
   if (e == cudaSuccess) e = cudaMemcpyAsync(lossbuf.data(), loss_, nblk * sizeof(float), cudaMemcpyDeviceToHost, stream_);

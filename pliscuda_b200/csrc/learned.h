@@ -93,6 +93,7 @@ class Learner {
   uint64_t capacity_ = 0, count_ = 0;
   TraceRec* recs_ = nullptr;
   float* w_ = nullptr;        // master weights [kNWeights]
+  float* wt_ = nullptr;       // W2^T and W3^T for the backward pass of the training kernel
   float* m_ = nullptr;        // Adam moments
   float* v_ = nullptr;
   float* partial_ = nullptr;  // per-CTA gradients
