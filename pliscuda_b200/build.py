@@ -34,7 +34,7 @@ CXX_FLAGS = ["-std=c++17", "-O2", "-fPIC", "-ffp-contract=off", "-Wall", "-Wextr
 SOURCES = ["inst_f64.cu", "inst_f32.cu", "batch_f64.cu", "batch_f32.cu", "engine.cu", "batch.cu", "noalloc.cu",
            "learned.cu",
            "capi.cpp", "loader.cpp", "simulate.cpp", "plis_model.cpp"]
-HEADERS = ["engine_kernels.cuh", "small_step.cuh", "net_step.cuh", "batch_kernels.cuh", "batch.h", "engine.cuh", "engine.h", "learned.h",
+HEADERS = ["engine_kernels.cuh", "small_step.cuh", "net_step.cuh", "batch_kernels.cuh", "batch.h", "engine.cuh", "engine.h", "host_stage.h", "learned.h",
            "tc_mlp.cuh", "learned_dev.cuh", "plis_model.h", "plis_stream.h"]
 
 

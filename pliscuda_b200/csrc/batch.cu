@@ -32,14 +32,31 @@ __global__ void k_batch_prepare(BatchArgs B, double t_end, unsigned long long n_
   B.ctrl[r] = k;
 }
 
-__global__ void k_batch_fill(double* tau0, double* tau1, uint8_t* f0, uint8_t* f1, uint32_t n) {
+// A replica's new state but for its counts (k_reset for one replica: its rows start at coff in buffers of
+// `pitch` subvolumes per species).
+struct ReplicaReset {
+  int32_t* X[3];
+  int32_t* D;
+  double* tau[2];
+  uint8_t* flag[2];
+  Ctrl* ctrl;
+  uint32_t N, Npad, S, pitch;
+};
+__global__ void __launch_bounds__(256) k_batch_reset(const __grid_constant__ ReplicaReset A, const __grid_constant__ Ctrl k) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    tau0[i] = PLIS_INF_D;
-    tau1[i] = PLIS_INF_D;
-    f0[i] = F_SSA_FF;
-    f1[i] = F_SSA_FF;
+  if (i == 0) *A.ctrl = k;
+  if (i >= A.Npad) return;
+  for (uint32_t s = 0; s < A.S; ++s) {
+    const size_t j = (size_t)s * A.pitch + i;
+    A.X[1][j] = 0;
+    A.X[2][j] = 0;
+    A.D[j] = 0;
+    if (i >= A.N) A.X[0][j] = 0;
   }
+  A.tau[0][i] = PLIS_INF_D;
+  A.tau[1][i] = PLIS_INF_D;
+  A.flag[0][i] = F_SSA_FF;
+  A.flag[1][i] = F_SSA_FF;
 }
 
 #define PLIS_CU(call)                                                               \
@@ -55,6 +72,7 @@ BatchEngine::BatchEngine() {}
 BatchEngine::~BatchEngine() { release(); }
 
 void BatchEngine::release() {
+  stage_.release();
   for (void* p : allocs_) cudaFree(p);
   allocs_.clear();
   if (ev0_) cudaEventDestroy(ev0_);
@@ -252,6 +270,11 @@ int BatchEngine::create(const plis_batch_desc& d, const plis_options& opt) {
   PLIS_CU(cudaMemcpy(d_ctrl_, h_ctrl_.data(), nrep_ * sizeof(Ctrl), cudaMemcpyHostToDevice));
   pending_.assign(nrep_, 2);  // 2 = never given a state
   launch_ = (opt.precision == PLIS_PREC_FP32) ? batch_pick_f32(S_, false, small_) : batch_pick_f64(S_, false, small_);
+  {
+    uint32_t most = 0;
+    for (uint32_t r = 0; r < nrep_; ++r) most = std::max(most, npad_[r]);
+    PLIS_CU(stage_.init(opt.device, (size_t)most * 4));
+  }
   int tile[3] = {opt.tile[0], opt.tile[1], opt.tile[2]};
   if (tile[0] <= 0 || tile[1] <= 0 || tile[2] <= 0) { tile[0] = 8; tile[1] = 8; tile[2] = 4; }
   rc = layout(tile);
@@ -370,6 +393,7 @@ void batch_prepare(const BatchArgs& B, double t_end, unsigned long long n_steps,
 }
 
 int BatchEngine::launch(uint32_t max_iters) {
+  ctrl_fresh_ = false;
   BatchArgs B = make_args(dm_, dopt_, geo_, d_views_, d_rep_, nrep_, R_, S_, d_rr_, d_dr_, d_ctrl_, d_X_, d_tau_,
                           d_flag_, d_D_, d_work_, d_bar_, d_err_,
                           max_iters);
@@ -417,39 +441,44 @@ int BatchEngine::set_proposer(const float* weights, double s_max) {
     pending_[r] = 1;
     any_pending_ = true;
   }
+  PLIS_CU(cudaStreamSynchronize(stream_));  // a state set just before is still on its way
   PLIS_CU(cudaMemcpy(d_ctrl_, h_ctrl_.data(), nrep_ * sizeof(Ctrl), cudaMemcpyHostToDevice));
   return init_pending();
 }
 
 int BatchEngine::read_ctrls() {
+  if (ctrl_fresh_) return PLIS_OK;
   PLIS_CU(cudaMemcpyAsync(h_ctrl_.data(), d_ctrl_, nrep_ * sizeof(Ctrl), cudaMemcpyDeviceToHost, stream_));
   PLIS_CU(cudaStreamSynchronize(stream_));
+  ctrl_fresh_ = true;
   return PLIS_OK;
 }
 
 int BatchEngine::set_state(uint32_t r, const uint32_t* counts) {
   if (r >= nrep_) { err_ = "replica index out of range"; return PLIS_ERR_INVALID; }
   const uint32_t n = dims_[3 * r] * dims_[3 * r + 1] * dims_[3 * r + 2];
-  for (size_t i = 0; i < (size_t)S_ * n; ++i)
-    if (counts[i] >= (1u << 30)) { err_ = "counts must be below 2^30"; return PLIS_ERR_OVERFLOW; }
-  int rc = read_ctrls();
-  if (rc) return rc;
-  const size_t pitch = ntot_ * 4;
-  for (int i = 0; i < 3; ++i) PLIS_CU(cudaMemset2DAsync(d_X_[i] + coff_[r], pitch, 0, (size_t)npad_[r] * 4, S_, stream_));
-  PLIS_CU(cudaMemset2DAsync(d_D_ + coff_[r], pitch, 0, (size_t)npad_[r] * 4, S_, stream_));
-  PLIS_CU(cudaMemcpy2DAsync(d_X_[0] + coff_[r], pitch, counts, (size_t)n * 4, (size_t)n * 4, S_,
-                            cudaMemcpyHostToDevice, stream_));
-  k_batch_fill<<<(npad_[r] + 255) / 256, 256, 0, stream_>>>(d_tau_[0] + coff_[r], d_tau_[1] + coff_[r],
-                                                           d_flag_[0] + coff_[r], d_flag_[1] + coff_[r], npad_[r]);
-  Ctrl& k = h_ctrl_[r];
+  if (!counts_in_range(counts, (size_t)S_ * n)) { err_ = "counts must be below 2^30"; return PLIS_ERR_OVERFLOW; }
+  const size_t pitch = ntot_ * 4, row = (size_t)n * 4;
+  PLIS_CU(stage_.upload(d_X_[0] + coff_[r], pitch, counts, row, row, S_, stream_));
+  Ctrl k;
   std::memset(&k, 0, sizeof k);
   k.cur = 0; k.tgt = 1; k.spare = 2; k.tf = 0;
   k.phase = 0;
   k.done = 0;
   k.argmin = -1;
   k.last_argmin = -1;
-  PLIS_CU(cudaMemcpyAsync(d_ctrl_ + r, &k, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_));
-  PLIS_CU(cudaStreamSynchronize(stream_));
+  ReplicaReset a;
+  for (int i = 0; i < 3; ++i) a.X[i] = d_X_[i] + coff_[r];
+  for (int i = 0; i < 2; ++i) {
+    a.tau[i] = d_tau_[i] + coff_[r];
+    a.flag[i] = d_flag_[i] + coff_[r];
+  }
+  a.D = d_D_ + coff_[r];
+  a.ctrl = d_ctrl_ + r;
+  a.N = n; a.Npad = npad_[r]; a.S = S_; a.pitch = (uint32_t)ntot_;
+  k_batch_reset<<<(npad_[r] + 255) / 256, 256, 0, stream_>>>(a, k);
+  PLIS_CU(cudaGetLastError());
+  h_ctrl_[r] = k;
   pending_[r] = 1;
   any_pending_ = true;
   return PLIS_OK;
@@ -477,6 +506,7 @@ int BatchEngine::run(double t_end, uint64_t n_steps) {
   if (rc) return rc;
   BatchArgs B = make_args(dm_, dopt_, geo_, d_views_, d_rep_, nrep_, R_, S_, d_rr_, d_dr_, d_ctrl_, d_X_, d_tau_,
                           d_flag_, d_D_, d_work_, d_bar_, d_err_, 0);
+  ctrl_fresh_ = false;
   PLIS_CU(cudaEventRecord(ev0_, stream_));
   batch_prepare(B, t_end, (unsigned long long)n_steps, stream_);
   launches_ += 1;
@@ -513,9 +543,7 @@ int BatchEngine::get_state(uint32_t r, uint32_t* counts) {
   rc = read_ctrls();
   if (rc) return rc;
   const uint32_t n = dims_[3 * r] * dims_[3 * r + 1] * dims_[3 * r + 2];
-  PLIS_CU(cudaMemcpy2DAsync(counts, (size_t)n * 4, d_X_[h_ctrl_[r].cur] + coff_[r], ntot_ * 4, (size_t)n * 4, S_,
-                            cudaMemcpyDeviceToHost, stream_));
-  PLIS_CU(cudaStreamSynchronize(stream_));
+  PLIS_CU(stage_.download(counts, (size_t)n * 4, d_X_[h_ctrl_[r].cur] + coff_[r], ntot_ * 4, (size_t)n * 4, S_, stream_));
   return PLIS_OK;
 }
 
@@ -586,6 +614,7 @@ int BatchEngine::autotune(uint64_t pilot_steps, plis_batch_tuning* out) {
                           nrep_ * sizeof(Ctrl)};
   for (int i = 0; i < 9 && rc == PLIS_OK; ++i) rc = save(srcs[i], sizes[i]);
   auto restore = [&]() {
+    ctrl_fresh_ = false;
     for (int i = 0; i < 9; ++i) cudaMemcpy((void*)srcs[i], saved[i], sizes[i], cudaMemcpyDeviceToDevice);
   };
   const int cands[][3] = {{8, 8, 4}, {16, 4, 4}, {8, 4, 8}, {16, 8, 2}, {32, 4, 2}, {32, 8, 1}, {8, 8, 2}, {4, 8, 8}};

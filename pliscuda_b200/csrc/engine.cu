@@ -29,6 +29,11 @@ namespace plis {
     }                                                                                    \
   } while (0)
 
+// States of at least this many bytes go through HostStage: below it its pinned slices (2 ms to
+// allocate) and threads cost more than they save (a state of 1 MB uploads in 0.1 ms either way, one of
+// 84 MB in 19.7 ms through the driver and 5.2 ms through the stage, and back in 17.4 against 6.4).
+constexpr size_t kStagedState = size_t(8) << 20;
+
 static uint32_t pow2_at_least(uint32_t v) {
   uint32_t p = 1;
   while (p < v) p <<= 1;
@@ -46,6 +51,7 @@ void Engine::release() {
   if (d_evhead_) cudaFree(d_evhead_);
   d_evrec_ = nullptr;
   d_evhead_ = nullptr;
+  stage_.release();
   for (void* p : allocs_) cudaFree(p);
   allocs_.clear();
   if (h_ctrl_) cudaFreeHost(h_ctrl_);
@@ -314,6 +320,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
 
   // buffers
   const size_t cells = (size_t)M.S * dm.Npad;
+  if (cells * 4 >= kStagedState) PLIS_CU(stage_.init(opt.device, cells * 4));
   DevBufs& b = args_.b;
   for (int i = 0; i < 3; ++i)
     if ((rc = dmalloc((void**)&b.X[i], cells * 4))) return rc;
@@ -428,27 +435,25 @@ int Engine::build_graph() {
 }
 
 int Engine::read_ctrl() {
+  if (ctrl_fresh_) return PLIS_OK;
   PLIS_CU(cudaMemcpyAsync(h_ctrl_, args_.b.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, stream_));
   PLIS_CU(cudaStreamSynchronize(stream_));
+  ctrl_fresh_ = true;
   return PLIS_OK;
 }
 
 int Engine::set_state(const uint32_t* counts, double t0, uint64_t step0) {
   const DevModel& dm = args_.m;
-  for (size_t i = 0; i < (size_t)dm.S * dm.N; ++i)
-    if (counts[i] >= (1u << 30)) {
-      err_ = "counts must be below 2^30";
-      return PLIS_ERR_OVERFLOW;
-    }
-  const size_t cells = (size_t)dm.S * dm.Npad;
-  PLIS_CU(cudaMemsetAsync(args_.b.X[0], 0, cells * 4, stream_));
-  PLIS_CU(cudaMemcpy2DAsync(args_.b.X[0], (size_t)dm.Npad * 4, counts, (size_t)dm.N * 4, (size_t)dm.N * 4, dm.S,
-                            cudaMemcpyHostToDevice, stream_));
-  PLIS_CU(cudaMemsetAsync(args_.b.X[1], 0, cells * 4, stream_));
-  PLIS_CU(cudaMemsetAsync(args_.b.X[2], 0, cells * 4, stream_));
-  PLIS_CU(cudaMemsetAsync(args_.b.D, 0, cells * 4, stream_));
-  k_fill_tau<<<(dm.Npad + 255) / 256, 256, 0, stream_>>>(args_.b.tau[0], args_.b.flag[0], dm.Npad);
-  k_fill_tau<<<(dm.Npad + 255) / 256, 256, 0, stream_>>>(args_.b.tau[1], args_.b.flag[1], dm.Npad);
+  if (!counts_in_range(counts, (size_t)dm.S * dm.N)) {
+    err_ = "counts must be below 2^30";
+    return PLIS_ERR_OVERFLOW;
+  }
+  ctrl_fresh_ = false;
+  const size_t row = (size_t)dm.N * 4, pitch = (size_t)dm.Npad * 4;
+  if (stage_.on() && !host_pinned(counts))
+    PLIS_CU(stage_.upload(args_.b.X[0], pitch, counts, row, row, dm.S, stream_));
+  else
+    PLIS_CU(cudaMemcpy2DAsync(args_.b.X[0], pitch, counts, row, row, dm.S, cudaMemcpyHostToDevice, stream_));
   Ctrl k;
   std::memset(&k, 0, sizeof k);
   k.cur = 0; k.tgt = 1; k.spare = 2; k.tf = 0;
@@ -460,10 +465,10 @@ int Engine::set_state(const uint32_t* counts, double t0, uint64_t step0) {
   k.t_end = 0.0;
   k.t = t0;
   k.step = step0;
-  *h_ctrl_ = k;
-  PLIS_CU(cudaMemcpyAsync(args_.b.ctrl, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_));
+  const uint32_t rb = (dm.Npad + 255u) / 256u;
+  k_reset<<<rb < 2048u ? rb : 2048u, 256, 0, stream_>>>(args_, k);
   launch_classify();
-  launches_ += 3;
+  launches_ += 2;
   PLIS_CU(cudaGetLastError());
   int rc = read_ctrl();
   if (rc) return rc;
@@ -482,6 +487,7 @@ int Engine::reclassify() {
   h_ctrl_->phase = 0;
   h_ctrl_->dt = 0.0;
   h_ctrl_->done = 0;
+  ctrl_fresh_ = false;
   PLIS_CU(cudaMemcpyAsync(args_.b.ctrl, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_));
   launch_classify();
   launches_ += 1;
@@ -567,8 +573,12 @@ int Engine::get_state(uint32_t* counts) {
   int rc = read_ctrl();
   if (rc) return rc;
   const DevModel& dm = args_.m;
-  PLIS_CU(cudaMemcpy2DAsync(counts, (size_t)dm.N * 4, args_.b.X[h_ctrl_->cur], (size_t)dm.Npad * 4, (size_t)dm.N * 4,
-                            dm.S, cudaMemcpyDeviceToHost, stream_));
+  const size_t row = (size_t)dm.N * 4, pitch = (size_t)dm.Npad * 4;
+  if (stage_.on() && !host_pinned(counts)) {
+    PLIS_CU(stage_.download(counts, row, args_.b.X[h_ctrl_->cur], pitch, row, dm.S, stream_));
+    return PLIS_OK;
+  }
+  PLIS_CU(cudaMemcpy2DAsync(counts, row, args_.b.X[h_ctrl_->cur], pitch, row, dm.S, cudaMemcpyDeviceToHost, stream_));
   PLIS_CU(cudaStreamSynchronize(stream_));
   return PLIS_OK;
 }
@@ -636,6 +646,7 @@ int Engine::advance(double t_end, uint64_t n_steps) {
     int rc = build_graph();
     if (rc) return rc;
   }
+  ctrl_fresh_ = false;
   PLIS_CU(cudaEventRecord(ev0_, stream_));
   k_prepare<<<1, 32, 0, stream_>>>(args_, t_end, (unsigned long long)n_steps);
   launches_ += 1;
@@ -646,6 +657,7 @@ int Engine::advance(double t_end, uint64_t n_steps) {
       if (rc) return rc;
       launches_ += kernels_per_step_;
       PLIS_CU(cudaGetLastError());
+      ctrl_fresh_ = false;
       rc = read_ctrl();
       if (rc) return rc;
       if (h_ctrl_->done) break;
@@ -668,6 +680,7 @@ int Engine::advance(double t_end, uint64_t n_steps) {
       launches_ += (uint64_t)graph_steps_ * kernels_per_step_;
     }
     PLIS_CU(cudaGetLastError());
+    ctrl_fresh_ = false;
     int rc = read_ctrl();
     if (rc) return rc;
     if (h_ctrl_->done) break;
@@ -762,6 +775,7 @@ int Engine::slab_phase(int phase, double t_end, uint64_t n_steps) {
   const dim3 gx(exact_blocks_), bx(256);
   const uint32_t lb = (args_.sl.layer + 255u) / 256u;
   const dim3 gl(lb < 1024u ? lb : 1024u), bl(256);
+  ctrl_fresh_ = false;
   PLIS_CU(cudaEventRecord(ev0_, stream_));
   switch (phase) {
     case PLIS_SLAB_CLASSIFY:

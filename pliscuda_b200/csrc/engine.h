@@ -10,6 +10,7 @@
 
 #include "../../include/plis.h"
 #include "engine.cuh"
+#include "host_stage.h"
 #include "learned.h"
 #include "plis_model.h"
 
@@ -77,6 +78,8 @@ class Engine {
   cudaGraphExec_t graph_exec_ = nullptr;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   Ctrl* h_ctrl_ = nullptr;
+  bool ctrl_fresh_ = false;  // h_ctrl_ holds the device's control block (nothing has run since it was read)
+  HostStage stage_;          // transfers of large states
   std::vector<void*> allocs_;
   std::string err_;
   int graph_steps_ = 32;

@@ -2173,9 +2173,27 @@ __global__ void k_slab_unpack_flags(KArgs A) {
 #endif
 
 #ifdef PLIS_ENGINE_HOST_TU
-__global__ void k_fill_tau(double* t, uint8_t* f, uint32_t n) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) { t[i] = PLIS_INF_D; f[i] = F_SSA_FF; }
+// A new state's buffers but for its counts: targets, deltas and the padding of the counts zero, taus
+// infinite, every subvolume SSA_FF, and the control block.
+__global__ void __launch_bounds__(256) k_reset(const __grid_constant__ KArgs A, const __grid_constant__ Ctrl k) {
+  const DevModel& m = A.m;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  const size_t words = (size_t)m.S * m.Npad / 4;  // Npad is a multiple of 32
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (size_t i = tid; i < words; i += nth) {
+    reinterpret_cast<uint4*>(A.b.X[1])[i] = zero;
+    reinterpret_cast<uint4*>(A.b.X[2])[i] = zero;
+    reinterpret_cast<uint4*>(A.b.D)[i] = zero;
+  }
+  for (uint32_t i = tid; i < m.Npad; i += nth) {
+    A.b.tau[0][i] = PLIS_INF_D;
+    A.b.tau[1][i] = PLIS_INF_D;
+    A.b.flag[0][i] = F_SSA_FF;
+    A.b.flag[1][i] = F_SSA_FF;
+    if (i >= m.N)
+      for (uint32_t s = 0; s < m.S; ++s) A.b.X[0][(size_t)s * m.Npad + i] = 0;
+  }
+  if (tid == 0) *A.b.ctrl = k;
 }
 #endif
 
