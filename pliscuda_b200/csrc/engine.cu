@@ -29,10 +29,12 @@ namespace plis {
     }                                                                                    \
   } while (0)
 
-// States of at least this many bytes go through HostStage: below it its pinned slices (2 ms to
-// allocate) and threads cost more than they save (a state of 1 MB uploads in 0.1 ms either way, one of
-// 84 MB in 19.7 ms through the driver and 5.2 ms through the stage, and back in 17.4 against 6.4).
-constexpr size_t kStagedState = size_t(8) << 20;
+// States of at least this many bytes go through HostStage: one of 84 MB uploads in 19.7 ms through the
+// driver and 5.2 ms through the stage, and comes back in 17.4 against 6.4; one of 10 MB gains 0.9 ms a
+// round trip, for which its pinned slices (4-8 ms to allocate) are not worth having.
+constexpr size_t kStagedState = size_t(32) << 20;
+
+constexpr uint64_t kStepsMin = 6;
 
 static uint32_t pow2_at_least(uint32_t v) {
   uint32_t p = 1;
@@ -365,6 +367,22 @@ int Engine::create(const Model& model, const plis_options& opt) {
       if (bytes > 48u * 1024u) PLIS_CU(launch_.leap_smem((int)bytes));
     }
   }
+  // systems whose bricks are all resident at once advance in k_steps (a caller's own wait limit keeps
+  // the phase kernels, which do not wait)
+  if ((args_.sm.on || o.net) && !opt.profile && opt.wait_polls == 0) {
+    const StepsKernel k = launch_.steps(args_);
+    int nsm = 0, per = 0, coop = 0;
+    PLIS_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, opt.device));
+    PLIS_CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, opt.device));
+    if (k.kernel && coop && g.nblocks <= (uint32_t)(kStepsCtas * nsm)) {
+      PLIS_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k.kernel, (int)g.threads, k.smem));
+      if (g.nblocks <= (uint32_t)(per * nsm)) {
+        steps_ = k;
+        if ((rc = dmalloc((void**)&d_bar_, sizeof(unsigned)))) return rc;
+        if ((rc = dmalloc((void**)&d_steps_slot_, (size_t)g.nblocks * sizeof(StepsSlot)))) return rc;
+      }
+    }
+  }
   kernels_per_step_ = (opt.mode == PLIS_MODE_REFERENCE) ? 4 : 3;
   graph_steps_ = opt.steps_per_launch > 0 ? opt.steps_per_launch : 32;
   PLIS_CU(cudaDeviceSynchronize());
@@ -639,16 +657,40 @@ int Engine::read_event_log(plis_event_record* out, uint64_t max_records, uint64_
   return PLIS_OK;
 }
 
+// The prepared run in k_steps launches (a launch ends after a few thousand attempts at the latest, so
+// that it does not hold the GPU for long).
+int Engine::advance_steps() {
+  NetArgs a = args_;
+  a.o.no_list = 1;
+  StepsRun run{d_bar_, (StepsSlot*)d_steps_slot_, 1ull << 26, 4096u};
+  void* args[] = {&a, &run};
+  for (bool first = true;; first = false) {
+    if (!first) PLIS_CU(cudaMemsetAsync(d_bar_, 0, sizeof(unsigned), stream_));
+    PLIS_CU(cudaLaunchCooperativeKernel(steps_.kernel, dim3(args_.g.nblocks), dim3(args_.g.threads), args, steps_.smem, stream_));
+    launches_ += 1;
+    ctrl_fresh_ = false;
+    int rc = read_ctrl();
+    if (rc) return rc;
+    if (h_ctrl_->status == PLIS_ERR_TIMEOUT) {  // the step was left half done: only a new state helps
+      err_ = "a grid barrier of the persistent kernel timed out";
+      return PLIS_ERR_TIMEOUT;
+    }
+    if (h_ctrl_->done) return PLIS_OK;
+  }
+}
+
 int Engine::advance(double t_end, uint64_t n_steps) {
   if (slab_blocks_) { err_ = "a z-slab advances through plis_slab_phase"; return PLIS_ERR_UNSUPPORTED; }
+  // a cooperative launch starts later than the phase kernels of a few steps finish
+  const bool resident = steps_.kernel && !use_learned_ && !args_.b.ev.rec && n_steps >= kStepsMin;
   const bool few = n_steps != ~0ull && n_steps < (uint64_t)graph_steps_;
-  if (!few && !opt_.profile) {  // the one-off capture and instantiation stay out of the timed interval
+  if (!few && !opt_.profile && !resident) {  // the one-off capture and instantiation stay out of the timed interval
     int rc = build_graph();
     if (rc) return rc;
   }
   ctrl_fresh_ = false;
   PLIS_CU(cudaEventRecord(ev0_, stream_));
-  k_prepare<<<1, 32, 0, stream_>>>(args_, t_end, (unsigned long long)n_steps);
+  k_prepare<<<1, 32, 0, stream_>>>(args_, t_end, (unsigned long long)n_steps, resident ? d_bar_ : nullptr);
   launches_ += 1;
   PLIS_CU(cudaGetLastError());
   if (opt_.profile) {  // one step at a time, events around every kernel
@@ -671,7 +713,11 @@ int Engine::advance(double t_end, uint64_t n_steps) {
     return PLIS_OK;
   }
   uint64_t budget = few ? n_steps : 0;
-  while (true) {
+  if (resident) {
+    int rc = advance_steps();
+    if (rc) return rc;
+  }
+  while (!resident) {
     if (few) {
       for (uint64_t i = 0; i < budget; ++i) enqueue_step();
       launches_ += budget * kernels_per_step_;
@@ -792,7 +838,7 @@ int Engine::slab_phase(int phase, double t_end, uint64_t n_steps) {
       launches_ += 1;
       break;
     case PLIS_SLAB_PREPARE:
-      k_prepare<<<1, 32, 0, stream_>>>(args_, t_end, (unsigned long long)n_steps);
+      k_prepare<<<1, 32, 0, stream_>>>(args_, t_end, (unsigned long long)n_steps, nullptr);
       launches_ += 1;
       break;
     case PLIS_SLAB_LEAP:

@@ -16,6 +16,12 @@
 
 namespace plis {
 
+// The persistent step kernel of a handle (k_steps) and its dynamic shared memory.
+struct StepsKernel {
+  const void* kernel;
+  size_t smem;
+};
+
 // Kernel launchers of one (precision, species-capacity) instantiation.
 struct Launchers {
   void (*leap)(const KArgs&, dim3, dim3, cudaStream_t);
@@ -23,6 +29,7 @@ struct Launchers {
   void (*classify)(const KArgs&, dim3, dim3, cudaStream_t);
   cudaError_t (*leap_smem)(int bytes);
   cudaError_t (*net_smem)();  // shared memory above the default limit for the network kernels
+  StepsKernel (*steps)(const KArgs&);
 };
 
 // SmallModel tables of a model (engine.cu); false, with sm->on = 0, when it does not fit.
@@ -67,6 +74,7 @@ class Engine {
   void enqueue_step();
   void launch_classify();
   int build_graph();
+  int advance_steps();
   int read_ctrl();
   int reclassify();
 
@@ -84,6 +92,9 @@ class Engine {
   std::string err_;
   int graph_steps_ = 32;
   uint32_t exact_blocks_ = 1;  // CTAs of k_exact / k_apply
+  StepsKernel steps_{nullptr, 0};  // set when the system is small enough for k_steps
+  unsigned* d_bar_ = nullptr;
+  void* d_steps_slot_ = nullptr;
   int kernels_per_step_ = 4;
   uint64_t launches_ = 0;
   double device_ms_ = 0.0;

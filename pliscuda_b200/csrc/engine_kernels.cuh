@@ -796,9 +796,11 @@ __device__ __forceinline__ void prepare_step(Ctrl& k, int mode) {
 }
 
 #ifdef PLIS_ENGINE_HOST_TU
-__global__ void k_prepare(KArgs A, double t_end, unsigned long long n_steps) {
+// bar: the barrier word of the k_steps launch that follows (null: phase kernels follow)
+__global__ void k_prepare(KArgs A, double t_end, unsigned long long n_steps, unsigned* bar) {
   Ctrl* K = A.b.ctrl;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  if (bar) *bar = 0u;
   Ctrl k = *K;
   if (k.status != PLIS_OK) {
     k.done = 1;
@@ -1259,7 +1261,7 @@ __device__ __forceinline__ uint32_t* touched_list(const KArgs& A) {
 }
 __device__ __forceinline__ void touch(const KArgs& A, uint32_t c) {
   Ctrl* K = A.b.ctrl;
-  if (!K->touched_on) return;
+  if (A.o.no_list || !K->touched_on) return;
   namespace cg = cooperative_groups;  // one atomic for the threads that get here together
   const cg::coalesced_group g = cg::coalesced_threads();
   uint32_t i = 0;
@@ -1720,24 +1722,13 @@ __device__ __forceinline__ void classify_tile(const KArgs& A, uint32_t tile, con
   ti = c;
 }
 
-// The same for a small model (small_step.cuh).
+// The same for a small model (small_step.cuh): one subvolume with its counts x, and its tau and flag.
 template <typename Real, int MAXS, bool LAT>
-__device__ __forceinline__ void classify_tile_small(const KArgs& A, const SmallModel& t, uint32_t tile, const ClassifyCtx& C,
-                                                    double& tn, uint32_t& ti, int& fl, int& bad, bool& valid) {
+__device__ __forceinline__ void classify_cell_small(const KArgs& A, const SmallModel& t, const Cell& cl, const int32_t x[MAXS],
+                                                    const ClassifyCtx& C, double tau_cur, uint8_t flag_cur, double& tn, int& fl,
+                                                    int& bad) {
   const DevModel& m = A.m;
-  Cell cl;
-  valid = cell_of(A, tile, cl);
   const uint32_t c = cl.c;
-  tn = PLIS_INF_D;
-  ti = kNoCell;
-  fl = F_SSA_FF;
-  bad = 0;
-  if (!valid) return;
-  const double tau_cur = C.tau_cur[c];
-  const uint8_t flag_cur = C.flag_cur[c];
-  int32_t x[MAXS];
-#pragma unroll
-  for (int s = 0; s < MAXS; ++s) x[s] = s < (int)m.S ? C.Xe[(size_t)s * m.Npad + c] : 0;
 #pragma unroll
   for (int s = 0; s < MAXS; ++s)
     if (s < (int)m.S) {
@@ -1751,26 +1742,34 @@ __device__ __forceinline__ void classify_tile_small(const KArgs& A, const SmallM
   }
   C.tau_new[c] = tn;
   C.flag_new[c] = (uint8_t)fl;
-  ti = c;
 }
-
-// The same for a network with NetTab (net_step.cuh); smem: the CTA's count and propensity columns.
-template <typename Real, bool LAT, bool COMP>
-__device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const ClassifyCtx& C,
-                                                  unsigned char* smem, double& tn, uint32_t& ti, int& fl, int& bad,
-                                                  bool& valid) {
-  const DevModel& m = A.m;
-  const int S = (int)m.S;
+template <typename Real, int MAXS, bool LAT>
+__device__ __forceinline__ void classify_tile_small(const KArgs& A, const SmallModel& t, uint32_t tile, const ClassifyCtx& C,
+                                                    double& tn, uint32_t& ti, int& fl, int& bad, bool& valid) {
   Cell cl;
   valid = cell_of(A, tile, cl);
-  const uint32_t c = cl.c;
   tn = PLIS_INF_D;
   ti = kNoCell;
   fl = F_SSA_FF;
   bad = 0;
   if (!valid) return;
-  const double tau_cur = C.tau_cur[c];
-  const uint8_t flag_cur = C.flag_cur[c];
+  const double tau_cur = C.tau_cur[cl.c];
+  const uint8_t flag_cur = C.flag_cur[cl.c];
+  int32_t x[MAXS];
+#pragma unroll
+  for (int s = 0; s < MAXS; ++s) x[s] = s < (int)A.m.S ? C.Xe[(size_t)s * A.m.Npad + cl.c] : 0;
+  classify_cell_small<Real, MAXS, LAT>(A, t, cl, x, C, tau_cur, flag_cur, tn, fl, bad);
+  ti = cl.c;
+}
+
+// The same for a network with NetTab (net_step.cuh); smem: the CTA's count and propensity rows.
+template <typename Real, bool LAT, bool COMP>
+__device__ __forceinline__ void classify_cell_net(const KArgs& A, const NetTab<Real>& T, const Cell& cl, const ClassifyCtx& C,
+                                                  double tau_cur, uint8_t flag_cur, unsigned char* smem, double& tn, int& fl,
+                                                  int& bad) {
+  const DevModel& m = A.m;
+  const int S = (int)m.S;
+  const uint32_t c = cl.c;
   const Column<Real> sx = column<Real>(smem, 0);
 #pragma unroll 4
   for (int s = 0; s < S; ++s) {
@@ -1786,7 +1785,20 @@ __device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<R
   }
   C.tau_new[c] = tn;
   C.flag_new[c] = (uint8_t)fl;
-  ti = c;
+}
+template <typename Real, bool LAT, bool COMP>
+__device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const ClassifyCtx& C,
+                                                  unsigned char* smem, double& tn, uint32_t& ti, int& fl, int& bad,
+                                                  bool& valid) {
+  Cell cl;
+  valid = cell_of(A, tile, cl);
+  tn = PLIS_INF_D;
+  ti = kNoCell;
+  fl = F_SSA_FF;
+  bad = 0;
+  if (!valid) return;
+  classify_cell_net<Real, LAT, COMP>(A, T, cl, C, C.tau_cur[cl.c], C.flag_cur[cl.c], smem, tn, fl, bad);
+  ti = cl.c;
 }
 
 // CTA reduction into slot `slot` of its threads' min tau with arg-min (key, ti), with PLAIN the min of
@@ -1852,14 +1864,10 @@ __device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t 
 // no subvolume can fire), #LEAP_CR gcr, #SSA_FF gff, a negative count or oversized draw `bad`, the min of
 // the plain taus gp (learned proposals) and the flag of the arg-min subvolume: rollback or accept, time,
 // the next plan.  One thread.
-__device__ __forceinline__ void step_decide(const KArgs& A, Ctrl* K, uint32_t phase, uint32_t tf, double gt, long long gi,
+__device__ __forceinline__ void step_decide(const KArgs& A, Ctrl& k, uint32_t phase, uint32_t tf, double gt, long long gi,
                                             unsigned long long gcr, unsigned long long gff, uint32_t bad, double gp,
                                             bool learned, uint32_t am_flag) {
   const int mode = A.o.mode;
-  Ctrl k = *K;
-  k.blocks_done = 0;  // these three may have changed since this SM first read the block
-  k.n_touched = 0;
-  k.status = __ldcg(&K->status);
   k.learned = learned ? 1u : 0u;
   if (phase == 0) {
     k.tau_min = gt;
@@ -1905,6 +1913,16 @@ __device__ __forceinline__ void step_decide(const KArgs& A, Ctrl* K, uint32_t ph
     k.argmin_flag = am_flag;
     prepare_step(k, mode);
   }
+}
+// the same on the control block itself
+__device__ __forceinline__ void step_decide(const KArgs& A, Ctrl* K, uint32_t phase, uint32_t tf, double gt, long long gi,
+                                            unsigned long long gcr, unsigned long long gff, uint32_t bad, double gp,
+                                            bool learned, uint32_t am_flag) {
+  Ctrl k = *K;
+  k.blocks_done = 0;  // these three may have changed since this SM first read the block
+  k.n_touched = 0;
+  k.status = __ldcg(&K->status);
+  step_decide(A, k, phase, tf, gt, gi, gcr, gff, bad, gp, learned, am_flag);
   *K = k;
 }
 
@@ -2023,6 +2041,289 @@ __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify(KArg
   classify_tile<Real, MAXS, true, CACHE>(A, blockIdx.x, C, tn, ti, fl, bad, valid, reinterpret_cast<Real*>(s_prop));
   if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
     classify_control(A, K, gridDim.x);
+}
+
+// ------------------------------------------------------------------------------------------------
+// k_steps: many steps of a small system in one cooperative launch
+// ------------------------------------------------------------------------------------------------
+// On a few thousand subvolumes a step of phase kernels is all latency: four launches, each of which reads
+// the control block before it can load anything, two kernels that usually find nothing to do, a ticket and
+// a last CTA that decides for all (15-19 us a step however small the system).  Here one CTA per brick
+// stays for all steps.  The phases are separated by grid barriers; after the classification's every CTA
+// reads all bricks' records and takes the step's decision itself, in its own copy of the control block
+// (the same inputs, so the same decision), and keeps its subvolumes' counts, flags and propensities for
+// the next leap.  A cooperative launch, so all CTAs are resident; every wait has a limit, after which the
+// CTA leaves with an error status.  Used up to kStepsCtas CTAs per SM (Engine::create); larger systems
+// fill the GPU with the phase kernels' higher occupancy.
+struct alignas(16) StepsSlot {   // what one CTA found: three 16-byte words
+  double tau;
+  uint32_t idx;                  // kNoCell: no subvolume
+  uint32_t bits;                 // flag of idx | 256: a negative count or a draw beyond the int32 guards
+  uint32_t ncr, nff;             // #LEAP_CR, #SSA_FF
+  unsigned long long ev;         // events of the attempt
+  unsigned long long ex;         // exact events among them
+  unsigned long long pad_;
+};
+static_assert(sizeof(StepsSlot) == 48, "StepsSlot is read as three uint4");
+struct StepsRun {
+  unsigned* bar;                 // arrivals; zeroed before the launch
+  StepsSlot* slot;               // [CTAs]
+  unsigned long long limit;      // polls of a wait before it gives up
+  uint32_t max_iters;            // attempts per launch
+};
+constexpr int kStepsCtas = 2;    // CTAs per SM: up to 128 registers a thread, no spills
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// Grid barrier; false (and an error status) when the limit ran out.
+__device__ __forceinline__ bool steps_sync(const StepsRun& R, Ctrl* K, unsigned& target) {
+  __shared__ int s_go;
+  target += gridDim.x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(R.bar, 1u);
+    int go = 1;
+    unsigned long long polls = 0;
+    while ((int)(ld_acquire(R.bar) - target) < 0) {
+      if (++polls > R.limit) {
+        atomicExch(&K->status, PLIS_ERR_TIMEOUT);
+        go = 0;
+        break;
+      }
+    }
+    __threadfence();
+    s_go = go;
+  }
+  __syncthreads();
+  return s_go != 0;
+}
+
+// the phases of a small model and of a network: one subvolume per thread, its state kept from one
+// classification to the next leap
+template <typename Real_, int MAXS_, bool LAT> struct SmallPhases {
+  using Real = Real_;
+  using Args = KArgs;
+  static constexpr int MAXS = MAXS_;
+  static constexpr bool kKeep = false;  // accept() only after accepted attempts
+  int32_t x[MAXS];  // counts of the current state
+  int32_t xe[MAXS]; // counts of the state classified last
+  __device__ __forceinline__ void start(const Args& A, uint32_t c, const int32_t* Xc, unsigned char*) {
+#pragma unroll
+    for (int s = 0; s < MAXS; ++s) x[s] = s < (int)A.m.S ? Xc[(size_t)s * A.m.Npad + c] : 0;
+  }
+  __device__ __forceinline__ void accept(bool) {
+#pragma unroll
+    for (int s = 0; s < MAXS; ++s) x[s] = xe[s];
+  }
+  __device__ __forceinline__ void leap(const Args& A, const Cell& cl, uint8_t f, const LeapCtx& L, Real tl, unsigned char*,
+                                       long long& ev, int& big) {
+    leap_cell_small<Real, MAXS, false, LAT, true>(A, A.sm, cl, x, f, L, tl, ev, big);
+  }
+  __device__ __forceinline__ int critical(const Args& A, uint32_t c, const LeapCtx& L, unsigned char*) {
+    Counts<MAXS> y;
+#pragma unroll
+    for (int s = 0; s < MAXS; ++s) y.v[s] = x[s];
+    return critical_event_ref<Real, false>(A, c, y, L.Xt, L.step, L.attempt, A.b.D, L.flag);
+  }
+  __device__ __forceinline__ void classify(const Args& A, const Cell& cl, const ClassifyCtx& C, double tau_cur, uint8_t flag_cur,
+                                           unsigned char*, double& tn, int& fl, int& bad) {
+#pragma unroll
+    for (int s = 0; s < MAXS; ++s) xe[s] = s < (int)A.m.S ? C.Xe[(size_t)s * A.m.Npad + cl.c] : 0;
+    classify_cell_small<Real, MAXS, LAT>(A, A.sm, cl, xe, C, tau_cur, flag_cur, tn, fl, bad);
+  }
+};
+template <typename Real_, bool LAT, bool COMP> struct NetPhases {
+  using Real = Real_;
+  using Args = NetArgs;
+  static constexpr int MAXS = kNetS;
+  static constexpr bool kKeep = true;
+  bool fresh;
+  __device__ __forceinline__ void start(const Args&, uint32_t, const int32_t*, unsigned char*) { fresh = false; }
+  // a fast-forwarded subvolume has no propensities in its rows, but it does not leap either
+  __device__ __forceinline__ void accept(bool accepted) { fresh = accepted; }
+  __device__ __forceinline__ void leap(const Args& A, const Cell& cl, uint8_t f, const LeapCtx& L, Real tl, unsigned char* sm,
+                                       long long& ev, int& big) {
+    leap_cell_net<Real, false, LAT, COMP>(A, net_tab<Real>(A), cl, f, fresh, L, tl, sm, ev, big);
+  }
+  __device__ __forceinline__ int critical(const Args& A, uint32_t c, const LeapCtx& L, unsigned char* sm) {
+    return critical_event_net<Real, false, COMP>(A, net_tab<Real>(A), c, column<Real>(sm, 0),
+                                                 column<Real>(sm, sizeof(Real) * (size_t)A.m.S), L.Xc, L.Xt, L.step, L.attempt,
+                                                 A.b.D, L.flag);
+  }
+  __device__ __forceinline__ void classify(const Args& A, const Cell& cl, const ClassifyCtx& C, double tau_cur, uint8_t flag_cur,
+                                           unsigned char* sm, double& tn, int& fl, int& bad) {
+    classify_cell_net<Real, LAT, COMP>(A, net_tab<Real>(A), cl, C, tau_cur, flag_cur, sm, tn, fl, bad);
+  }
+};
+
+template <class P>
+__global__ void __launch_bounds__(256, kStepsCtas) k_steps(const __grid_constant__ typename P::Args A, const __grid_constant__ StepsRun R) {
+  using Real = typename P::Real;
+  extern __shared__ __align__(16) unsigned char s_net[];
+  __shared__ Ctrl s_k;           // this CTA's control block
+  __shared__ uint64_t s_key[8];
+  __shared__ uint32_t s_i[8], s_cr[8], s_ff[8], s_fl[8];
+  __shared__ unsigned long long s_ev, s_ex;
+  __shared__ uint32_t s_bad;
+  const DevModel& m = A.m;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  unsigned target = 0;
+  Cell cl;
+  const bool mine = cell_of(A, blockIdx.x, cl);
+  const uint32_t c = cl.c;
+  if (threadIdx.x == 0) {
+    s_k = *A.b.ctrl;
+    s_ev = s_ex = 0ull;
+    s_bad = 0u;
+  }
+  __syncthreads();
+  P p;
+  uint8_t flag = F_SSA_FF;       // of this thread's subvolume
+  double tau = PLIS_INF_D;
+  if (mine) {
+    flag = A.b.flag[s_k.tf][c];
+    tau = A.b.tau[s_k.tf][c];
+    p.start(A, c, A.b.X[s_k.cur], s_net);
+  }
+  for (uint32_t it = 0; it < R.max_iters && !s_k.done; ++it) {
+    const uint32_t ex = s_k.exact;
+    const long long am = s_k.argmin;
+    const LeapCtx L = leap_ctx(A, &s_k);
+    const ClassifyCtx C = classify_ctx(A, &s_k);
+    const Real tl = (Real)s_k.tau_leap;
+    long long ev = 0;
+    int big = 0;
+    if (mine) p.leap(A, cl, flag, L, tl, s_net, ev, big);
+    ev = warp_sum(ev);
+    if (lane == 0 && ev) atomicAdd(&s_ev, (unsigned long long)ev);
+    if (big) s_bad = 1u;
+    if (!steps_sync(R, A.b.ctrl, target)) return;
+    if (ex) {
+      int fired = 0;
+      if ((ex & 1u) && flag == F_LEAP_CR) fired += p.critical(A, c, L, s_net);
+      if ((ex & 2u) && blockIdx.x == 0 && threadIdx.x == 0) {
+        const uint8_t fa = L.flag[am];
+        if (fa == F_SSA || fa == F_SSA_FF || (A.o.mode != 0 && fa == F_LEAP_CR)) {
+          Counts<P::MAXS> y;
+          load_counts(m, L.Xc, (uint32_t)am, y);
+          fired += argmin_event<Real, false>(A, (uint32_t)am, y, L.step, L.attempt, (ex & 1u) ? A.b.D : L.Xt, L.flag,
+                                             fa == F_LEAP_CR);
+        }
+      }
+      fired = __reduce_add_sync(0xffffffffu, fired);
+      if (lane == 0 && fired) {
+        atomicAdd(&s_ev, (unsigned long long)fired);
+        atomicAdd(&s_ex, (unsigned long long)fired);
+      }
+      if (!steps_sync(R, A.b.ctrl, target)) return;
+      if (ex & 1u) {  // the staged deltas of this CTA's subvolumes
+        if (mine) {
+          for (uint32_t s = 0; s < m.S; ++s) {
+            const size_t j = (size_t)s * m.Npad + c;
+            const int32_t v = A.b.D[j];
+            if (v) {
+              L.Xt[j] += v;
+              A.b.D[j] = 0;
+            }
+          }
+        }
+        if (!steps_sync(R, A.b.ctrl, target)) return;
+      }
+    }
+    double tn = PLIS_INF_D;
+    int fl = F_SSA_FF, bad = 0;
+    if (mine) {
+      // another subvolume's jump may have ended this one's fast-forward since its classification
+      const uint8_t f = flag == F_SSA_FF ? L.flag[c] : flag;
+      p.classify(A, cl, C, tau, f, s_net, tn, fl, bad);
+    }
+    {  // the CTA's record
+      const uint64_t key = mine ? tau_key(tn) : ~0ull;
+      uint64_t k = key;
+      uint32_t i = mine ? c : kNoCell;
+      if (bad) s_bad = 1u;
+      const uint32_t ncr = (uint32_t)__popc(__ballot_sync(0xffffffffu, mine && fl == F_LEAP_CR));
+      const uint32_t nff = (uint32_t)__popc(__ballot_sync(0xffffffffu, mine && fl == F_SSA_FF));
+      warp_min_key(k, i);
+      if (mine ? i == c : (lane == 0 && i == kNoCell)) {  // one lane: the owner, or lane 0 of an empty warp
+        s_key[wid] = k;
+        s_i[wid] = i;
+        s_fl[wid] = (uint32_t)fl;
+        s_cr[wid] = ncr;
+        s_ff[wid] = nff;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        StepsSlot q;
+        int w = 0;
+        q.ncr = s_cr[0];
+        q.nff = s_ff[0];
+        for (int v = 1; v < nw; ++v) {
+          if (s_key[v] < s_key[w] || (s_key[v] == s_key[w] && s_i[v] < s_i[w])) w = v;
+          q.ncr += s_cr[v];
+          q.nff += s_ff[v];
+        }
+        q.tau = key_tau(s_key[w]);
+        q.idx = s_i[w];
+        q.bits = s_fl[w] | (s_bad ? 256u : 0u);
+        q.ev = s_ev;
+        q.ex = s_ex;
+        q.pad_ = 0;
+        R.slot[blockIdx.x] = q;
+        s_ev = s_ex = 0ull;
+        s_bad = 0u;
+      }
+    }
+    if (!steps_sync(R, A.b.ctrl, target)) return;
+    {  // every CTA: all records, the decision
+      uint64_t gk = tau_key(PLIS_INF_D);
+      uint32_t gi = kNoCell, gfl = F_SSA_FF, gcr = 0, gff = 0, gbad = 0;
+      unsigned long long gev = 0, gex = 0;
+      if (wid == 0) {
+        for (uint32_t b = lane; b < gridDim.x; b += 32) {
+          const uint4* q = reinterpret_cast<const uint4*>(R.slot + b);
+          const uint4 u = __ldcg(q), v = __ldcg(q + 1), w = __ldcg(q + 2);
+          const uint64_t k = tau_key(__hiloint2double((int)u.y, (int)u.x));
+          if (k < gk || (k == gk && u.z < gi)) { gk = k; gi = u.z; gfl = u.w & 255u; }
+          gbad |= u.w & 256u;
+          gcr += v.x;
+          gff += v.y;
+          gev += (unsigned long long)v.w << 32 | v.z;
+          gex += (unsigned long long)w.y << 32 | w.x;
+        }
+        const uint32_t my = gi;
+        warp_min_key(gk, gi);
+        const unsigned who = __ballot_sync(0xffffffffu, my == gi);
+        gfl = __shfl_sync(0xffffffffu, gfl, __ffs(who) - 1);
+        gcr = __reduce_add_sync(0xffffffffu, gcr);
+        gff = __reduce_add_sync(0xffffffffu, gff);
+        gbad = __reduce_or_sync(0xffffffffu, gbad);
+        gev = (unsigned long long)warp_sum((long long)gev);
+        gex = (unsigned long long)warp_sum((long long)gex);
+        if (lane == 0) {
+          s_k.ev_attempt = gev;
+          s_k.ex_attempt = gex;
+          step_decide(A, s_k, 1u, s_k.tf, key_tau(gk), gi == kNoCell ? -1ll : (long long)gi, gcr, gff, gbad, PLIS_INF_D, false,
+                      gi == kNoCell ? (uint32_t)F_SSA_FF : gfl);
+        }
+      }
+      __syncthreads();
+    }
+    const bool accepted = s_k.step == L.step;  // else the attempt was rolled back: the old state stays
+    if (accepted) {
+      flag = (uint8_t)fl;
+      tau = tn;
+    }
+    if (P::kKeep || accepted) p.accept(accepted);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    s_k.status = s_k.status != PLIS_OK ? s_k.status : __ldcg(&A.b.ctrl->status);
+    *A.b.ctrl = s_k;
+  }
 }
 
 #ifdef PLIS_ENGINE_HOST_TU
@@ -2228,8 +2529,12 @@ struct KernelSet {
   // the largest shared memory any network asks for: one value, so that no handle lowers another's limit
   static cudaError_t net_smem_limit() {
     constexpr int leap = (int)net_smem<Real>(kNetS, kNetR, true), rest = (int)net_smem<Real>(kNetS, kNetR, false);
+    const void* steps[] = {(const void*)k_steps<NetPhases<Real, true, true>>, (const void*)k_steps<NetPhases<Real, true, false>>,
+                           (const void*)k_steps<NetPhases<Real, false, true>>, (const void*)k_steps<NetPhases<Real, false, false>>};
     cudaError_t e = net_limits<false>(leap, rest);
-    return e == cudaSuccess ? net_limits<true>(leap, rest) : e;
+    if (e == cudaSuccess) e = net_limits<true>(leap, rest);
+    for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaFuncSetAttribute(steps[i], cudaFuncAttributeMaxDynamicSharedMemorySize, leap);
+    return e;
   }
   template <bool COMP>
   static cudaError_t net_limits(int leap, int rest) {
@@ -2253,6 +2558,25 @@ struct KernelSet {
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_leap<Real, MAXS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e;
+  }
+  // the persistent kernel of a handle and its shared memory; null where only the phase kernels exist
+  static StepsKernel steps(const KArgs& a) {
+    if constexpr (kSmallOk) {
+      if (a.sm.on) {
+        if (a.m.lattice) return {(const void*)k_steps<SmallPhases<Real, MAXS, true>>, 0};
+        return {(const void*)k_steps<SmallPhases<Real, MAXS, false>>, 0};
+      }
+    }
+    if (a.o.net) {
+      const size_t bytes = net_smem<Real>(a.m.S, a.m.R, true);
+      if (a.m.lattice) {
+        if (a.m.comp) return {(const void*)k_steps<NetPhases<Real, true, true>>, bytes};
+        return {(const void*)k_steps<NetPhases<Real, true, false>>, bytes};
+      }
+      if (a.m.comp) return {(const void*)k_steps<NetPhases<Real, false, true>>, bytes};
+      return {(const void*)k_steps<NetPhases<Real, false, false>>, bytes};
+    }
+    return {nullptr, 0};
   }
   static void exact(const KArgs& a, dim3 g, dim3 b, cudaStream_t s) {
     if (a.o.net) {
@@ -2301,14 +2625,14 @@ struct KernelSet {
 
 template <typename Real>
 Launchers pick_impl(uint32_t S) {
-  if (S <= 1) return {KernelSet<Real, 1>::leap, KernelSet<Real, 1>::exact, KernelSet<Real, 1>::classify, KernelSet<Real, 1>::leap_smem, KernelSet<Real, 1>::net_smem_limit};
-  if (S <= 2) return {KernelSet<Real, 2>::leap, KernelSet<Real, 2>::exact, KernelSet<Real, 2>::classify, KernelSet<Real, 2>::leap_smem, KernelSet<Real, 2>::net_smem_limit};
-  if (S <= 4) return {KernelSet<Real, 4>::leap, KernelSet<Real, 4>::exact, KernelSet<Real, 4>::classify, KernelSet<Real, 4>::leap_smem, KernelSet<Real, 4>::net_smem_limit};
-  if (S <= 8) return {KernelSet<Real, 8>::leap, KernelSet<Real, 8>::exact, KernelSet<Real, 8>::classify, KernelSet<Real, 8>::leap_smem, KernelSet<Real, 8>::net_smem_limit};
-  if (S <= 16) return {KernelSet<Real, 16>::leap, KernelSet<Real, 16>::exact, KernelSet<Real, 16>::classify, KernelSet<Real, 16>::leap_smem, KernelSet<Real, 16>::net_smem_limit};
-  if (S <= 32) return {KernelSet<Real, 32>::leap, KernelSet<Real, 32>::exact, KernelSet<Real, 32>::classify, KernelSet<Real, 32>::leap_smem, KernelSet<Real, 32>::net_smem_limit};
-  if (S <= 64) return {KernelSet<Real, 64>::leap, KernelSet<Real, 64>::exact, KernelSet<Real, 64>::classify, KernelSet<Real, 64>::leap_smem, KernelSet<Real, 64>::net_smem_limit};
-  return {KernelSet<Real, 256>::leap, KernelSet<Real, 256>::exact, KernelSet<Real, 256>::classify, KernelSet<Real, 256>::leap_smem, KernelSet<Real, 256>::net_smem_limit};
+  if (S <= 1) return {KernelSet<Real, 1>::leap, KernelSet<Real, 1>::exact, KernelSet<Real, 1>::classify, KernelSet<Real, 1>::leap_smem, KernelSet<Real, 1>::net_smem_limit, KernelSet<Real, 1>::steps};
+  if (S <= 2) return {KernelSet<Real, 2>::leap, KernelSet<Real, 2>::exact, KernelSet<Real, 2>::classify, KernelSet<Real, 2>::leap_smem, KernelSet<Real, 2>::net_smem_limit, KernelSet<Real, 2>::steps};
+  if (S <= 4) return {KernelSet<Real, 4>::leap, KernelSet<Real, 4>::exact, KernelSet<Real, 4>::classify, KernelSet<Real, 4>::leap_smem, KernelSet<Real, 4>::net_smem_limit, KernelSet<Real, 4>::steps};
+  if (S <= 8) return {KernelSet<Real, 8>::leap, KernelSet<Real, 8>::exact, KernelSet<Real, 8>::classify, KernelSet<Real, 8>::leap_smem, KernelSet<Real, 8>::net_smem_limit, KernelSet<Real, 8>::steps};
+  if (S <= 16) return {KernelSet<Real, 16>::leap, KernelSet<Real, 16>::exact, KernelSet<Real, 16>::classify, KernelSet<Real, 16>::leap_smem, KernelSet<Real, 16>::net_smem_limit, KernelSet<Real, 16>::steps};
+  if (S <= 32) return {KernelSet<Real, 32>::leap, KernelSet<Real, 32>::exact, KernelSet<Real, 32>::classify, KernelSet<Real, 32>::leap_smem, KernelSet<Real, 32>::net_smem_limit, KernelSet<Real, 32>::steps};
+  if (S <= 64) return {KernelSet<Real, 64>::leap, KernelSet<Real, 64>::exact, KernelSet<Real, 64>::classify, KernelSet<Real, 64>::leap_smem, KernelSet<Real, 64>::net_smem_limit, KernelSet<Real, 64>::steps};
+  return {KernelSet<Real, 256>::leap, KernelSet<Real, 256>::exact, KernelSet<Real, 256>::classify, KernelSet<Real, 256>::leap_smem, KernelSet<Real, 256>::net_smem_limit, KernelSet<Real, 256>::steps};
 }
 
 

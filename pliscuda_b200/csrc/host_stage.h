@@ -2,7 +2,7 @@
 //
 // A copy from pageable memory goes through the driver's staging on the calling thread, 4-5 GB/s on the
 // measured host for states of tens of megabytes, and a small one waits for the device.  Here the
-// bytes pass through pinned slices that belong to the handle (at most kSlices x 1 MB, freed with it):
+// bytes pass through pinned slices that belong to the handle (at most kSlices x 512 KB, freed with it):
 // large states with kWorkers threads, each alternating between its own slices so that its memcpy
 // overlaps its DMA (pages of a fresh result array are then touched by several threads too), small ones
 // by the caller, which need not wait for the device before it returns from an upload.
@@ -67,10 +67,10 @@ class HostStage {
   static constexpr int kSlices = 8, kWorkers = 4;
   ~HostStage() { release(); }
 
-  // slices for pieces of up to `piece` bytes (a piece above 1 MB passes in parts)
+  // slices for pieces of up to `piece` bytes (a piece above 512 KB passes in parts)
   cudaError_t init(int device, size_t piece) {
     device_ = device;
-    slice_ = std::min<size_t>(size_t(1) << 20, (piece + 4095) / 4096 * 4096);
+    slice_ = std::min<size_t>(size_t(512) << 10, (piece + 4095) / 4096 * 4096);
     if (slice_ == 0) slice_ = 4096;
     cudaError_t e = cudaMallocHost((void**)&buf_, slice_ * kSlices);
     if (e != cudaSuccess) { buf_ = nullptr; return e; }

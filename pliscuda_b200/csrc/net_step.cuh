@@ -119,18 +119,15 @@ __device__ __forceinline__ void net_dirs(const DevModel& m, const Cell& cl, Dirs
 // ------------------------------------------------------------------------------------------------
 // leap of one brick (leap_step, leap.cu:3-65), pooled or not
 // ------------------------------------------------------------------------------------------------
+// One subvolume's leap.  fresh: the rows still hold the counts and, 0 for critical reactions, the
+// propensities that its classification put there; else they are read and formed here.
 template <typename Real, bool LOG, bool LAT, bool COMP>
-__device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const LeapCtx& L,
-                                              Real tl, unsigned char* smem, long long& ev_out, int& big) {
+__device__ __forceinline__ void leap_cell_net(const KArgs& A, const NetTab<Real>& T, const Cell& cl, uint8_t f, bool fresh,
+                                              const LeapCtx& L, Real tl, unsigned char* smem, long long& ev_out, int& big) {
   const DevModel& m = A.m;
   const int nc = A.o.nc, mode = A.o.mode;
   const int S = (int)m.S, R = (int)m.R;
-  ev_out = 0;
-  big = 0;
-  Cell cl;
-  if (!cell_of(A, tile, cl)) return;
   const uint32_t c = cl.c;
-  const uint8_t f = L.flag[c];
   const Column<Real> sx = column<Real>(smem, 0);                                       // [S] counts
   const Column<Real> sl = column<Real>(smem, sizeof(Real) * (size_t)S);                // [R] means of the firing reactions
   const Column<int32_t> sd = column<int32_t>(smem, sizeof(Real) * (size_t)(S + R));    // [S] net changes
@@ -144,7 +141,7 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
   }
 #pragma unroll 4
   for (int s = 0; s < S; ++s) {
-    sx[s] = (Real)L.Xc[(size_t)s * m.Npad + c];
+    if (!fresh) sx[s] = (Real)L.Xc[(size_t)s * m.Npad + c];
     sd[s] = 0;
   }
   // Net changes of 2^24 and more go to 64-bit sums in local memory; the others, at most one per
@@ -188,8 +185,8 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
       const int r = r0 + i;
       lam[i] = (Real)0;
       if (r < R) {
-        bool crit;
-        const Real a = net_prop<Real, COMP>(T, m, comp, sx, r, crit);
+        bool crit = false;
+        const Real a = fresh ? sl[r] : net_prop<Real, COMP>(T, m, comp, sx, r, crit);
         Real lr = crit ? (Real)0 : tl * a;
         if (!(lr > (Real)0)) lr = (Real)0;
         sl[r] = lr;
@@ -344,6 +341,16 @@ __device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>
     if (tv >= kBigTile || tv <= -kBigTile) big = 1;
     atomicAdd(&L.Xt[(size_t)s * m.Npad + c], (int)tv);
   }
+}
+
+template <typename Real, bool LOG, bool LAT, bool COMP>
+__device__ __forceinline__ void leap_tile_net(const KArgs& A, const NetTab<Real>& T, uint32_t tile, const LeapCtx& L,
+                                              Real tl, unsigned char* smem, long long& ev_out, int& big) {
+  ev_out = 0;
+  big = 0;
+  Cell cl;
+  if (!cell_of(A, tile, cl)) return;
+  leap_cell_net<Real, LOG, LAT, COMP>(A, T, cl, L.flag[cl.c], false, L, tl, smem, ev_out, big);
 }
 
 // ------------------------------------------------------------------------------------------------

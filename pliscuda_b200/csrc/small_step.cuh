@@ -180,26 +180,21 @@ __device__ __forceinline__ uint32_t lattice_dirs(const DevModel& m, const Cell& 
          (cl.z > 0 ? 16u : 0u) | (cl.z + 1 < m.Z ? 32u : 0u);
 }
 
+// One subvolume's leap from its counts x and flag f.
 // LAT: a lattice (directions by coordinates), else a neighbour table (slot j = direction j).
 // RK: group blocks from the round keys in the kernel arguments.
 template <typename Real, int MAXS, bool LOG, bool LAT, bool RK>
-__device__ __forceinline__ void leap_tile_small(const KArgs& A, const SmallModel& t, uint32_t tile, const LeapCtx& L,
-                                                Real tl, long long& ev_out, int& big) {
+__device__ __forceinline__ void leap_cell_small(const KArgs& A, const SmallModel& t, const Cell& cl, const int32_t x[MAXS],
+                                                uint8_t f, const LeapCtx& L, Real tl, long long& ev_out, int& big) {
   const DevModel& m = A.m;
   const int nc = A.o.nc, mode = A.o.mode;
   const int S = (int)m.S;
-  ev_out = 0;
-  big = 0;
-  Cell cl;
-  if (!cell_of(A, tile, cl)) return;
   const uint32_t c = cl.c;
-  const uint8_t f = L.flag[c];
-  int32_t x[MAXS], dl[MAXS];
+  int32_t dl[MAXS];
   long long dbig[MAXS];  // net changes of the draws counted in 64 bits
   bool wide = false;
 #pragma unroll
   for (int s = 0; s < MAXS; ++s) {
-    x[s] = s < S ? L.Xc[(size_t)s * m.Npad + c] : 0;
     dl[s] = 0;
     dbig[s] = 0;
   }
@@ -354,6 +349,21 @@ __device__ __forceinline__ void leap_tile_small(const KArgs& A, const SmallModel
     if (tv >= kBigTile || tv <= -kBigTile) big = 1;
     atomicAdd(&L.Xt[(size_t)s * m.Npad + c], (int)tv);
   }
+}
+
+template <typename Real, int MAXS, bool LOG, bool LAT, bool RK>
+__device__ __forceinline__ void leap_tile_small(const KArgs& A, const SmallModel& t, uint32_t tile, const LeapCtx& L,
+                                                Real tl, long long& ev_out, int& big) {
+  const DevModel& m = A.m;
+  ev_out = 0;
+  big = 0;
+  Cell cl;
+  if (!cell_of(A, tile, cl)) return;
+  const uint8_t f = L.flag[cl.c];
+  int32_t x[MAXS];
+#pragma unroll
+  for (int s = 0; s < MAXS; ++s) x[s] = s < (int)m.S ? L.Xc[(size_t)s * m.Npad + cl.c] : 0;
+  leap_cell_small<Real, MAXS, LOG, LAT, RK>(A, t, cl, x, f, L, tl, ev_out, big);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -13,8 +13,8 @@ def _sim(n, species):
     return Simulation(m)
 
 
-@pytest.mark.parametrize("n,species", [(1, 1), (1000, 3), ((1 << 21) - 1, 1), (1 << 21, 1), ((1 << 21) + 33, 1), (700_001, 3),
-                                       (262_144, 16), (262_145, 17)])
+@pytest.mark.parametrize("n,species", [(1, 1), (1000, 3), ((1 << 21) + 33, 1), ((1 << 23) - 1, 1), (1 << 23, 1), ((1 << 23) + 33, 1),
+                                       (700_001, 13), (524_289, 17)])
 def test_round_trip(n, species):
     import torch
     rng = np.random.default_rng(n)
@@ -32,7 +32,7 @@ def test_round_trip(n, species):
         assert np.array_equal(sim.get_state(out), keep[::-1]) and np.array_equal(sim.get_state(), keep[::-1])
 
 
-@pytest.mark.parametrize("n", [100, (1 << 21) + 5])
+@pytest.mark.parametrize("n", [100, (1 << 23) + 5])
 def test_refused_state_leaves_the_old_one(n):
     from pliscuda_b200 import PlisError
     rng = np.random.default_rng(1)
