@@ -34,7 +34,10 @@ namespace plis {
 // round trip, for which its pinned slices (4-8 ms to allocate) are not worth having.
 constexpr size_t kStagedState = size_t(32) << 20;
 
-constexpr uint64_t kStepsMin = 6;
+// Steps of one call from which k_steps is used: its cooperative launch costs about 40 us over the first of
+// the phase kernels, and a step about 10 us against 17 (1,000 subvolumes: 2 steps 65 us with the phase
+// kernels, 6 steps 100 us in k_steps against 136).
+constexpr uint64_t kStepsMin = 3;
 
 static uint32_t pow2_at_least(uint32_t v) {
   uint32_t p = 1;

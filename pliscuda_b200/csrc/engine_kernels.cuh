@@ -1605,9 +1605,11 @@ __global__ void __launch_bounds__(256) k_exact_net(const __grid_constant__ NetAr
       }
       __syncthreads();
       const uint32_t n = s_n;
-      for (uint32_t j = threadIdx.x; j < n; j += blockDim.x)
-        fired += critical_event_net<Real, LOG, COMP>(A, net_tab<Real>(A), base + s_cell[j], sx, sa, Xc, Xt, step, attempt,
-                                                     A.b.D, flag);
+      for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+        const uint32_t c = base + s_cell[j];
+        net_rows(m, Xc, c, (int)m.S, [&](int s, int32_t xs) { sx[s] = (Real)xs; });
+        fired += critical_event_net<Real, LOG, COMP>(A, net_tab<Real>(A), c, sx, sa, Xt, step, attempt, A.b.D, flag);
+      }
       __syncthreads();
     }
   }
@@ -1637,10 +1639,13 @@ __global__ void __launch_bounds__(256) k_apply(KArgs A) {
     const uint32_t* list = touched_list(A);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
       const uint32_t c = list[i];
-      for (uint32_t s = 0; s < m.S; ++s) {
-        const size_t j = (size_t)s * m.Npad + c;
-        const int32_t v = atomicExch(&A.b.D[j], 0);
-        if (v) atomicAdd(&Xt[j], v);
+      for (uint32_t s0 = 0; s0 < m.S; s0 += 5) {  // five exchanges in flight
+        int32_t v[5];
+#pragma unroll
+        for (uint32_t k = 0; k < 5; ++k) v[k] = s0 + k < m.S ? atomicExch(&A.b.D[(size_t)(s0 + k) * m.Npad + c], 0) : 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 5; ++k)
+          if (v[k]) atomicAdd(&Xt[(size_t)(s0 + k) * m.Npad + c], v[k]);
       }
     }
     return;
@@ -2150,9 +2155,9 @@ template <typename Real_, bool LAT, bool COMP> struct NetPhases {
     leap_cell_net<Real, false, LAT, COMP>(A, net_tab<Real>(A), cl, f, fresh, L, tl, sm, ev, big);
   }
   __device__ __forceinline__ int critical(const Args& A, uint32_t c, const LeapCtx& L, unsigned char* sm) {
-    return critical_event_net<Real, false, COMP>(A, net_tab<Real>(A), c, column<Real>(sm, 0),
-                                                 column<Real>(sm, sizeof(Real) * (size_t)A.m.S), L.Xc, L.Xt, L.step, L.attempt,
-                                                 A.b.D, L.flag);
+    const Column<Real> sx = column<Real>(sm, 0);  // still the counts the leap started from
+    return critical_event_net<Real, false, COMP>(A, net_tab<Real>(A), c, sx, column<Real>(sm, sizeof(Real) * (size_t)A.m.S), L.Xt,
+                                                 L.step, L.attempt, A.b.D, L.flag);
   }
   __device__ __forceinline__ void classify(const Args& A, const Cell& cl, const ClassifyCtx& C, double tau_cur, uint8_t flag_cur,
                                            unsigned char* sm, double& tn, int& fl, int& bad) {
@@ -2221,16 +2226,14 @@ __global__ void __launch_bounds__(256, kStepsCtas) k_steps(const __grid_constant
       }
       if (!steps_sync(R, A.b.ctrl, target)) return;
       if (ex & 1u) {  // the staged deltas of this CTA's subvolumes
-        if (mine) {
-          for (uint32_t s = 0; s < m.S; ++s) {
+        if (mine)
+          net_rows(m, A.b.D, c, (int)m.S, [&](int s, int32_t v) {
             const size_t j = (size_t)s * m.Npad + c;
-            const int32_t v = A.b.D[j];
             if (v) {
               L.Xt[j] += v;
               A.b.D[j] = 0;
             }
-          }
-        }
+          });
         if (!steps_sync(R, A.b.ctrl, target)) return;
       }
     }
