@@ -50,8 +50,7 @@ Engine::Engine() {}
 Engine::~Engine() { release(); }
 
 void Engine::release() {
-  if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-  graph_exec_ = nullptr;
+  drop_graphs();
   if (d_evrec_) cudaFree(d_evrec_);
   if (d_evhead_) cudaFree(d_evhead_);
   d_evrec_ = nullptr;
@@ -392,19 +391,28 @@ int Engine::create(const Model& model, const plis_options& opt) {
   return PLIS_OK;
 }
 
-void Engine::launch_classify() {
-  const dim3 gc(slab_blocks_ ? slab_blocks_ : args_.g.nblocks), bc(args_.g.threads);
-  if (use_learned_) llaunch_.classify(args_, gc, bc, stream_);
-  else launch_.classify(args_, gc, bc, stream_);
+void Engine::drop_graphs() {
+  for (auto& g : graph_exec_) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
 }
 
-void Engine::enqueue_step() {
-  const dim3 gc(args_.g.nblocks), bc(args_.g.threads);
+void Engine::launch_classify(const NetArgs& a) {
+  const dim3 gc(slab_blocks_ ? slab_blocks_ : a.g.nblocks), bc(a.g.threads);
+  if (use_learned_) llaunch_.classify(a, gc, bc, stream_);
+  else launch_.classify(a, gc, bc, stream_);
+}
+
+void Engine::enqueue_step(const NetArgs& a, bool lean) {
+  const dim3 gc(a.g.nblocks), bc(a.g.threads);
   const dim3 gx(exact_blocks_), bx(256);
-  launch_.leap(args_, gc, bc, stream_);
-  launch_.exact(args_, gx, bx, stream_);
-  if (opt_.mode == PLIS_MODE_REFERENCE) launch_pdl(k_apply, gx, bx, 0, stream_, args_);
-  launch_classify();
+  launch_.leap(a, gc, bc, stream_);
+  if (!lean) {
+    launch_.exact(a, gx, bx, stream_);
+    if (opt_.mode == PLIS_MODE_REFERENCE) launch_pdl(k_apply, gx, bx, 0, stream_, (KArgs)a);
+  }
+  launch_classify(a);
 }
 
 // Profiled step: the same four launches with CUDA events between them, accumulated per kernel.
@@ -418,9 +426,9 @@ int Engine::enqueue_step_profiled() {
   PLIS_CU(cudaEventRecord(pev_[1], stream_));
   launch_.exact(args_, gx, bx, stream_);
   PLIS_CU(cudaEventRecord(pev_[2], stream_));
-  if (opt_.mode == PLIS_MODE_REFERENCE) launch_pdl(k_apply, gx, bx, 0, stream_, args_);
+  if (opt_.mode == PLIS_MODE_REFERENCE) launch_pdl(k_apply, gx, bx, 0, stream_, (KArgs)args_);
   PLIS_CU(cudaEventRecord(pev_[3], stream_));
-  launch_classify();
+  launch_classify(args_);
   PLIS_CU(cudaEventRecord(pev_[4], stream_));
   PLIS_CU(cudaEventSynchronize(pev_[4]));
   const int kind[4] = {PLIS_KERNEL_LEAP, PLIS_KERNEL_EXACT, PLIS_KERNEL_APPLY, PLIS_KERNEL_CLASSIFY};
@@ -439,17 +447,20 @@ int Engine::profile(plis_profile* p) {
   return PLIS_OK;
 }
 
-int Engine::build_graph() {
-  if (graph_exec_) return PLIS_OK;
+int Engine::build_graph(bool lean) {
+  cudaGraphExec_t& exec = graph_exec_[lean ? 1 : 0];
+  if (exec) return PLIS_OK;
+  NetArgs a = args_;
+  a.o.lean = lean ? 1u : 0u;
   cudaGraph_t graph = nullptr;
   PLIS_CU(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < graph_steps_; ++i) enqueue_step();
+  for (int i = 0; i < graph_steps_; ++i) enqueue_step(a, lean);
   PLIS_CU(cudaStreamEndCapture(stream_, &graph));
-  cudaError_t e = cudaGraphInstantiate(&graph_exec_, graph, 0);
+  cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) {
     err_ = std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e);
-    graph_exec_ = nullptr;
+    exec = nullptr;
     return PLIS_ERR_CUDA;
   }
   return PLIS_OK;
@@ -488,7 +499,7 @@ int Engine::set_state(const uint32_t* counts, double t0, uint64_t step0) {
   k.step = step0;
   const uint32_t rb = (dm.Npad + 255u) / 256u;
   k_reset<<<rb < 2048u ? rb : 2048u, 256, 0, stream_>>>(args_, k);
-  launch_classify();
+  launch_classify(args_);
   launches_ += 2;
   PLIS_CU(cudaGetLastError());
   int rc = read_ctrl();
@@ -510,7 +521,7 @@ int Engine::reclassify() {
   h_ctrl_->done = 0;
   ctrl_fresh_ = false;
   PLIS_CU(cudaMemcpyAsync(args_.b.ctrl, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_));
-  launch_classify();
+  launch_classify(args_);
   launches_ += 1;
   PLIS_CU(cudaGetLastError());
   return read_ctrl();
@@ -552,10 +563,7 @@ int Engine::set_proposer(const float* weights, double s_max) {
   use_learned_ = on;
   const int classify_launches = (on && opt_.learned_mlp == PLIS_MLP_TCGEN05) ? 2 : 1;
   kernels_per_step_ = ((opt_.mode == PLIS_MODE_REFERENCE) ? 4 : 3) + classify_launches - 1;
-  if (graph_exec_) {  // the graph holds the kernel arguments by value
-    cudaGraphExecDestroy(graph_exec_);
-    graph_exec_ = nullptr;
-  }
+  drop_graphs();  // they hold the kernel arguments by value
   return state_set_ ? reclassify() : PLIS_OK;
 }
 
@@ -630,10 +638,7 @@ int Engine::set_event_log(uint64_t capacity) {
     PLIS_CU(cudaStreamSynchronize(stream_));
     args_.b.ev = EvLog{d_evrec_, d_evhead_, (unsigned long long)capacity};
   }
-  if (graph_exec_) {  // the graph holds the kernel arguments by value
-    cudaGraphExecDestroy(graph_exec_);
-    graph_exec_ = nullptr;
-  }
+  drop_graphs();  // they hold the kernel arguments by value
   return PLIS_OK;
 }
 
@@ -659,6 +664,11 @@ int Engine::read_event_log(plis_event_record* out, uint64_t max_records, uint64_
   *n_dropped = head - stored;
   return PLIS_OK;
 }
+
+// Batches of steps.  Most steps of a system without scarce species have no exact events, and the two kernels
+// for them, which then find nothing to do, cost 1 us each (31.6 -> 29.6 us a step on Schlogl 64^3 without).
+// So a batch first goes without them (DevOpts::lean); where a step needs them the batch stops there, and
+// the following ones carry them, twice as many each time that happens, before it is tried again.
 
 // The prepared run in k_steps launches (a launch ends after a few thousand attempts at the latest, so
 // that it does not hold the GPU for long).
@@ -687,8 +697,13 @@ int Engine::advance(double t_end, uint64_t n_steps) {
   // a cooperative launch starts later than the phase kernels of a few steps finish
   const bool resident = steps_.kernel && !use_learned_ && !args_.b.ev.rec && n_steps >= kStepsMin;
   const bool few = n_steps != ~0ull && n_steps < (uint64_t)graph_steps_;
+  if (ctrl_fresh_ && lean_) {  // the first step's exact events are known before it is planned
+    const uint32_t af = h_ctrl_->argmin_flag;
+    const bool events = opt_.mode == PLIS_MODE_REFERENCE ? h_ctrl_->n_leap_cr > 0 || af == F_SSA || af == F_SSA_FF : af != F_LEAP_NOCR;
+    if (events) lean_ = false;
+  }
   if (!few && !opt_.profile && !resident) {  // the one-off capture and instantiation stay out of the timed interval
-    int rc = build_graph();
+    int rc = build_graph(lean_);
     if (rc) return rc;
   }
   ctrl_fresh_ = false;
@@ -722,11 +737,13 @@ int Engine::advance(double t_end, uint64_t n_steps) {
   }
   while (!resident) {
     if (few) {
-      for (uint64_t i = 0; i < budget; ++i) enqueue_step();
+      for (uint64_t i = 0; i < budget; ++i) enqueue_step(args_, false);
       launches_ += budget * kernels_per_step_;
     } else {
-      PLIS_CU(cudaGraphLaunch(graph_exec_, stream_));
-      launches_ += (uint64_t)graph_steps_ * kernels_per_step_;
+      int rc = build_graph(lean_);
+      if (rc) return rc;
+      PLIS_CU(cudaGraphLaunch(graph_exec_[lean_ ? 1 : 0], stream_));
+      launches_ += (uint64_t)graph_steps_ * (lean_ ? kernels_per_step_ - (opt_.mode == PLIS_MODE_REFERENCE ? 2 : 1) : kernels_per_step_);
     }
     PLIS_CU(cudaGetLastError());
     ctrl_fresh_ = false;
@@ -735,6 +752,18 @@ int Engine::advance(double t_end, uint64_t n_steps) {
     if (h_ctrl_->done) break;
     if (few) {  // rollbacks used up some of the per-call launches
       budget = 1;
+    } else if (lean_) {
+      if (h_ctrl_->exact) {  // the batch stopped at a step with exact events: the next ones carry their kernels
+        lean_ = false;
+        lean_wait_ = lean_back_;
+        if (lean_back_ < 1024u) lean_back_ *= 2;
+      } else {
+        lean_back_ = 1;
+      }
+    } else if (lean_wait_ > 0) {
+      --lean_wait_;
+    } else if (h_ctrl_->exact == 0) {
+      lean_ = true;
     }
   }
   PLIS_CU(cudaEventRecord(ev1_, stream_));
@@ -793,10 +822,7 @@ int Engine::slab_setup(uint32_t z0, uint32_t z1, uint32_t world, uint32_t rank) 
   PLIS_CU(cudaMemset((void*)L.all, 0, (size_t)world * sizeof(SlabSummary)));
   PLIS_CU(cudaMemset((void*)L.remote_all, 0, (size_t)world * sizeof(SlabRemote)));
   L.on = 1;
-  if (graph_exec_) {  // the graph holds the kernel arguments by value
-    cudaGraphExecDestroy(graph_exec_);
-    graph_exec_ = nullptr;
-  }
+  drop_graphs();  // they hold the kernel arguments by value
   return PLIS_OK;
 }
 
@@ -828,7 +854,7 @@ int Engine::slab_phase(int phase, double t_end, uint64_t n_steps) {
   PLIS_CU(cudaEventRecord(ev0_, stream_));
   switch (phase) {
     case PLIS_SLAB_CLASSIFY:
-      launch_classify();
+      launch_classify(args_);
       launches_ += 1;
       break;
     case PLIS_SLAB_CONTROL:

@@ -129,6 +129,8 @@ struct DevOpts {
   uint32_t replica;
   uint32_t pool;      // 1: pooled draws of small-mean channels in the generic leap (plis_stream.h)
   uint32_t net;       // 1: the arguments are a NetArgs with filled tables
+  uint32_t lean;      // 1: no exact-event kernels between the leap and the classification: both leave a step that
+                      // needs them alone, for a launch with them (Engine::advance)
   uint32_t no_list;   // 1: exact events do not list the delta rows they write (k_steps applies every row)
   uint32_t rk0[10], rk1[10];  // Philox round keys of (seed, replica): plis_round_keys, set with devopts_keys
 };

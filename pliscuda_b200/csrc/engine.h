@@ -71,9 +71,10 @@ class Engine {
   void release();
   int dmalloc(void** p, size_t bytes);
   template <typename T> int upload(const std::vector<T>& v, const T** out);
-  void enqueue_step();
-  void launch_classify();
-  int build_graph();
+  void enqueue_step(const NetArgs& a, bool lean);
+  void launch_classify(const NetArgs& a);
+  int build_graph(bool lean);
+  void drop_graphs();
   int advance_steps();
   int read_ctrl();
   int reclassify();
@@ -83,7 +84,10 @@ class Engine {
   NetArgs args_{};
   Launchers launch_{};
   cudaStream_t stream_ = nullptr;
-  cudaGraphExec_t graph_exec_ = nullptr;
+  cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};  // batches of steps: with the exact-event kernels, without
+  bool lean_ = true;         // the next batch is tried without them
+  uint32_t lean_wait_ = 0;   // batches with them before that is tried again
+  uint32_t lean_back_ = 1;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   Ctrl* h_ctrl_ = nullptr;
   bool ctrl_fresh_ = false;  // h_ctrl_ holds the device's control block (nothing has run since it was read)

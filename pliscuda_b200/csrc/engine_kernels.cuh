@@ -1218,11 +1218,17 @@ __device__ __forceinline__ void leap_totals(Ctrl* K, long long ev, int big) {
   }
 }
 
+// nothing to do for the leap and the classification: the run has ended, or the step waits for a launch
+// with the exact-event kernels
+__device__ __forceinline__ int step_idle(const KArgs& A, const Ctrl* K) {
+  return K->done | (int)(A.o.lean & (K->exact != 0u ? 1u : 0u));
+}
+
 template <typename Real, int MAXS, bool LOG, bool LAT>
 __global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap_small(const __grid_constant__ KArgs A) {
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  const int done = K->done;
+  const int done = step_idle(A, K);
   const LeapCtx L = leap_ctx(A, K);
   const Real tl = (Real)K->tau_leap;
   if (done) return;
@@ -1236,7 +1242,7 @@ template <typename Real, int MAXS, bool LOG>
 __global__ void __launch_bounds__(256, PLIS_LEAP_MIN_BLOCKS) k_leap(KArgs A) {
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  if (K->done) return;
+  if (step_idle(A, K)) return;
   extern __shared__ int32_t s_box[];
   const LeapCtx L = leap_ctx(A, K);
   const Real tl = (Real)K->tau_leap;
@@ -1555,7 +1561,7 @@ __global__ void __launch_bounds__(256, 3) k_leap_net(const __grid_constant__ Net
   extern __shared__ __align__(16) unsigned char s_net[];
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  const int done = K->done;
+  const int done = step_idle(A, K);
   const LeapCtx L = leap_ctx(A, K);
   const Real tl = (Real)K->tau_leap;
   if (done) return;
@@ -2000,7 +2006,7 @@ template <typename Real, int MAXS, bool LAT>
 __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify_small(const __grid_constant__ KArgs A) {
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  const int done = K->done;
+  const int done = step_idle(A, K);
   const ClassifyCtx C = classify_ctx(A, K);
   if (blockIdx.x == 0 && threadIdx.x == 0) K->n_touched = 0;  // k_apply has consumed the list
   if (done) return;
@@ -2018,7 +2024,7 @@ __global__ void __launch_bounds__(256, NetCtas<Real>::n) k_classify_net(const __
   extern __shared__ __align__(16) unsigned char s_net[];
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  const int done = K->done;
+  const int done = step_idle(A, K);
   const ClassifyCtx C = classify_ctx(A, K);
   if (blockIdx.x == 0 && threadIdx.x == 0) K->n_touched = 0;  // k_apply has consumed the list
   if (done) return;
@@ -2037,7 +2043,7 @@ __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify(KArg
   pdl_entry();
   if (blockIdx.x == 0 && threadIdx.x == 0) A.b.ctrl->n_touched = 0;  // k_apply has consumed the list
   Ctrl* K = A.b.ctrl;
-  if (K->done) return;
+  if (step_idle(A, K)) return;
   const ClassifyCtx C = classify_ctx(A, K);
   double tn;
   uint32_t ti;

@@ -64,7 +64,7 @@ template <typename Real, int MAXS>
 __global__ void __launch_bounds__(256, 2) k_classify_learned(KArgs A) {
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  if (K->done) return;
+  if (step_idle(A, K)) return;
   const ClassifyCtx C = classify_ctx(A, K);
   if (learned_classify_tile<Real, MAXS>(A, K, C, blockIdx.x, gridDim.x)) classify_control(A, K, gridDim.x);
 }
@@ -80,7 +80,7 @@ template <typename Real, int MAXS, bool SMALL>
 __global__ void __launch_bounds__(256, 4) k_learned_pre(const __grid_constant__ KArgs A) {
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  const int done = K->done;
+  const int done = step_idle(A, K);
   const ClassifyCtx C = classify_ctx(A, K);
   if (done) return;
   const LearnedParams* P = A.b.lp;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2) k_learned_decide(const __grid
   extern __shared__ __align__(128) uint8_t tsm[];
   pdl_entry();
   Ctrl* K = A.b.ctrl;
-  const int done = K->done;
+  const int done = step_idle(A, K);
   const ClassifyCtx C = classify_ctx(A, K);
   if (blockIdx.x == 0 && threadIdx.x == 0) K->n_touched = 0;
   if (done) return;
