@@ -385,7 +385,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
       }
     }
   }
-  kernels_per_step_ = (opt.mode == PLIS_MODE_REFERENCE) ? 4 : 3;
+  kernels_per_step_ = ((opt.mode == PLIS_MODE_REFERENCE) ? 3 : 2) + classify_kernels();
   graph_steps_ = opt.steps_per_launch > 0 ? opt.steps_per_launch : 32;
   PLIS_CU(cudaDeviceSynchronize());
   return PLIS_OK;
@@ -400,8 +400,18 @@ void Engine::drop_graphs() {
 
 void Engine::launch_classify(const NetArgs& a) {
   const dim3 gc(slab_blocks_ ? slab_blocks_ : a.g.nblocks), bc(a.g.threads);
-  if (use_learned_) llaunch_.classify(a, gc, bc, stream_);
-  else launch_.classify(a, gc, bc, stream_);
+  if (use_learned_) {
+    llaunch_.classify(a, gc, bc, stream_);
+    return;
+  }
+  launch_.classify(a, gc, bc, stream_);
+  if (a.sm.on || a.o.net) launch_pdl(k_control, dim3(1), dim3(512), 0, stream_, (KArgs)a, gc.x);
+}
+
+// kernels of a classification, and of a step
+int Engine::classify_kernels() const {
+  if (use_learned_) return opt_.learned_mlp == PLIS_MLP_TCGEN05 ? 2 : 1;
+  return args_.sm.on || args_.o.net ? 2 : 1;
 }
 
 void Engine::enqueue_step(const NetArgs& a, bool lean) {
@@ -500,7 +510,7 @@ int Engine::set_state(const uint32_t* counts, double t0, uint64_t step0) {
   const uint32_t rb = (dm.Npad + 255u) / 256u;
   k_reset<<<rb < 2048u ? rb : 2048u, 256, 0, stream_>>>(args_, k);
   launch_classify(args_);
-  launches_ += 2;
+  launches_ += 1 + classify_kernels();
   PLIS_CU(cudaGetLastError());
   int rc = read_ctrl();
   if (rc) return rc;
@@ -522,7 +532,7 @@ int Engine::reclassify() {
   ctrl_fresh_ = false;
   PLIS_CU(cudaMemcpyAsync(args_.b.ctrl, h_ctrl_, sizeof(Ctrl), cudaMemcpyHostToDevice, stream_));
   launch_classify(args_);
-  launches_ += 1;
+  launches_ += classify_kernels();
   PLIS_CU(cudaGetLastError());
   return read_ctrl();
 }
@@ -561,8 +571,7 @@ int Engine::set_proposer(const float* weights, double s_max) {
     args_.b.lp = nullptr;
   }
   use_learned_ = on;
-  const int classify_launches = (on && opt_.learned_mlp == PLIS_MLP_TCGEN05) ? 2 : 1;
-  kernels_per_step_ = ((opt_.mode == PLIS_MODE_REFERENCE) ? 4 : 3) + classify_launches - 1;
+  kernels_per_step_ = ((opt_.mode == PLIS_MODE_REFERENCE) ? 3 : 2) + classify_kernels();
   drop_graphs();  // they hold the kernel arguments by value
   return state_set_ ? reclassify() : PLIS_OK;
 }
@@ -855,7 +864,7 @@ int Engine::slab_phase(int phase, double t_end, uint64_t n_steps) {
   switch (phase) {
     case PLIS_SLAB_CLASSIFY:
       launch_classify(args_);
-      launches_ += 1;
+      launches_ += classify_kernels();
       break;
     case PLIS_SLAB_CONTROL:
       k_slab_control<<<1, 32, 0, stream_>>>(args_);

@@ -73,6 +73,7 @@ class Engine {
   template <typename T> int upload(const std::vector<T>& v, const T** out);
   void enqueue_step(const NetArgs& a, bool lean);
   void launch_classify(const NetArgs& a);
+  int classify_kernels() const;
   int build_graph(bool lean);
   void drop_graphs();
   int advance_steps();

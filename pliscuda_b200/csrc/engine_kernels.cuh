@@ -739,7 +739,7 @@ __device__ void classify_cell(const KArgs& A, uint32_t c, const Nbr& q, const Co
 }
 
 // ------------------------------------------------------------------------------------------------
-// control (runs in one thread of the last CTA of k_classify, or in k_prepare)
+// control (runs in one thread of k_control, of the last CTA of k_classify, or in k_prepare)
 // ------------------------------------------------------------------------------------------------
 // Both work on a copy of the control block: loaded and stored whole, its fields cost one round trip to
 // L2 instead of one each.
@@ -1815,8 +1815,8 @@ __device__ __forceinline__ void classify_tile_net(const KArgs& A, const NetTab<R
 // CTA reduction into slot `slot` of its threads' min tau with arg-min (key, ti), with PLAIN the min of
 // their plain taus tp, #LEAP_CR, #SSA_FF and negative flags, then the count of finished CTAs; true in
 // the CTA that finished last of `nslots`.  Two CTA barriers: after the warps' partial results, and for
-// the verdict.
-template <bool PLAIN>
+// the verdict.  TICKET false: no count and no verdict, k_control follows.
+template <bool PLAIN, bool TICKET = true>
 __device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t slot, uint32_t nslots, uint64_t key,
                                               uint32_t ti, double tp, uint32_t ncr, uint32_t nff, int bad) {
   __shared__ uint64_t s_k[32];
@@ -1856,11 +1856,14 @@ __device__ __forceinline__ bool classify_slot(const KArgs& A, Ctrl* K, uint32_t 
       q.nff = nff;
       q.bad = cbad ? 1u : 0u;
       A.b.slot[slot] = q;
-      __threadfence();
-      const uint32_t prev = atomicAdd(&K->blocks_done, 1u);
-      s_last = ((prev & 0x7FFFFFFFu) == nslots - 1);
+      if constexpr (TICKET) {
+        __threadfence();
+        const uint32_t prev = atomicAdd(&K->blocks_done, 1u);
+        s_last = ((prev & 0x7FFFFFFFu) == nslots - 1);
+      }
     }
   }
+  if constexpr (!TICKET) return false;
   __syncthreads();
   return s_last;
 }
@@ -1937,7 +1940,7 @@ __device__ __forceinline__ void step_decide(const KArgs& A, Ctrl* K, uint32_t ph
   *K = k;
 }
 
-// The whole last CTA: reduce the `nslots` slots (independent L2 loads spread over the block), then
+// A whole CTA (the last of k_classify, or k_control's): reduce the `nslots` slots (independent L2 loads spread over the block), then
 // one thread takes the step decision (driver.cu:267-334): rollback or accept, time, the next plan.
 __device__ __forceinline__ void classify_control(const KArgs& A, Ctrl* K, uint32_t nslots) {
   __shared__ uint64_t s_k[32];
@@ -2015,8 +2018,8 @@ __global__ void __launch_bounds__(256, PLIS_CLASSIFY_MIN_BLOCKS) k_classify_smal
   int fl, bad;
   bool valid;
   classify_tile_small<Real, MAXS, LAT>(A, A.sm, blockIdx.x, C, tn, ti, fl, bad, valid);
-  if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
-    classify_control(A, K, gridDim.x);
+  classify_slot<false, false>(A, K, blockIdx.x, gridDim.x, tau_key(tn), ti, 0.0, valid && fl == F_LEAP_CR,
+                              valid && fl == F_SSA_FF, bad);
 }
 
 template <typename Real, bool LAT, bool COMP>
@@ -2033,8 +2036,8 @@ __global__ void __launch_bounds__(256, NetCtas<Real>::n) k_classify_net(const __
   int fl, bad;
   bool valid;
   classify_tile_net<Real, LAT, COMP>(A, net_tab<Real>(A), blockIdx.x, C, s_net, tn, ti, fl, bad, valid);
-  if (classify_slot<false>(A, K, blockIdx.x, gridDim.x, tn, ti, 0.0, valid && fl == F_LEAP_CR, bad, valid && fl == F_SSA_FF))
-    classify_control(A, K, gridDim.x);
+  classify_slot<false, false>(A, K, blockIdx.x, gridDim.x, tau_key(tn), ti, 0.0, valid && fl == F_LEAP_CR,
+                              valid && fl == F_SSA_FF, bad);
 }
 
 template <typename Real, int MAXS, bool CACHE>
@@ -2334,6 +2337,19 @@ __global__ void __launch_bounds__(256, kStepsCtas) k_steps(const __grid_constant
     *A.b.ctrl = s_k;
   }
 }
+
+#ifdef PLIS_ENGINE_HOST_TU
+// The step decision after k_classify_small / k_classify_net, from the records of their CTAs.  A ticket per CTA
+// and a last CTA that decides cost every CTA of a full wave a fence and an atomic round trip at its end
+// during which its place on the SM does no work; as a kernel of its own, launched before the classification
+// ends, the decision takes Schlogl 64^3 from 29.6 to 28.9 us a step, 67x45x53 in binary32 from 22.6 to 20.9,
+// a network at 64^3 from 124.3 to 121.9 and at 128^3 from 842 to 826.
+__global__ void __launch_bounds__(512) k_control(const __grid_constant__ KArgs A, uint32_t nslots) {
+  pdl_entry();
+  if (step_idle(A, A.b.ctrl)) return;
+  classify_control(A, A.b.ctrl, nslots);
+}
+#endif
 
 #ifdef PLIS_ENGINE_HOST_TU
 // ------------------------------------------------------------------------------------------------
