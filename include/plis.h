@@ -103,7 +103,8 @@ typedef struct plis_options {
   int32_t device;             /* CUDA device ordinal, default 0 */
   int32_t max_rollbacks;      /* per step before PLIS_ERR_STUCK, default 64 */
   int32_t steps_per_launch;   /* steps captured per CUDA-graph launch, 0 = auto */
-  int32_t tile[3];            /* lattice brick per CTA (x, y, z), 0 = auto */
+  int32_t tile[3];            /* lattice brick per CTA (x, y, z); all 0 = auto: bricks, or runs of 256 consecutive
+                               * subvolumes where bricks would leave many threads without one */
   int32_t persistent;         /* reserved, ignored by plis_create: a handle's step is always the graph of phase
                                * kernels; the persistent cooperative launch is the batched form (plis_batch_*,
                                * one replica or many) */
@@ -327,7 +328,8 @@ typedef struct plis_batch_desc {
 } plis_batch_desc;
 
 typedef struct plis_batch_tuning {
-  int32_t tile[3];            /* brick shape of the bricks CTAs take from the work queue */
+  int32_t tile[3];            /* brick shape of the bricks CTAs take from the work queue (with the default
+                               * 8 x 8 x 4, replicas that bricks fit badly are cut into runs of 256 instead) */
   int32_t blocks_per_sm;      /* co-resident CTAs per SM of the persistent launch */
   int32_t grid;               /* CTAs of the persistent launch */
   double events_per_s;        /* measured by plis_batch_autotune (0 if not tuned) */

@@ -300,6 +300,7 @@ int BatchEngine::layout(const int tile[3]) {
     }
   }
   std::vector<RepDesc> rep(nrep_);
+  std::vector<Geo> geo(nrep_);
   uint64_t toff = 0;
   for (uint32_t r = 0; r < nrep_; ++r) {
     RepDesc& q = rep[r];
@@ -310,6 +311,14 @@ int BatchEngine::layout(const int tile[3]) {
     q.ntiles = q.ntx * q.nty * q.ntz;
     q.tile_off = (uint32_t)toff;
     q.replica_id = ids_[r];
+    Geo& g = geo[r];
+    g = geo_;
+    g.ntx = q.ntx; g.nty = q.nty; g.ntz = q.ntz;
+    g.nblocks = q.ntiles;
+    geo_divisors(g);
+    // the default brick only: another one is the caller's or the tuner's choice
+    if (!geo_.staged && tx == 8 && ty == 8 && tz == 4) geo_rows(g, q.X, q.Y, q.Z, 0, false);
+    q.ntiles = g.nblocks;
     toff += q.ntiles;
   }
   if (toff >= (1ull << 31)) { err_ = "too many bricks"; return PLIS_ERR_LIMIT; }
@@ -332,10 +341,7 @@ int BatchEngine::layout(const int tile[3]) {
     v.o = dopt_;
     v.o.replica = ids_[r];
     devopts_keys(v.o);
-    v.g = geo_;
-    v.g.ntx = rep[r].ntx; v.g.nty = rep[r].nty; v.g.ntz = rep[r].ntz;
-    geo_divisors(v.g);
-    v.g.nblocks = rep[r].ntiles;
+    v.g = geo[r];
     for (int i = 0; i < 3; ++i) v.b.X[i] = d_X_[i] + coff_[r];
     for (int i = 0; i < 2; ++i) {
       v.b.tau[i] = d_tau_[i] + coff_[r];

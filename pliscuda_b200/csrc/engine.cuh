@@ -162,7 +162,8 @@ struct Geo {
   uint32_t threads;        // threads per CTA
   uint32_t staged;         // 1: the leap stages the brick + halo in shared memory
   uint32_t box_bytes;      // dynamic shared memory of the staged leap
-  FastDiv dtx, dty, dntx, dnty;  // divisions by tx, ty, ntx, nty (geo_divisors)
+  uint32_t rows;           // 1: no bricks, a CTA takes 256 consecutive subvolumes (geo_rows)
+  FastDiv dtx, dty, dntx, dnty;  // divisions by tx, ty, ntx, nty (geo_divisors); with rows dntx, dnty: by X, Y
 };
 // Sets the divisors of g from its tx, ty, ntx, nty.
 inline void geo_divisors(Geo& g) {
@@ -170,6 +171,31 @@ inline void geo_divisors(Geo& g) {
   g.dty = fastdiv_make(g.ty ? g.ty : 1);
   g.dntx = fastdiv_make(g.ntx ? g.ntx : 1);
   g.dnty = fastdiv_make(g.nty ? g.nty : 1);
+}
+// Cuts the X x Y x Z lattice of g into runs of 256 consecutive subvolumes instead of its bricks where that is
+// the better cut (call after geo_divisors; g keeps the brick's sides for geo_bricks).  Bricks share more of
+// their neighbours' lines, but lanes beyond the lattice idle; every lane of a run has a subvolume, and a run's
+// loads and atomics are whole lines.  Measured, us per step, bricks -> runs:
+//   more than 1/16 of the bricks' lanes beyond the lattice: Schlogl 100^3 89.6 -> 85.1, 101^3 in binary32 77.2 -> 71.4,
+//     42^3 19.4 -> 14.6, 20^3 10.64 -> 10.18, a network on 50x61x47 98.3 -> 88.0; 256 Brusselators of side 8..48
+//     in a batch 1386 -> 1153 a round (24 % of the bricks' lanes idle), 4200 -> 3492 with learned proposals.  Not below `least` subvolumes: few CTAs
+//     are latency, which more and emptier ones hide (A/B 10^3: 10.15 -> 10.26 with 4 runs for 12 bricks).
+//   nothing beyond the lattice, runs of whole x rows or parts of one (`whole`: small models in phase kernels):
+//     64^3 30.8 -> 28.9, 128x128x16 30.4 -> 28.3, 256x16x64 30.5 -> 28.2, 128^3 164.9 -> 162.6.  Runs that break
+//     rows lose (96^3 76.2 -> 77.1, 112^3 114 -> 116), as do networks (128^3 826 -> 841) and 16^3 batches (63.4 -> 63.8).
+inline void geo_rows(Geo& g, uint32_t X, uint32_t Y, uint32_t Z, uint64_t least, bool whole) {
+  const uint64_t n = (uint64_t)X * Y * Z;
+  const bool padded = (uint64_t)g.nblocks * 256 * 16 > n * 17;
+  if (g.threads != 256 || n < least || !(padded || (whole && (256 % X == 0 || X % 256 == 0)))) return;
+  g.rows = 1;
+  g.nblocks = (uint32_t)((n + 255) / 256);
+  g.dntx = fastdiv_make(X);
+  g.dnty = fastdiv_make(Y);
+}
+inline void geo_bricks(Geo& g) {  // undoes geo_rows
+  g.rows = 0;
+  g.nblocks = g.ntx * g.nty * g.ntz;
+  geo_divisors(g);
 }
 
 // The tables of a small model (at most kSmallR reactions and kSmallS species, one set of rate

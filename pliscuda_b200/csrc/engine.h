@@ -101,6 +101,7 @@ class Engine {
   unsigned* d_bar_ = nullptr;
   void* d_steps_slot_ = nullptr;
   int kernels_per_step_ = 4;
+  bool rows_ = false;  // runs of subvolumes instead of bricks (geo_rows), but for slabs and learned classification
   uint64_t launches_ = 0;
   double device_ms_ = 0.0;
   plis_profile prof_{};

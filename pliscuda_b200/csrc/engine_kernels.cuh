@@ -314,6 +314,15 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
 }
 
 __device__ __forceinline__ bool cell_of(const KArgs& A, uint32_t block, Cell& cl) {
+  if (A.g.rows) {
+    cl.c = block * 256u + threadIdx.x;
+    if (cl.c >= A.m.N) return false;
+    const uint32_t r = fdiv(cl.c, A.g.dntx);
+    cl.x = cl.c - r * A.m.X;
+    cl.z = fdiv(r, A.g.dnty);
+    cl.y = r - cl.z * A.m.Y;
+    return true;
+  }
   if (A.m.lattice) {
     const uint32_t b = block + A.sl.brick0, t = threadIdx.x;  // brick0: first brick of a z-slab (0 otherwise)
     if (t >= A.g.tx * A.g.ty * A.g.tz) return false;  // block rounded up to whole warps
