@@ -64,16 +64,16 @@ def _peaks():
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the committed
-# ncu capture of the same kernel on the same workload (profiles/k_leap_schlogl64.md: 2.44 MB read,
-# 0.02 MB written per launch under ncu's cache flush).  Keyed by (workload, semantics, precision, kernel); absent
+# ncu capture of the same kernel on the same workload (profiles/k_leap_schlogl64.md: 2.43 MB read,
+# 4 KB written per launch under ncu's cache flush).  Keyed by (workload, semantics, precision, kernel); absent
 # keys report null.
-NCU_TRAFFIC = {("schlogl64", "reference", "fp64", "leap"): (2.437120e6 + 0.010752e6, "profiles/k_leap_schlogl64.md")}
+NCU_TRAFFIC = {("schlogl64", "reference", "fp64", "leap"): (2.426368e6 + 4.096e3, "profiles/k_leap_schlogl64.md")}
 # smsp__inst_executed.sum per launch (warp instructions) of the same capture.  The kernel is bound by
 # instruction issue and dependent latency, not by DRAM, so the line also reports the achieved warp-
 # instruction rate against the issue peak (148 SMs x 4 schedulers x the SM clock sampled during the
-# timed region).  The count is that of step 41 from the initial state; later steps of the bench
+# timed region).  The count is that of an early step from the initial state; later steps of the bench
 # trajectory draw from similar Poisson means, so the rate is an estimate.
-NCU_WARP_INSTR = {("schlogl64", "reference", "fp64", "leap"): (17.785662e6, "profiles/k_leap_schlogl64.md")}
+NCU_WARP_INSTR = {("schlogl64", "reference", "fp64", "leap"): (11.100745e6, "profiles/k_leap_schlogl64.md")}
 SM_COUNT, SCHEDULERS_PER_SM = 148, 4
 
 def issue_roofline(instr, ms_launch, clocks):
@@ -242,7 +242,7 @@ def cpu_baseline_sample(workload, threads, mode=0, precision=0, budget_s=12.0):
 
 def ncu_case(args):
     """Fixed small case for ncu captures: the bench workload, 40 leap steps of warm-up, then 3
-    profiled ones (capture with -k regex:k_leap -s 40 -c 3, or the classify kernel likewise)."""
+    profiled ones (capture with -k regex:k_leap_small -s 40 -c 3, or k_classify_small likewise)."""
     from pliscuda_b200 import Simulation
     model, state = _workload(args.workload)
     with Simulation(model, mode=args.mode, precision=args.precision, seed=1000) as sim:
@@ -256,7 +256,7 @@ def ncu_case(args):
 
 def ncu_network_case(args):
     """Fixed small case for ncu captures of the random network (10 species, 20 reactions, the precision
-    configuration's network) on a 64^3 lattice: 10 + 3 steps (capture with -k regex:"^k_leap$" -s 10 -c 1,
+    configuration's network) on a 64^3 lattice: 10 + 3 steps (capture with -k regex:"^k_leap_net$" -s 10 -c 1,
     or the classification likewise).  64^3 keeps the device memory to a few tens of MB while the
     counts (10.5 MB per buffer) still exceed what the L1s hold."""
     from pliscuda_b200 import Simulation, workloads
@@ -272,7 +272,7 @@ def ncu_network_case(args):
 def ncu_learned_case(args):
     """Fixed small case for ncu captures of the learned step: a proposer trained briefly on 10 plain
     corrected steps of the workload (clamp 16), then 10 + 3 learned steps (plain launches).  Filter
-    the capture to the step's kernels, e.g. -k regex:"k_leap|k_exact|k_learned|k_mlp"."""
+    the capture to the step's kernels, e.g. -k regex:"k_leap|k_exact|k_learned"."""
     from pliscuda_b200 import Simulation
     from pliscuda_b200.learned import train_proposer
     model, state = _workload(args.workload)

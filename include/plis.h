@@ -105,15 +105,15 @@ typedef struct plis_options {
   int32_t steps_per_launch;   /* steps captured per CUDA-graph launch, 0 = auto */
   int32_t tile[3];            /* lattice brick per CTA (x, y, z); all 0 = auto: bricks, or runs of 256 consecutive
                                * subvolumes where bricks would leave many threads without one */
-  int32_t persistent;         /* reserved, ignored by plis_create: a handle's step is always the graph of phase
-                               * kernels; the persistent cooperative launch is the batched form (plis_batch_*,
-                               * one replica or many) */
+  int32_t persistent;         /* reserved, ignored by plis_create: three steps or more of a system small enough to
+                               * stay on the SMs (two CTAs each) run in one persistent cooperative launch, all
+                               * others as the graph of phase kernels, with the same results */
   int32_t profile;            /* 1 = launch phase kernels one by one with CUDA events around each (plis_get_profile) */
   int32_t stage_halo;         /* lattice leap: 1 = stage brick + halo in shared memory, 0 = global atomics (default) */
   int32_t learned_mlp;        /* learned tau MLP: 0 = tcgen05.mma with TMEM accumulators (default), 1 = mma.sync */
   uint64_t wait_polls;        /* polls after which a device-side wait gives up with PLIS_ERR_TIMEOUT: the grid
                                * barrier of the persistent batched kernel (>= 32 ns per poll) and the mbarrier
-                               * waits of the tcgen05 MLP; 0 = defaults (2^26 and 2^22 polls).  The reference
+                               * waits of the tcgen05 MLP (a handle with a limit keeps to the phase kernels); 0 = defaults (2^26 and 2^22 polls).  The reference
                                * has no device waits (its host loop synchronises, driver.cu:259-376). */
   int32_t pooled_draws;       /* leap: 1 = channels of small mean (below 1/8) drawn as one pooled Poisson total
                                * split over them, 0 = one draw per channel, -1 = auto (default: pooled for
