@@ -14,8 +14,9 @@
 // Every floating-point value is formed by the same operations in the same order as in the generic
 // phases, which larger networks keep.
 // Measured on one B200 against the generic phases (us a step): 10 species and 20 reactions on 128^3 in
-// binary64 2130 -> 1150 (leap 767 -> 440, exact events 168 -> 122, classification 1053 -> 572), on
-// 64^3 in binary32 279 -> 161; a cell of 9,300 subvolumes as a table with two compartments 71.6 -> 44.
+// binary64 2130 -> 826 (leap 767 -> 331, exact events 168 -> 62, classification 1053 -> 417), on
+// 64^3 in binary32 279 -> 121; a cell of 9,300 subvolumes as a table with two compartments 71.6 -> 27.4
+// (there in the persistent kernel, k_steps).
 #ifndef PLIS_NET_STEP_CUH_
 #define PLIS_NET_STEP_CUH_
 

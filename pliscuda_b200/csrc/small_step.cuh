@@ -5,10 +5,10 @@
 // 1 MB per species and sit in L2), so this file spends as few instructions per subvolume as it can
 // while every floating-point result keeps the bits of the generic phases (engine_kernels.cuh).
 // Measured on one B200, Schlogl 64^3 in binary64, against the generic loops over byte tables: the
-// leap went from 17.8 M to 11.3 M warp instructions and from 31.6 to 21.2 us a launch, the
-// classification from 10.7 M to 5.5 M and from 29.2 to 16.7 us (both cold), the step from 51.3 to
-// 32 us; 1,000 subvolumes (A/B network) 30.8 to 18.6 us a step; 256 Brusselator replicas 2.7 to
-// 1.5 ms a round.
+// leap went from 17.8 M to 11.1 M warp instructions and from 31.6 to 19.8 us a launch, the
+// classification from 10.7 M to 5.6 M and from 29.2 to 13.2 us (both cold), the step from 51.3 to
+// 27.2 us; 1,000 subvolumes (A/B network) 30.8 to 10.2 us a step (in k_steps); 256 Brusselator
+// replicas 2.7 to 1.15 ms a round.
 //   * the tables are whole words at compile-time offsets (constant-bank operands: no byte loads);
 //     criticality is one compare per reactant species against a threshold made at set-up;
 //   * the inversion searches count the CDF terms a uniform exceeds (u > F_0, u > F_1, ...) instead of
