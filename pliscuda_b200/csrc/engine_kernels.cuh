@@ -15,8 +15,9 @@
 //   k_classify  negativity check (check_state, leap.cu:203-212), rates, criticality, Cao tau,
 //               tau_cr, flags and fast-forward (rates.cu, tau.cu:197-252) of the post-step state,
 //               a warp-shuffle + CTA min-tau with arg-min, and in the last CTA to finish (small and
-//               network models: in k_control): the grid-wide arg-min, rollback-or-accept, the time update and the next step's plan
-//               (driver.cu:267-334).  It also zeroes the buffer the next leap will reduce into.
+//               network models: in k_control): the grid-wide arg-min, rollback-or-accept, the time
+//               update and the next step's plan (driver.cu:267-334).  It also zeroes the buffer the
+//               next leap will reduce into.
 //
 // Counts are int32 species-major [S][Npad] in three rotating buffers (current, target, spare), so
 // accepting a step is an index rotation and a rollback discards the target: no device-to-device
