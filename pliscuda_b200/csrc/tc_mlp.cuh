@@ -20,7 +20,10 @@
 //
 // Synchronisation.  One thread of a group issues the MMAs and commits them to the group's mbarrier;
 // every thread of the group waits on it with an iteration limit, and one named barrier per layer
-// joins the group.  A wait that runs out stops the group with a status; TMEM is always freed.  A CTA
+// joins the group.  That barrier also reduces the threads' verdicts on their wait, so that a wait that
+// runs out in any of them stops the whole group after the same layer (a flag in shared memory would
+// not do: a thread that is through the barrier could set it for the next layer before another has read
+// it for this one, and the two would part).  The status is set then; TMEM is always freed.  A CTA
 // allocates 256 TMEM columns and its shared memory keeps at most two on an SM: allocation never has
 // to wait.
 #ifndef PLIS_TC_MLP_CUH_
@@ -112,13 +115,10 @@ __device__ __forceinline__ uint32_t canon(uint32_t row, uint32_t k, uint32_t chu
   return (k >> 3) * chunk + (row >> 3) * 128u + (row & 7u) * 16u + (k & 7u) * 2u;
 }
 
-// wait for the mbarrier phase `parity`; false (and *err set) when the limit ran out
-__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volatile int* err, uint32_t limit) {
-  for (uint32_t i = 0; i < limit; ++i) {
+// wait for the mbarrier phase `parity`; false when the limit ran out
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, uint32_t limit) {
+  for (uint32_t i = 0; i < limit; ++i)
     if (try_wait(bar, parity)) return true;
-    if (*err) return false;
-  }
-  *err = 1;
   return false;
 }
 
@@ -145,6 +145,17 @@ constexpr uint32_t kPTmemCols = kGroups * 64;
 static_assert(kPSmemBytes * 3 > 228 * 1024 && kPTmemCols * 2 <= 512, "two CTAs per SM, and TMEM for both");
 
 __device__ __forceinline__ void group_sync(uint32_t group) { asm volatile("bar.sync %0, 128;" ::"r"(group + 1u) : "memory"); }
+// the same barrier; true in all 128 threads when `v` is true in any of them
+__device__ __forceinline__ bool group_any(uint32_t group, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\tbar.red.or.pred q, %1, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(group + 1u), "r"(v ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
 
 // The MLP on tcgen05 for the rows of `feats` (normalised BF16 features, 16 bytes per row, rows
 // 0 .. 128 * ntiles - 1 readable), tiles taken round robin by the groups of the grid.
@@ -154,7 +165,6 @@ template <class Sink>
 static __device__ __forceinline__ void mlp_tiles(const Params& P, const uint4* __restrict__ feats, uint32_t ntiles,
                                                  uint8_t* smem, int* status, uint32_t wait_limit, Sink& sink) {
   if (wait_limit == 0) wait_limit = kWaitLimit;
-  __shared__ int s_err[kGroups];
   const uint32_t tid = threadIdx.x;  // blockDim.x == kThreads
   const uint32_t group = tid >> 7, t = tid & 127u;
   const uint32_t sbase = smem_u32(smem);
@@ -171,10 +181,7 @@ static __device__ __forceinline__ void mlp_tiles(const Params& P, const uint4* _
       vec[128 + tid] = __ldg(&P.b3[tid]);
       vec[192 + tid] = __ldg(&P.w4[tid]);
     }
-    if (t == 0) {
-      s_err[group] = 0;
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    }
+    if (t == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
     if (tid < 32) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
                    "r"(kPTmemCols)
@@ -191,7 +198,6 @@ static __device__ __forceinline__ void mlp_tiles(const Params& P, const uint4* _
   uint8_t* a1 = smem + kPOffA1 + 2048u * group;
   uint8_t* a = smem + kPOffA + kABytes * group;
   const uint32_t sa1 = sbase + kPOffA1 + 2048u * group, sa = sbase + kPOffA + kABytes * group;
-  volatile int* err = &s_err[group];
   uint32_t phase = 0;
   const uint32_t first = blockIdx.x * kGroups + group, step = gridDim.x * kGroups;
   uint4 next = first < ntiles ? feats[first * 128u + t] : make_uint4(0u, 0u, 0u, 0u);
@@ -219,7 +225,7 @@ static __device__ __forceinline__ void mlp_tiles(const Params& P, const uint4* _
         }
         commit(bar);
       }
-      const bool got = wait_phase(bar, phase & 1u, err, wait_limit);
+      const bool got = wait_phase(bar, phase & 1u, wait_limit);
       phase += 1;
       fence_after();
       __syncwarp();
@@ -258,29 +264,23 @@ static __device__ __forceinline__ void mlp_tiles(const Params& P, const uint4* _
           }
           out = out + P.b4;
         }
-      } else {
-        *err = 1;
       }
       fence_before();
       fence_async_smem();
-      group_sync(group);
-      if (*err) {  // the same for the whole group: only its own threads set it, before the barrier
+      if (group_any(group, !got)) {
         ok = false;
         break;
       }
     }
     if (ok) sink.end(row, out);
   }
-  if (!ok) {  // the MMAs in flight finish before their TMEM is freed
-    int late = 0;
-    wait_phase(bar, (phase - 1u) & 1u, &late, kWaitLimit);
-  }
+  if (!ok) wait_phase(bar, (phase - 1u) & 1u, kWaitLimit);  // the MMAs in flight finish before their TMEM is freed
   fence_before();
   __syncthreads();
   fence_after();
   if (tid < 32)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*slot), "r"(kPTmemCols) : "memory");
-  if (t == 0 && s_err[group]) atomicExch(status, 6 /* PLIS_ERR_TIMEOUT */);
+  if (t == 0 && !ok) atomicExch(status, 6 /* PLIS_ERR_TIMEOUT */);
 }
 
 }  // namespace tc
