@@ -823,7 +823,8 @@ int Engine::slab_setup(uint32_t z0, uint32_t z1, uint32_t world, uint32_t rank) 
   L.has_hi = z1 < dm.Z ? 1u : 0u;
   L.world = world;
   L.rank = rank;
-  if (g.rows) geo_bricks(g);  // a slab is whole bricks
+  if (rows_) geo_bricks(g);  // a slab is whole bricks, and stays so when a proposer is detached
+  rows_ = false;
   L.brick0 = (z0 / g.tz) * g.ntx * g.nty;
   slab_blocks_ = ((z1 - z0 + g.tz - 1) / g.tz) * g.ntx * g.nty;
   slab_stage_ = (size_t)(dm.S + 1) * L.layer;
