@@ -564,6 +564,7 @@ int Engine::set_proposer(const float* weights, double s_max) {
       PLIS_CU(cudaMemset(d_feat_, 0, rows * sizeof(uint4)));
       if ((rc = dmalloc((void**)&d_pre_, (size_t)args_.m.Npad * sizeof(double2)))) return rc;
       if ((rc = dmalloc((void**)&d_pre_kind_, (size_t)args_.m.Npad))) return rc;
+      PLIS_CU(cudaMemset(d_pre_kind_, 0, (size_t)args_.m.Npad));  // a slab writes its own subvolumes only: 0 is no subvolume
     }
     PLIS_CU(cudaMemcpyAsync(d_lw_, weights, PLIS_PROPOSER_WEIGHTS * sizeof(float), cudaMemcpyHostToDevice, stream_));
     learned_pack(d_lw_, s_max, d_lp_, stream_);
