@@ -205,6 +205,17 @@ static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* 
   return true;
 }
 
+// False for a neighbour table with a row that lists a subvolume without neighbours of its own (a one-way
+// edge into a sink).  Reference semantics divide that one's jumps by its neighbour count, 0: inf or NaN, which
+// the generic phases' division gives and div_small (small and network models) does not.
+static bool neighbours_have_neighbours(const Topology& t) {
+  if (t.is_lattice()) return true;
+  for (uint32_t c = 0; c < t.n; ++c)
+    for (uint32_t j = 0; j < t.ncount[c]; ++j)
+      if (t.ncount[t.canon[(size_t)c * 6 + j]] == 0) return false;
+  return true;
+}
+
 int Engine::create(const Model& model, const plis_options& opt) {
   model_ = model;
   opt_ = opt;
@@ -271,8 +282,9 @@ int Engine::create(const Model& model, const plis_options& opt) {
     dm.dr = p;
   }
 
-  // a small model's tables in the kernel arguments (SmallModel)
-  fill_small_model(M, M.comp.empty() ? M.rrate.data() : nullptr, M.drate.data(), opt, &args_.sm);
+  // a small model's tables in the kernel arguments (SmallModel), or below those of a network (NetTab)
+  const bool divisible = opt.mode != PLIS_MODE_REFERENCE || neighbours_have_neighbours(M.topo);
+  if (divisible) fill_small_model(M, M.comp.empty() ? M.rrate.data() : nullptr, M.drate.data(), opt, &args_.sm);
 
   // geometry
   Geo& g = args_.g;
@@ -354,7 +366,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
   if (o.pool || opt.stage_halo) args_.sm.on = 0;  // pooled draws and the staged box live in the generic leap only
 
   launch_ = (opt.precision == PLIS_PREC_FP32) ? pick_f32(M.S) : pick_f64(M.S);
-  if (!args_.sm.on && !opt.stage_halo) {
+  if (!args_.sm.on && !opt.stage_halo && divisible) {
     o.net = opt.precision == PLIS_PREC_FP32 ? fill_net_tab(M, opt, &args_.net.f) : fill_net_tab(M, opt, &args_.net.d);
     if (o.net) PLIS_CU(launch_.net_smem());
   }
