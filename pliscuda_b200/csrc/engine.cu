@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -89,10 +90,16 @@ int Engine::upload(const std::vector<T>& v, const T** out) {
   return PLIS_OK;
 }
 
+// A rate constant beyond binary32 gives inf x 0 = NaN for a reaction without reactants.  Corrected semantics
+// leave out what is not positive, but the critical bits of the small and network kernels (small_rates,
+// net_prop) let a NaN through: such models take the generic phases.
+static bool rate_in_range(double rate, bool f32) { return !f32 || std::isfinite((float)rate); }
+
 // The SmallModel block of a model that fits it; sm->on = 0 otherwise.  It fits with at most kSmallR
 // reactions and kSmallS species, net changes within int8 (32-bit sums of the leap), one set of rate
-// constants (rrate[R] and drate[S]; rrate null = several sets), and jump rates that are zero or far
-// from the ends of the working precision's range (the neighbour terms' division, div_small).
+// constants (rrate[R] and drate[S]; rrate null = several sets), jump rates that are zero or far
+// from the ends of the working precision's range (the neighbour terms' division, div_small), and rates
+// that are finite in it.
 bool fill_small_model(const Model& M, const double* rrate, const double* drate, const plis_options& opt, SmallModel* out) {
   SmallModel& sm = *out;
   std::memset(&sm, 0, sizeof sm);
@@ -106,6 +113,7 @@ bool fill_small_model(const Model& M, const double* rrate, const double* drate, 
   const bool f32 = opt.precision == PLIS_PREC_FP32;
   const double lo = f32 ? 1e-25 : 1e-250, hi = f32 ? 1e25 : 1e250;
   for (size_t s = 0; fits && s < M.S; ++s) fits = drate[s] == 0.0 || (drate[s] >= lo && drate[s] <= hi);
+  for (size_t r = 0; fits && r < M.R; ++r) fits = rate_in_range(rrate[r], f32);
   if (!fits) return false;
   for (int r = 0; r < kSmallR; ++r)
     for (int s = 0; s < kSmallS; ++s) sm.thr[r][s] = INT32_MIN;
@@ -141,8 +149,8 @@ bool fill_small_model(const Model& M, const double* rrate, const double* drate, 
   return true;
 }
 
-// NetTab of a model that fits it, false otherwise: sizes, thresholds exact in binary32, jump rates as
-// for a small model, compartments in five bits.
+// NetTab of a model that fits it, false otherwise: sizes, thresholds exact in binary32, jump rates and rates
+// as for a small model, compartments in five bits.
 template <typename Real>
 static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* out) {
   const ReactionTables& t = M.rt;
@@ -152,6 +160,8 @@ static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* 
   const double lo = sizeof(Real) == 4 ? 1e-25 : 1e-250, hi = sizeof(Real) == 4 ? 1e25 : 1e250;
   for (double d : M.drate)
     if (d != 0.0 && !(d >= lo && d <= hi)) return false;
+  for (double d : M.rrate)
+    if (!rate_in_range(d, sizeof(Real) == 4)) return false;
   NetTab<Real>& n = *out;
   std::memset(&n, 0, sizeof n);
   uint32_t e = 0;
