@@ -157,6 +157,7 @@ static bool fill_net_tab(const Model& M, const plis_options& opt, NetTab<Real>* 
   if (M.R > (uint32_t)kNetR || M.S > (uint32_t)kNetS || M.C > 32u) return false;
   const int64_t nc = opt.critical_threshold, most = 1 << 24;
   if (nc > most || nc < -most || t.sp_r.size() > (size_t)kNetE) return false;
+  if (opt.epsilon > 1e9) return false;  // (epsilon x count)^2, counts below 2^30, within binary32: net_tau_near
   const double lo = sizeof(Real) == 4 ? 1e-25 : 1e-250, hi = sizeof(Real) == 4 ? 1e25 : 1e250;
   for (double d : M.drate)
     if (d != 0.0 && !(d >= lo && d <= hi)) return false;
