@@ -273,7 +273,7 @@ int BatchEngine::create(const plis_batch_desc& d, const plis_options& opt) {
   {
     uint32_t most = 0;
     for (uint32_t r = 0; r < nrep_; ++r) most = std::max(most, npad_[r]);
-    PLIS_CU(stage_.init(opt.device, (size_t)most * 4));
+    stage_.init(opt.device, (size_t)most * 4);
   }
   int tile[3] = {opt.tile[0], opt.tile[1], opt.tile[2]};
   if (tile[0] <= 0 || tile[1] <= 0 || tile[2] <= 0) { tile[0] = 8; tile[1] = 8; tile[2] = 4; }

@@ -347,7 +347,7 @@ int Engine::create(const Model& model, const plis_options& opt) {
 
   // buffers
   const size_t cells = (size_t)M.S * dm.Npad;
-  if (cells * 4 >= kStagedState) PLIS_CU(stage_.init(opt.device, cells * 4));
+  if (cells * 4 >= kStagedState) stage_.init(opt.device, cells * 4);
   DevBufs& b = args_.b;
   for (int i = 0; i < 3; ++i)
     if ((rc = dmalloc((void**)&b.X[i], cells * 4))) return rc;

@@ -5,7 +5,8 @@
 // bytes pass through pinned slices that belong to the handle (at most kSlices x 512 KB, freed with it):
 // large states with kWorkers threads, each alternating between its own slices so that its memcpy
 // overlaps its DMA (pages of a fresh result array are then touched by several threads too), small ones
-// by the caller, which need not wait for the device before it returns from an upload.
+// by the caller, which need not wait for the device before it returns from an upload.  The slices are an
+// optimisation: where they cannot be had, the copies go through the driver.
 #ifndef PLIS_HOST_STAGE_H_
 #define PLIS_HOST_STAGE_H_
 
@@ -68,15 +69,18 @@ class HostStage {
   ~HostStage() { release(); }
 
   // slices for pieces of up to `piece` bytes (a piece above 512 KB passes in parts)
-  cudaError_t init(int device, size_t piece) {
+  void init(int device, size_t piece) {
     device_ = device;
     slice_ = std::min<size_t>(size_t(512) << 10, (piece + 4095) / 4096 * 4096);
     if (slice_ == 0) slice_ = 4096;
     cudaError_t e = cudaMallocHost((void**)&buf_, slice_ * kSlices);
-    if (e != cudaSuccess) { buf_ = nullptr; return e; }
+    if (e != cudaSuccess) buf_ = nullptr;
     for (auto& v : ev_)
-      if ((e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) return e;
-    return cudaSuccess;
+      if (e == cudaSuccess && (e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming)) != cudaSuccess) v = nullptr;
+    if (e != cudaSuccess) {
+      release();
+      cudaGetLastError();  // not the error of a later launch
+    }
   }
   bool on() const { return buf_ != nullptr; }
   void release() {
@@ -93,9 +97,17 @@ class HostStage {
   // `rows` rows of `bytes` each; dpitch / hpitch: distance of two rows on the device / host.  An upload
   // returns with the host buffer free and the copies enqueued on s; a download returns with the data.
   cudaError_t upload(void* dev, size_t dpitch, const void* host, size_t hpitch, size_t bytes, size_t rows, cudaStream_t s) {
+    if (!on()) {
+      const cudaError_t e = cudaMemcpy2DAsync(dev, dpitch, host, hpitch, bytes, rows, cudaMemcpyHostToDevice, s);
+      return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+    }
     return copy(true, (char*)dev, dpitch, (char*)const_cast<void*>(host), hpitch, bytes, rows, s);
   }
   cudaError_t download(void* host, size_t hpitch, const void* dev, size_t dpitch, size_t bytes, size_t rows, cudaStream_t s) {
+    if (!on()) {
+      const cudaError_t e = cudaMemcpy2DAsync(host, hpitch, dev, dpitch, bytes, rows, cudaMemcpyDeviceToHost, s);
+      return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+    }
     return copy(false, (char*)const_cast<void*>(dev), dpitch, (char*)host, hpitch, bytes, rows, s);
   }
 
