@@ -91,7 +91,6 @@ class BatchEngine {
   int* d_err_ = nullptr;
   std::vector<Ctrl> h_ctrl_;
   bool ctrl_fresh_ = false;   // h_ctrl_ holds the device's control blocks (nothing has run since they were read)
-  HostStage stage_;           // transfers of the replicas' states
   double device_ms_ = 0.0;
   uint64_t launches_ = 0;
   bool learned_ = false;

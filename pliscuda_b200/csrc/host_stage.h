@@ -1,12 +1,11 @@
 // host_stage.h — copies between pageable host memory and the device through a handle's own pinned slices.
 //
 // A copy from pageable memory goes through the driver's staging on the calling thread, 4-5 GB/s on the
-// measured host for states of tens of megabytes, and a small one waits for the device.  Here the
-// bytes pass through pinned slices that belong to the handle (at most kSlices x 512 KB, freed with it):
-// large states with kWorkers threads, each alternating between its own slices so that its memcpy
-// overlaps its DMA (pages of a fresh result array are then touched by several threads too), small ones
-// by the caller, which need not wait for the device before it returns from an upload.  The slices are an
-// optimisation: where they cannot be had, the copies go through the driver.
+// measured host for states of tens of megabytes.  Here the bytes pass through pinned slices that belong
+// to the handle (kSlices x 512 KB, freed with it), with kWorkers threads, each alternating between its
+// own slices so that its memcpy overlaps its DMA (pages of a fresh result array are then touched by
+// several threads too).  The slices are an optimisation: where they cannot be had, the copies go through
+// the driver.
 #ifndef PLIS_HOST_STAGE_H_
 #define PLIS_HOST_STAGE_H_
 
@@ -20,15 +19,18 @@
 
 namespace plis {
 
-// true when the caller's buffer is pinned already: a plain asynchronous copy runs at DMA speed
-inline bool host_pinned(const void* p) {
+inline cudaMemoryType host_memory(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return cudaMemoryTypeUnregistered;
   }
-  return a.type == cudaMemoryTypeHost;
+  return a.type;
 }
+// true when the caller's buffer is pinned already: a plain asynchronous copy runs at DMA speed
+inline bool host_pinned(const void* p) { return host_memory(p) == cudaMemoryTypeHost; }
+// true for a buffer the CUDA runtime does not know
+inline bool host_pageable(const void* p) { return host_memory(p) == cudaMemoryTypeUnregistered; }
 
 // Runs f(0) .. f(n - 1), on threads of their own but for the first; inline where a thread cannot be had.
 template <class F>
@@ -114,11 +116,11 @@ class HostStage {
  private:
   cudaError_t copy(bool up, char* dev, size_t dp, char* host, size_t hp, size_t bytes, size_t rows, cudaStream_t s) {
     const size_t parts = (bytes + slice_ - 1) / slice_, n = parts * rows;
-    const int workers = n >= (size_t)kSlices ? kWorkers : 1, per = kSlices / workers;
+    constexpr int workers = kWorkers, per = kSlices / workers;
     cudaError_t err[kWorkers] = {};
     // worker w moves parts w, w + workers, ... through its slices w * per .. + per - 1 in turn
     auto run = [&](int w) {
-      cudaError_t e = workers > 1 ? cudaSetDevice(device_) : cudaSuccess;
+      cudaError_t e = cudaSetDevice(device_);
       size_t done = 0;  // downloads: parts of this worker taken out of its slices
       auto place = [&](size_t j, char*& d, char*& h, size_t& len) {
         const size_t i = w + j * workers, row = i / parts, off = i % parts * slice_;
@@ -141,7 +143,7 @@ class HostStage {
         size_t len;
         place(j, d, h, len);
         if (!up && j >= (size_t)per) take();
-        const int k = workers == 1 ? (int)(up ? next_++ % kSlices : j % per) : w * per + (int)(j % per);
+        const int k = w * per + (int)(j % per);
         char* b = buf_ + k * slice_;
         if (e == cudaSuccess) e = cudaEventSynchronize(ev_[k]);  // the slice's last copy
         if (e != cudaSuccess) break;
@@ -152,8 +154,7 @@ class HostStage {
       while (!up && done < j) take();
       err[w] = e;
     };
-    if (workers > 1) run_workers(workers, run);
-    else run(0);
+    run_workers(workers, run);
     for (cudaError_t e : err)
       if (e != cudaSuccess) return e;
     return cudaSuccess;
@@ -161,7 +162,6 @@ class HostStage {
 
   int device_ = 0;
   size_t slice_ = 0;
-  unsigned next_ = 0;
   char* buf_ = nullptr;
   cudaEvent_t ev_[kSlices] = {};
 };
