@@ -113,7 +113,8 @@ typedef struct plis_options {
   int32_t learned_mlp;        /* learned tau MLP: 0 = tcgen05.mma with TMEM accumulators (default), 1 = mma.sync */
   uint64_t wait_polls;        /* polls after which a device-side wait gives up with PLIS_ERR_TIMEOUT: the grid
                                * barrier of the persistent batched kernel (>= 32 ns per poll) and the mbarrier
-                               * waits of the tcgen05 MLP (a handle with a limit keeps to the phase kernels); 0 = defaults (2^26 and 2^22 polls).  The reference
+                               * waits of the tcgen05 MLP (a handle with a limit keeps to the phase kernels, whose
+                               * only waits are the MLP's); 0 = defaults (2^26 and 2^22 polls).  The reference
                                * has no device waits (its host loop synchronises, driver.cu:259-376). */
   int32_t pooled_draws;       /* leap: 1 = channels of small mean (below 1/8) drawn as one pooled Poisson total
                                * split over them, 0 = one draw per channel, -1 = auto (default: pooled for
@@ -328,8 +329,9 @@ typedef struct plis_batch_desc {
 } plis_batch_desc;
 
 typedef struct plis_batch_tuning {
-  int32_t tile[3];            /* brick shape of the bricks CTAs take from the work queue (with the default
-                               * 8 x 8 x 4, replicas that bricks fit badly are cut into runs of 256 instead) */
+  int32_t tile[3];            /* brick shape of the bricks CTAs take from the work queue (8 x 8 x 4 by default or
+                               * by the autotuner: replicas that bricks fit badly are cut into runs of 256
+                               * instead; options.tile of 8 x 8 x 4 keeps bricks) */
   int32_t blocks_per_sm;      /* co-resident CTAs per SM of the persistent launch */
   int32_t grid;               /* CTAs of the persistent launch */
   double events_per_s;        /* measured by plis_batch_autotune (0 if not tuned) */

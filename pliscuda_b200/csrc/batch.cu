@@ -270,17 +270,20 @@ int BatchEngine::create(const plis_batch_desc& d, const plis_options& opt) {
   pending_.assign(nrep_, 2);  // 2 = never given a state
   launch_ = (opt.precision == PLIS_PREC_FP32) ? batch_pick_f32(S_, false, small_) : batch_pick_f64(S_, false, small_);
   int tile[3] = {opt.tile[0], opt.tile[1], opt.tile[2]};
-  if (tile[0] <= 0 || tile[1] <= 0 || tile[2] <= 0) { tile[0] = 8; tile[1] = 8; tile[2] = 4; }
-  rc = layout(tile);
+  const bool given = tile[0] > 0 && tile[1] > 0 && tile[2] > 0;
+  if (!given) { tile[0] = 8; tile[1] = 8; tile[2] = 4; }
+  rc = layout(tile, !given);
   if (rc) return rc;
   PLIS_CU(cudaDeviceSynchronize());
   return PLIS_OK;
 }
 
-int BatchEngine::layout(const int tile[3]) {
+// runs: replicas that bricks fit badly are cut into runs (geo_rows); a brick that the caller gave is kept
+int BatchEngine::layout(const int tile[3], bool runs) {
   const uint32_t tx = (uint32_t)tile[0], ty = (uint32_t)tile[1], tz = (uint32_t)tile[2];
   if (tx * ty * tz < 1 || tx * ty * tz > 256) { err_ = "tile must hold 1..256 subvolumes"; return PLIS_ERR_INVALID; }
   tile_[0] = tx; tile_[1] = ty; tile_[2] = tz;
+  runs_ = runs;
   std::memset(&geo_, 0, sizeof geo_);
   geo_.tx = tx; geo_.ty = ty; geo_.tz = tz;
   geo_.threads = (tx * ty * tz + 31u) & ~31u;
@@ -310,8 +313,7 @@ int BatchEngine::layout(const int tile[3]) {
     g.ntx = q.ntx; g.nty = q.nty; g.ntz = q.ntz;
     g.nblocks = q.ntiles;
     geo_divisors(g);
-    // the default brick only: another one is the caller's or the tuner's choice
-    if (!geo_.staged && tx == 8 && ty == 8 && tz == 4) geo_rows(g, q.X, q.Y, q.Z, 0, false);
+    if (!geo_.staged && runs) geo_rows(g, q.X, q.Y, q.Z, 0, false);
     q.ntiles = g.nblocks;
     toff += q.ntiles;
   }
@@ -427,7 +429,7 @@ int BatchEngine::set_proposer(const float* weights, double s_max) {
   learned_ = on;
   launch_ = (opt_.precision == PLIS_PREC_FP32) ? batch_pick_f32(S_, on, small_) : batch_pick_f64(S_, on, small_);
   const int tile[3] = {(int)tile_[0], (int)tile_[1], (int)tile_[2]};
-  int rc = layout(tile);
+  int rc = layout(tile, runs_);
   if (rc) return rc;
   // classify every replica's current state again (time, step and statistics are kept)
   if ((rc = read_ctrls())) return rc;
@@ -624,12 +626,13 @@ int BatchEngine::autotune(uint64_t pilot_steps, plis_batch_tuning* out) {
     ctrl_fresh_ = false;
     for (int i = 0; i < 9; ++i) cudaMemcpy((void*)srcs[i], saved[i], sizes[i], cudaMemcpyDeviceToDevice);
   };
+  // the first one stands for the default cut, with runs where bricks fit badly
   const int cands[][3] = {{8, 8, 4}, {16, 4, 4}, {8, 4, 8}, {16, 8, 2}, {32, 4, 2}, {32, 8, 1}, {8, 8, 2}, {4, 8, 8}};
   double best = -1.0;
   int best_i = -1;
   const double ms0 = device_ms_;
   for (int i = 0; i < 8 && rc == PLIS_OK; ++i) {
-    rc = layout(cands[i]);
+    rc = layout(cands[i], i == 0);
     if (rc) break;
     restore();
     std::vector<Ctrl> before(nrep_);
@@ -643,7 +646,7 @@ int BatchEngine::autotune(uint64_t pilot_steps, plis_batch_tuning* out) {
     if (rate > best) { best = rate; best_i = i; }
   }
   if (rc == PLIS_OK && best_i >= 0) {
-    rc = layout(cands[best_i]);
+    rc = layout(cands[best_i], best_i == 0);
     tuned_rate_ = best;
   }
   restore();

@@ -46,7 +46,7 @@ class BatchEngine {
  private:
   void release();
   int dmalloc(void** p, size_t bytes);
-  int layout(const int tile[3]);        // bricks, views, grid for a brick shape
+  int layout(const int tile[3], bool runs);  // bricks, views, grid for a brick shape
   int launch(uint32_t max_iters);       // one persistent launch
   int init_pending();
   int read_ctrls();
@@ -61,6 +61,7 @@ class BatchEngine {
   bool small_ = false;
   uint64_t ntot_ = 0;
   uint32_t tile_[3] = {0, 0, 0};
+  bool runs_ = true;
   uint32_t total_tiles_ = 0, max_tiles_ = 0;
   int grid_ = 0, blocks_per_sm_ = 0;
   double tuned_rate_ = 0.0;
