@@ -274,7 +274,8 @@ int BatchEngine::create(const plis_batch_desc& d, const plis_options& opt) {
   if (!given) { tile[0] = 8; tile[1] = 8; tile[2] = 4; }
   rc = layout(tile, !given);
   if (rc) return rc;
-  PLIS_CU(cudaDeviceSynchronize());
+  // the uploads and clears above; not the whole device, which fails while another thread captures a graph
+  PLIS_CU(cudaStreamSynchronize(cudaStreamLegacy));
   return PLIS_OK;
 }
 

@@ -415,7 +415,8 @@ int Engine::create(const Model& model, const plis_options& opt) {
   }
   kernels_per_step_ = ((opt.mode == PLIS_MODE_REFERENCE) ? 3 : 2) + classify_kernels();
   graph_steps_ = opt.steps_per_launch > 0 ? opt.steps_per_launch : 32;
-  PLIS_CU(cudaDeviceSynchronize());
+  // the uploads and clears above; not the whole device, which fails while another thread captures a graph
+  PLIS_CU(cudaStreamSynchronize(cudaStreamLegacy));
   return PLIS_OK;
 }
 
