@@ -65,15 +65,15 @@ def _peaks():
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the committed
 # ncu capture of the same kernel on the same workload (profiles/k_leap_schlogl64.md: 2.43 MB read,
-# 4 KB written per launch under ncu's cache flush).  Keyed by (workload, semantics, precision, kernel); absent
+# 2 KB written per launch under ncu's cache flush).  Keyed by (workload, semantics, precision, kernel); absent
 # keys report null.
-NCU_TRAFFIC = {("schlogl64", "reference", "fp64", "leap"): (2.426368e6 + 4.096e3, "profiles/k_leap_schlogl64.md")}
+NCU_TRAFFIC = {("schlogl64", "reference", "fp64", "leap"): (2.426368e6 + 1.792e3, "profiles/k_leap_schlogl64.md")}
 # smsp__inst_executed.sum per launch (warp instructions) of the same capture.  The kernel is bound by
 # instruction issue and dependent latency, not by DRAM, so the line also reports the achieved warp-
 # instruction rate against the issue peak (148 SMs x 4 schedulers x the SM clock sampled during the
-# timed region).  The count is that of an early step from the initial state; later steps of the bench
+# timed region).  The count is that of step 41 from the initial state; later steps of the bench
 # trajectory draw from similar Poisson means, so the rate is an estimate.
-NCU_WARP_INSTR = {("schlogl64", "reference", "fp64", "leap"): (11.100745e6, "profiles/k_leap_schlogl64.md")}
+NCU_WARP_INSTR = {("schlogl64", "reference", "fp64", "leap"): (11.100816e6, "profiles/k_leap_schlogl64.md")}
 SM_COUNT, SCHEDULERS_PER_SM = 148, 4
 
 def issue_roofline(instr, ms_launch, clocks):
@@ -287,13 +287,13 @@ def ncu_learned_case(args):
 
 
 def ncu_batch_case(args):
-    """Fixed small case for ncu captures of the batched form: 32 Brusselator replicas (sides 8..24),
-    brick 8x8x2, one persistent launch of 20 steps after a 5-step one (capture with -k regex:k_batch
-    -s 1 -c 1)."""
+    """Fixed small case for ncu captures of the batched form: 32 Brusselator replicas (sides 8..24) in
+    the default cut, one persistent launch of 20 steps after a 5-step one (capture with
+    -k regex:"^k_batch$" -s 2 -c 1)."""
     from pliscuda_b200 import workloads
     from pliscuda_b200.batch import Batch
     reps = workloads.brusselator_batch(32, side_range=(8, 24))
-    with Batch.from_models([r[0] for r in reps], seed=1, tile=(8, 8, 2)) as b:
+    with Batch.from_models([r[0] for r in reps], seed=1) as b:
         for i, r in enumerate(reps):
             b.set_state(i, r[1])
         b.step(5)

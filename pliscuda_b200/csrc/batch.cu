@@ -365,7 +365,8 @@ int BatchEngine::layout(const int tile[3], bool runs) {
 
 static BatchArgs make_args(const DevModel& dm, const DevOpts& o, const Geo& g, void* views, void* rep, uint32_t nrep,
                            uint32_t R, uint32_t S, void* rr, void* dr, Ctrl* ctrl, int32_t* const X[3],
-                           double* const tau[2], uint8_t* const flag[2], int32_t* D, unsigned* work, unsigned* bar, int* err, uint32_t iters) {
+                           double* const tau[2], uint8_t* const flag[2], int32_t* D, unsigned* work, unsigned* bar,
+                           int* err, uint32_t iters) {
   BatchArgs B;
   std::memset(&B, 0, sizeof B);
   B.m = dm;

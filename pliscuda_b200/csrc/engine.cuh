@@ -176,13 +176,15 @@ inline void geo_divisors(Geo& g) {
 // the better cut (call after geo_divisors; g keeps the brick's sides for geo_bricks).  Bricks share more of
 // their neighbours' lines, but lanes beyond the lattice idle; every lane of a run has a subvolume, and a run's
 // loads and atomics are whole lines.  Measured, us per step, bricks -> runs:
-//   more than 1/16 of the bricks' lanes beyond the lattice: Schlogl 100^3 89.6 -> 85.1, 101^3 in binary32 77.2 -> 71.4,
-//     42^3 19.4 -> 14.6, 20^3 10.64 -> 10.18, a network on 50x61x47 98.3 -> 88.0; 256 Brusselators of side 8..48
-//     in a batch 1386 -> 1153 a round (24 % of the bricks' lanes idle), 4200 -> 3492 with learned proposals.  Not below `least` subvolumes: few CTAs
-//     are latency, which more and emptier ones hide (A/B 10^3: 10.15 -> 10.26 with 4 runs for 12 bricks).
+//   more than 1/16 of the bricks' lanes beyond the lattice: Schlogl 100^3 85.1 -> 80.8, 101^3 in binary32
+//     78.3 -> 74.4, 67x45x53 in binary32 22.6 -> 21.4, 42^3 17.8 -> 14.1, 20^3 10.1 -> 9.8, a network on 50x61x47
+//     98.3 -> 88.0; 256 Brusselators of side 8..48 in a batch 1386 -> 1153 a round (24 % of the bricks' lanes
+//     idle), 4200 -> 3492 with learned proposals.  Not below `least` subvolumes: few CTAs are latency, which
+//     more and emptier ones hide (A/B 10^3: 10.15 -> 10.26 with 4 runs for 12 bricks).
 //   nothing beyond the lattice, runs of whole x rows or parts of one (`whole`: small models in phase kernels):
-//     64^3 30.8 -> 28.9, 128x128x16 30.4 -> 28.3, 256x16x64 30.5 -> 28.2, 128^3 164.9 -> 162.6.  Runs that break
-//     rows lose (96^3 76.2 -> 77.1, 112^3 114 -> 116), as do networks (128^3 826 -> 841) and 16^3 batches (63.4 -> 63.8).
+//     64^3 28.8 -> 27.1, 128x128x16 28.7 -> 26.8, 256x16x64 28.7 -> 26.4, 128^3 156.8 -> 154.8.  Runs that break
+//     rows lose (96^3 76.2 -> 77.1, 112^3 114 -> 116 in an earlier build), as do networks (128^3 826 -> 841) and
+//     batches of 16^3 (63.4 -> 63.8).
 inline void geo_rows(Geo& g, uint32_t X, uint32_t Y, uint32_t Z, uint64_t least, bool whole) {
   const uint64_t n = (uint64_t)X * Y * Z;
   const bool padded = (uint64_t)g.nblocks * 256 * 16 > n * 17;

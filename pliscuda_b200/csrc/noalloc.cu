@@ -71,9 +71,10 @@ __device__ __forceinline__ void block_min(double& t, long long& i, double* st, l
 }
 
 // Pass 1, one partial per CTA (direct: a single CTA, its result is the answer).  The pass is bound by
-// memory: a thread keeps kUnroll 16-byte loads in flight, 192 KB per SM.  On 2^24 taus a call takes
-// 28.8 us on one B200 (20.5 at the measured copy bandwidth); one 8-byte load per iteration took 34.8.  head = 1 when only tau + 1 is 16-byte
-// aligned; tau[0] is then thread 0's.  Indices of a thread grow, so a strict < keeps its first minimum.
+// memory: a thread keeps kUnroll 16-byte loads in flight, 128 KB per SM (four CTAs at 51 registers).  On 2^24
+// taus a call takes 29.2 us on one B200 (20.5 at the measured copy bandwidth); one 8-byte load per iteration
+// took 34.8.  head = 1 when only tau + 1 is 16-byte aligned; tau[0] is then thread 0's.  Indices of a thread
+// grow, so a strict < keeps its first minimum.
 constexpr int kUnroll = 8;
 __global__ void __launch_bounds__(kThreads) k_argmin_partials(const double* __restrict__ tau, long long n, int head, Partial* part,
                                                               double* out_tau, long long* out_idx) {
@@ -151,8 +152,8 @@ extern "C" int plis_tau_argmin_noalloc(const double* d_tau, uint64_t n, double* 
   const long long nn = (long long)n;
   cudaStream_t s = (cudaStream_t)stream;
   const int head = (int)(((uintptr_t)d_tau >> 3) & 1u);
-  // up to 8192 taus one CTA does it in one launch; above, a CTA for every 16 taus of a thread, six CTAs
-  // per SM of a B200 (888) at most
+  // up to 8192 taus one CTA does it in one launch; above, a CTA for every 16 taus of a thread, 888 at most
+  // (six for each SM of a B200, four of them resident)
   long long blocks = nn <= 8192 ? 1 : (nn + 16 * kThreads - 1) / (16 * kThreads);
   if (blocks > 888) blocks = 888;
   if (blocks == 1) {
